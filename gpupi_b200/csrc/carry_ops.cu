@@ -14,16 +14,20 @@
 // which gives the reference's "computed over max+1 limbs, truncated or
 // zero-extended to L_c" semantics directly.
 //
-// Launch shapes (all sm_100a, no inter-CTA waiting):
-//   * lanes per row    - short rows (L_c <= 32) in huge batches: 8, 16 or
-//                        32 lanes per row, one ballot pair;
-//   * warp per row     - 32-limb groups resolved with two ballots and one
-//                        64-bit add (common.cuh), carry kept warp-uniform;
+// Every thread handles four consecutive limbs whose first output word lies on
+// a 16-byte boundary of the row (a row's first chunk starts up to three limbs
+// below limb 0, where both streams read as 0), so C is written in 128-bit
+// stores; operands are read in 128-bit loads too, whatever their alignment
+// (read4).  Launch shapes (no inter-CTA waiting):
+//   * lanes per row    - rows of up to 125 limbs: 4, 8, 16 or 32 lanes per
+//                        row, one ballot pair;
+//   * warp per row     - longer rows up to 4096 limbs (or very many rows):
+//                        512 limbs per step, the carry kept warp-uniform;
 //   * tiles + fix-up   - long rows: each CTA owns a 4096-limb tile, writes its
-//                        result assuming carry-in 0 plus (generate, propagate,
-//                        ones-prefix) flags; a second kernel scans the flags
-//                        of each row and patches only the all-ones prefix of
-//                        tiles that receive a carry (usually one limb).
+//                        result assuming carry-in 0 plus (generate, propagate)
+//                        flags; a second kernel scans the flags of each row and
+//                        adds the carry to the tiles that receive one (usually
+//                        one limb).
 // Traffic is the algorithmic minimum (read operands once, write C once)
 // except for the few fix-up limbs.
 #include "common.cuh"
@@ -40,17 +44,51 @@
 namespace gpupi {
 
 // ---------------------------------------------------------------------------
-// Operand generators
+// Operand generators: read() gives limbs j .. j + 3 of the two streams (j may
+// be as low as -3; limbs below 0 are 0).
 // ---------------------------------------------------------------------------
+
+// out[v] = r[j + v], 0 outside [0, len).  Inside the row: one 128-bit load
+// when r + j is 16-byte aligned; otherwise the two aligned words that hold the
+// four limbs, where both lie inside the row (the second is the neighbouring
+// thread's first and comes from L1); limb by limb at the row's ends.  The
+// misalignment is the same for all chunks of a row.
+template <bool VEC>
+__device__ __forceinline__ void read4(const uint32_t *r, uint32_t len, int64_t j, uint32_t (&o)[4]) {
+    const uint32_t *p = r + j;
+    if (VEC && j >= 0 && j + 4 <= (int64_t)len) {
+        const uint32_t m = ((uintptr_t)p >> 2) & 3u;
+        if (m == 0u) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(p);
+            o[0] = q.x;
+            o[1] = q.y;
+            o[2] = q.z;
+            o[3] = q.w;
+            return;
+        }
+        if (j >= (int64_t)m && j - m + 8 <= (int64_t)len) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(p - m);
+            const uint4 b = *reinterpret_cast<const uint4 *>(p - m + 4);
+            o[0] = m == 1u ? a.y : (m == 2u ? a.z : a.w);
+            o[1] = m == 1u ? a.z : (m == 2u ? a.w : b.x);
+            o[2] = m == 1u ? a.w : (m == 2u ? b.x : b.y);
+            o[3] = m == 1u ? b.x : (m == 2u ? b.y : b.z);
+            return;
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) o[v] = ((uint64_t)(j + v) < (uint64_t)len) ? p[v] : 0u;   // j + v < 0 wraps
+}
+
 struct GenTwo {
     const uint32_t *A;
     const uint32_t *B;
     uint32_t La, Lb;
     uint64_t sA, sB;
-    __device__ __forceinline__ void operator()(uint32_t row, uint32_t j, uint32_t &x,
-                                               uint32_t &y) const {
-        x = (j < La) ? A[row * sA + j] : 0u;
-        y = (j < Lb) ? B[row * sB + j] : 0u;
+    template <bool VEC>
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+        read4<VEC>(A + row * sA, La, j, x);
+        read4<VEC>(B + row * sB, Lb, j, y);
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc) + std::min(Lb, Lc); }
 };
@@ -60,10 +98,11 @@ struct GenSmall {
     uint32_t b;
     uint32_t La;
     uint64_t sA;
-    __device__ __forceinline__ void operator()(uint32_t row, uint32_t j, uint32_t &x,
-                                               uint32_t &y) const {
-        x = (j < La) ? A[row * sA + j] : 0u;
-        y = (j == 0u) ? b : 0u;
+    template <bool VEC>
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+        read4<VEC>(A + row * sA, La, j, x);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) y[v] = (j + v == 0) ? b : 0u;
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
@@ -73,11 +112,17 @@ struct GenMulSmall {
     uint32_t b;
     uint32_t La;
     uint64_t sA;
-    __device__ __forceinline__ void operator()(uint32_t row, uint32_t j, uint32_t &x,
-                                               uint32_t &y) const {
+    template <bool VEC>
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
         const uint32_t *r = A + row * sA;
-        x = (j < La) ? r[j] * b : 0u;
-        y = (j >= 1u && j - 1u < La) ? __umulhi(r[j - 1u], b) : 0u;
+        uint32_t a[4];
+        read4<VEC>(r, La, j, a);
+        const uint32_t prev = ((uint64_t)(j - 1) < (uint64_t)La) ? r[j - 1] : 0u;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            x[v] = a[v] * b;
+            y[v] = __umulhi(v ? a[v - 1] : prev, b);
+        }
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
@@ -88,55 +133,116 @@ struct GenShiftTwo {
     uint32_t La, Lb;
     uint64_t sA, sB;
     uint32_t word, bit;
-    __device__ __forceinline__ void operator()(uint32_t row, uint32_t j, uint32_t &x,
-                                               uint32_t &y) const {
+    template <bool VEC>
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
         const uint32_t *r = A + row * sA;
-        uint32_t lo = 0u, prev = 0u;
-        if (j >= word) {
-            const uint32_t src = j - word;
-            lo = (src < La) ? r[src] : 0u;
-            prev = (bit != 0u && src >= 1u && src - 1u < La) ? r[src - 1u] : 0u;
-        }
-        x = (bit == 0u) ? lo : ((lo << bit) | (prev >> (32u - bit)));
-        y = (j < Lb) ? B[row * sB + j] : 0u;
+        const int64_t i = j - (int64_t)word;
+        uint32_t a[4];
+        read4<VEC>(r, La, i, a);
+        const uint32_t prev = ((uint64_t)(i - 1) < (uint64_t)La) ? r[i - 1] : 0u;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) x[v] = __funnelshift_l(v ? a[v - 1] : prev, a[v], bit);   // bit < 32
+        read4<VEC>(B + row * sB, Lb, j, y);
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc) + std::min(Lb, Lc); }
 };
 
 // ---------------------------------------------------------------------------
+// Four-limb chunks
+// ---------------------------------------------------------------------------
+// s = x +/- y with carry-in 0; g: carry out, p: a carry in would run through.
+template <bool SUB>
+__device__ __forceinline__ void chunk_raw(const uint32_t (&x)[4], const uint32_t (&y)[4], uint32_t (&s)[4], bool &g,
+                                          bool &p) {
+    uint32_t c;
+    if (SUB)
+        asm("sub.cc.u32 %0, %5, %9;\n\tsubc.cc.u32 %1, %6, %10;\n\tsubc.cc.u32 %2, %7, %11;\n\t"
+            "subc.cc.u32 %3, %8, %12;\n\tsubc.u32 %4, 0, 0;"
+            : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(c)
+            : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
+    else
+        asm("add.cc.u32 %0, %5, %9;\n\taddc.cc.u32 %1, %6, %10;\n\taddc.cc.u32 %2, %7, %11;\n\t"
+            "addc.cc.u32 %3, %8, %12;\n\taddc.u32 %4, 0, 0;"
+            : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(c)
+            : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
+    g = c != 0u;
+    p = SUB ? (s[0] | s[1] | s[2] | s[3]) == 0u : (s[0] & s[1] & s[2] & s[3]) == 0xffffffffu;
+}
+
+template <bool SUB>
+__device__ __forceinline__ void chunk_carry(uint32_t (&s)[4], uint32_t cin) {
+    if (SUB)
+        asm("sub.cc.u32 %0, %0, %4;\n\tsubc.cc.u32 %1, %1, 0;\n\tsubc.cc.u32 %2, %2, 0;\n\tsubc.u32 %3, %3, 0;"
+            : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3])
+            : "r"(cin));
+    else
+        asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.cc.u32 %2, %2, 0;\n\taddc.u32 %3, %3, 0;"
+            : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3])
+            : "r"(cin));
+}
+
+// Limbs j .. j + 3 of a row; out + j is 16-byte aligned.
+__device__ __forceinline__ void chunk_write(uint32_t *out, uint32_t Lc, int64_t j, const uint32_t (&s)[4]) {
+    if (j >= 0 && j + 4 <= (int64_t)Lc) {
+        *reinterpret_cast<uint4 *>(out + j) = make_uint4(s[0], s[1], s[2], s[3]);
+    } else {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            if ((uint64_t)(j + v) < (uint64_t)Lc) out[j + v] = s[v];
+    }
+}
+
+// Limbs from the last 16-byte boundary at or below a row to the row.
+__device__ __forceinline__ int64_t row_offset(const uint32_t *out) { return (int64_t)(((uintptr_t)out >> 2) & 3u); }
+
+// ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-// G lanes per row (G = 8, 16, 32; L_c <= G), 32 / G rows per warp: the
-// short rows of the splitting tree's lower levels (millions of 6..32-limb
-// rows) with whole groups of lanes reading and writing each row's limbs
-// contiguously.
-template <class Gen, bool SUB, int G>
-__global__ void carry_seg_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
+// G lanes per row (L_c + 3 <= 4 G), 32 / G rows per warp, ROWS such sets per
+// step so that each lane has the loads of several rows in flight.  Rows this
+// short are read limb by limb (from L1 after the first of a chunk's loads):
+// most chunks of a row that is not 16-byte aligned touch one of its ends, and
+// a warp that takes both of read4's paths is slower than the plain loads.
+template <class Gen, bool SUB, int G, int ROWS>
+__global__ void __launch_bounds__(256) carry_lane_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
     constexpr uint32_t kMask = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
+    constexpr int PW = 32 / G;
     const uint32_t lane = lane_id();
     const uint32_t grp = lane / G, gl = lane % G;
     const uint32_t warps_per_cta = blockDim.x >> 5;
     const uint64_t gwarp = (uint64_t)blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
     const uint64_t nwarps = (uint64_t)gridDim.x * warps_per_cta;
     // the whole warp runs every iteration (ballots); rows past N do nothing
-    for (uint64_t base = gwarp * (32 / G); base < N; base += nwarps * (32 / G)) {
-        const uint64_t row = base + grp;
-        const bool valid = row < N && gl < Lc;
-        uint32_t x = 0u, y = 0u;
-        if (valid) gen((uint32_t)row, gl, x, y);
-        bool g, p;
-        const uint32_t s = raw_limb<SUB>(x, y, g, p);
-        if (!valid) g = p = false;
-        const uint32_t gm = (__ballot_sync(0xffffffffu, g) >> (grp * G)) & kMask;
-        const uint32_t pm = (__ballot_sync(0xffffffffu, p) >> (grp * G)) & kMask;
-        const GroupCarry gc = resolve_group_n(gm, pm, 0u, G);
-        const uint32_t r = apply_carry<SUB>(s, (gc.carry_in_mask >> gl) & 1u);
-        if (valid) C[row * sC + gl] = r;
+    for (uint64_t base = gwarp * (PW * ROWS); base < N; base += nwarps * (PW * ROWS)) {
+        uint32_t s[ROWS][4];
+        bool g[ROWS], p[ROWS];
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const uint64_t row = base + u * PW + grp;
+            g[u] = p[u] = false;
+            if (row < N) {
+                uint32_t x[4], y[4];
+                gen.template read<false>((uint32_t)row, 4 * (int64_t)gl - row_offset(C + row * sC), x, y);
+                chunk_raw<SUB>(x, y, s[u], g[u], p[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+            const uint64_t row = base + u * PW + grp;
+            const uint32_t gm = (__ballot_sync(0xffffffffu, g[u]) >> (grp * G)) & kMask;
+            const uint32_t pm = (__ballot_sync(0xffffffffu, p[u]) >> (grp * G)) & kMask;
+            const GroupCarry gc = resolve_group_n(gm, pm, 0u, G);
+            if (row < N) {
+                uint32_t *out = C + row * sC;
+                chunk_carry<SUB>(s[u], (gc.carry_in_mask >> gl) & 1u);
+                chunk_write(out, Lc, 4 * (int64_t)gl - row_offset(out), s[u]);
+            }
+        }
     }
 }
 
 template <class Gen, bool SUB, int UNROLL>
-__global__ void carry_warp_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
+__global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
     const uint32_t lane = lane_id();
     const uint32_t warps_per_cta = blockDim.x >> 5;
     const uint32_t gwarp = blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
@@ -144,116 +250,82 @@ __global__ void carry_warp_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, u
     for (uint32_t row = gwarp; row < N; row += nwarps) {
         uint32_t cin = 0u;
         uint32_t *out = C + row * sC;
-        for (uint32_t base = 0; base < Lc; base += 32u * UNROLL) {
-            uint32_t s[UNROLL], gm[UNROLL], pm[UNROLL];
+        for (int64_t base = -row_offset(out); base < (int64_t)Lc; base += 128 * UNROLL) {
+            uint32_t s[UNROLL][4], gm[UNROLL], pm[UNROLL];
 #pragma unroll
             for (int u = 0; u < UNROLL; ++u) {
-                const uint32_t j = base + u * 32u + lane;
-                uint32_t x = 0u, y = 0u;
-                if (j < Lc) gen(row, j, x, y);
+                uint32_t x[4], y[4];
                 bool g, p;
-                s[u] = raw_limb<SUB>(x, y, g, p);
-                if (j >= Lc) g = p = false;
+                gen.template read<true>(row, base + u * 128 + 4 * lane, x, y);
+                chunk_raw<SUB>(x, y, s[u], g, p);
                 gm[u] = __ballot_sync(0xffffffffu, g);
                 pm[u] = __ballot_sync(0xffffffffu, p);
             }
 #pragma unroll
             for (int u = 0; u < UNROLL; ++u) {
-                const uint32_t j = base + u * 32u + lane;
                 const GroupCarry gc = resolve_group(gm[u], pm[u], cin);
                 cin = gc.carry_out;
-                const uint32_t r = apply_carry<SUB>(s[u], (gc.carry_in_mask >> lane) & 1u);
-                if (j < Lc) out[j] = r;
+                chunk_carry<SUB>(s[u], (gc.carry_in_mask >> lane) & 1u);
+                chunk_write(out, Lc, base + u * 128 + 4 * lane, s[u]);
             }
         }
     }
 }
 
 constexpr int kTileWarps = 8;
-constexpr int kTileGroups = 16;                          // 32-limb groups per warp
-constexpr uint32_t kWarpSpan = 32u * kTileGroups;        // 512 limbs
-constexpr uint32_t kTileSpan = kWarpSpan * kTileWarps;   // 4096 limbs
+constexpr int kTileSub = 4;                                   // 128-limb groups per warp
+constexpr uint32_t kTileSpan = 128u * kTileWarps * kTileSub;   // 4096 limbs
+static_assert(kTileWarps * kTileSub == 32, "one lane per 128-limb group of the tile");
 
-// Per-tile flags: bit 0 = generates a carry with carry-in 0, bit 1 = lets a
-// carry through (result with carry-in 0 is all ones / all zeros for sub),
-// bits 2.. = length of the all-ones (all-zeros) prefix of the tile result.
+// A row's tiles start at its last 16-byte boundary at or below limb 0.
+static uint32_t carry_tile_count(uint32_t Lc) { return (uint32_t)(((uint64_t)Lc + 3u + kTileSpan - 1u) / kTileSpan); }
+
+// One 4096-limb tile per CTA: group (u, w) = 128 limbs, u-th of warp w.  The
+// 32 groups' carries are resolved by one warp-wide ballot.  Flags: bit 0 =
+// generates a carry with carry-in 0, bit 1 = lets a carry through.
+// Bound by HBM: shift_add of two 2^26-limb rows 489 -> 162 us (805 MB,
+// 5.0 TB/s), sub 443 -> 151 us, mul_small 428 -> 96 us (537 MB, 5.6 TB/s)
+// against one limb per lane and ballot, whose 16 ballot pairs and resolutions
+// per 512 limbs kept the loads apart.
 template <class Gen, bool SUB>
 __global__ void __launch_bounds__(kTileWarps * 32)
-carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_row,
-            uint32_t *flags) {
-    __shared__ uint32_t warp_g[kTileWarps], warp_p[kTileWarps], warp_prefix[kTileWarps];
+carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_row, uint32_t *flags) {
+    __shared__ uint32_t group_g[32], group_p[32];
     const uint32_t lane = lane_id();
     const uint32_t w = threadIdx.x >> 5;
     const uint32_t tile = blockIdx.x;
     const uint32_t row = tile / tiles_per_row;
     const uint32_t t = tile - row * tiles_per_row;
-    const uint32_t wbase = t * kTileSpan + w * kWarpSpan;
     uint32_t *out = C + row * sC;
-
-    uint32_t s[kTileGroups], gm[kTileGroups], pm[kTileGroups];
-    const uint32_t ones = SUB ? 0u : 0xffffffffu;
+    const int64_t base = (int64_t)t * kTileSpan - row_offset(out) + w * 128 + 4 * lane;
+    uint32_t s[kTileSub][4], gm[kTileSub], pm[kTileSub];
 #pragma unroll
-    for (int u = 0; u < kTileGroups; ++u) {
-        const uint32_t j = wbase + u * 32u + lane;
-        uint32_t x = 0u, y = 0u;
-        if (j < Lc) gen(row, j, x, y);
+    for (int u = 0; u < kTileSub; ++u) {
+        uint32_t x[4], y[4];
         bool g, p;
-        s[u] = raw_limb<SUB>(x, y, g, p);
-        if (j >= Lc) g = p = false;
+        gen.template read<true>(row, base + u * (128 * kTileWarps), x, y);
+        chunk_raw<SUB>(x, y, s[u], g, p);
         gm[u] = __ballot_sync(0xffffffffu, g);
         pm[u] = __ballot_sync(0xffffffffu, p);
-    }
-    // Pass 1: carry-in 0 for this warp's span.
-    uint32_t c = 0u;
-    bool all_p = true;
-#pragma unroll
-    for (int u = 0; u < kTileGroups; ++u) {
-        c = resolve_group(gm[u], pm[u], c).carry_out;
-        all_p = all_p && (pm[u] == 0xffffffffu);
-    }
-    if (lane == 0) {
-        warp_g[w] = c;
-        warp_p[w] = all_p ? 1u : 0u;
+        if (lane == 0) {
+            group_g[u * kTileWarps + w] = resolve_group(gm[u], pm[u], 0u).carry_out;
+            group_p[u * kTileWarps + w] = (pm[u] == 0xffffffffu) ? 1u : 0u;
+        }
     }
     __syncthreads();
-    // Carry into each warp of the tile (tile carry-in assumed 0).
-    uint32_t gmask = 0u, pmask = 0u;
+    const uint32_t tg = __ballot_sync(0xffffffffu, group_g[lane] != 0u);
+    const uint32_t tp = __ballot_sync(0xffffffffu, group_p[lane] != 0u);
+    const GroupCarry tc = resolve_group(tg, tp, 0u);
 #pragma unroll
-    for (int k = 0; k < kTileWarps; ++k) {
-        gmask |= warp_g[k] << k;
-        pmask |= warp_p[k] << k;
-    }
-    const GroupCarry tc = resolve_group_n(gmask, pmask, 0u, kTileWarps);
-    uint32_t cin = (tc.carry_in_mask >> w) & 1u;
-    // Pass 2: final values, stored, and this warp's ones-prefix.
-    uint32_t prefix = kWarpSpan;
-    bool prefix_open = true;
-#pragma unroll
-    for (int u = 0; u < kTileGroups; ++u) {
-        const uint32_t j = wbase + u * 32u + lane;
+    for (int u = 0; u < kTileSub; ++u) {
+        const uint32_t cin = (tc.carry_in_mask >> (u * kTileWarps + w)) & 1u;
         const GroupCarry gc = resolve_group(gm[u], pm[u], cin);
-        cin = gc.carry_out;
-        const uint32_t r = apply_carry<SUB>(s[u], (gc.carry_in_mask >> lane) & 1u);
-        if (j < Lc) out[j] = r;
-        const uint32_t not_ones = __ballot_sync(0xffffffffu, (r != ones) || (j >= Lc));
-        if (prefix_open && not_ones != 0u) {
-            prefix = u * 32u + (uint32_t)(__ffs(not_ones) - 1);
-            prefix_open = false;
-        }
+        chunk_carry<SUB>(s[u], (gc.carry_in_mask >> lane) & 1u);
+        chunk_write(out, Lc, base + u * (128 * kTileWarps), s[u]);
     }
-    if (lane == 0) warp_prefix[w] = prefix;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t pre = 0u;
-        for (int k = 0; k < kTileWarps; ++k) {
-            pre += warp_prefix[k];
-            if (warp_prefix[k] != kWarpSpan) break;
-        }
-        // tile generate/propagate: warp 7's outgoing carry with tile cin 0
-        const uint32_t G = tc.carry_out;
-        const uint32_t P = (pmask == 0xffu) ? 1u : 0u;
-        flags[tile] = G | (P << 1) | (pre << 2);
-    }
+    // P: the tile's result is all ones (all zeros), which with carry-in 0 means
+    // that every limb's raw sum is
+    if (threadIdx.x == 0) flags[tile] = tc.carry_out | ((tp == 0xffffffffu) ? 2u : 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -262,15 +334,20 @@ carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_r
 enum class CarryPlan { Lanes, Warp, Tiles };
 
 static CarryPlan plan_for(uint32_t N, uint32_t Lc) {
-    if (Lc <= 32u && N >= 2048u) return CarryPlan::Lanes;
+    if (Lc <= 125u) return CarryPlan::Lanes;   // with the 3 limbs below a row: 4 limbs x 32 lanes
     if (Lc <= kTileSpan || (uint64_t)N >= (uint64_t)kNumSMs * 64u) return CarryPlan::Warp;
     return CarryPlan::Tiles;
 }
 
 static size_t carry_workspace_bytes(uint32_t N, uint32_t Lc) {
     if (N == 0u || Lc == 0u || plan_for(N, Lc) != CarryPlan::Tiles) return 0;
-    const uint64_t tiles = (Lc + kTileSpan - 1u) / kTileSpan;
-    return (size_t)N * tiles * sizeof(uint32_t);
+    return (size_t)N * carry_tile_count(Lc) * sizeof(uint32_t);
+}
+
+template <class Gen, bool SUB, int G, int ROWS>
+static void launch_lanes(const Gen &gen, uint32_t *C, uint32_t N, uint32_t Lc, uint32_t sC, cudaStream_t st) {
+    carry_lane_rows<Gen, SUB, G, ROWS>
+        <<<grid_for(N, 8 * (32 / G) * ROWS, kNumSMs * 32), 256, 0, st>>>(gen, C, sC, N, Lc);
 }
 
 template <class Gen, bool SUB>
@@ -281,32 +358,26 @@ static void run_carry(const Gen &gen, uint32_t *C, uint32_t N, uint32_t Lc, uint
     const CarryPlan plan = plan_for(N, Lc);
     KernelTimed kt("carry_chain", 4.0 * N * (gen.read_limbs(Lc) + (double)Lc));
     if (plan == CarryPlan::Lanes) {
-        // rows per 256-thread CTA: 8 warps x 32 / G
-        if (Lc <= 8u)
-            carry_seg_rows<Gen, SUB, 8><<<grid_for(N, 32, kNumSMs * 32), 256, 0, st>>>(gen, C, sC, N, Lc);
-        else if (Lc <= 16u)
-            carry_seg_rows<Gen, SUB, 16><<<grid_for(N, 16, kNumSMs * 32), 256, 0, st>>>(gen, C, sC, N, Lc);
+        if (Lc <= 13u)
+            launch_lanes<Gen, SUB, 4, 2>(gen, C, N, Lc, sC, st);
+        else if (Lc <= 29u)
+            launch_lanes<Gen, SUB, 8, 2>(gen, C, N, Lc, sC, st);
+        else if (Lc <= 61u)
+            launch_lanes<Gen, SUB, 16, 2>(gen, C, N, Lc, sC, st);
         else
-            carry_seg_rows<Gen, SUB, 32><<<grid_for(N, 8, kNumSMs * 32), 256, 0, st>>>(gen, C, sC, N, Lc);
+            launch_lanes<Gen, SUB, 32, 2>(gen, C, N, Lc, sC, st);
         GPUPI_LAUNCH_CHECK();
     } else if (plan == CarryPlan::Warp) {
         const unsigned warps = 8;
-        if (Lc <= 64u) {
-            carry_warp_rows<Gen, SUB, 2><<<grid_for(N, warps), warps * 32, 0, st>>>(gen, C, sC, N, Lc);
-        } else if (Lc <= 1024u) {
-            carry_warp_rows<Gen, SUB, 4><<<grid_for(N, warps), warps * 32, 0, st>>>(gen, C, sC, N, Lc);
-        } else {
-            // long rows: more 32-limb groups in flight per warp
-            carry_warp_rows<Gen, SUB, 8><<<grid_for(N, warps), warps * 32, 0, st>>>(gen, C, sC, N, Lc);
-        }
+        carry_warp_rows<Gen, SUB, 4><<<grid_for(N, warps), warps * 32, 0, st>>>(gen, C, sC, N, Lc);
         GPUPI_LAUNCH_CHECK();
     } else {
-        const uint32_t tiles = (Lc + kTileSpan - 1u) / kTileSpan;
+        const uint32_t tiles = carry_tile_count(Lc);
         const uint64_t total = (uint64_t)tiles * N;
         carry_tiles<Gen, SUB><<<(unsigned)total, kTileWarps * 32, 0, st>>>(gen, C, sC, Lc, tiles,
                                                                          workspace);
         GPUPI_LAUNCH_CHECK();
-        launch_carry_fixup(SUB, C, sC, N, Lc, tiles, kTileSpan, workspace, st);
+        launch_carry_fixup(SUB, C, sC, N, Lc, tiles, kTileSpan, true, workspace, st);
     }
 }
 
@@ -430,7 +501,9 @@ size_t batch_shift_sub_simple_workspace_size(uint32_t N, uint32_t L_a, uint32_t 
 namespace gpupi {
 
 constexpr uint64_t kNoAllocMaxTiles = 65536;
-static __device__ __align__(256) uint32_t g_noalloc_flags[kNoAllocMaxTiles];
+// rows on the multi-tile path (fewer than 64 per SM) have one tile more than
+// ceil(L_c / 4096) when their last tile has fewer than three limbs to spare
+static __device__ __align__(256) uint32_t g_noalloc_flags[kNoAllocMaxTiles + (uint64_t)kNumSMs * 64u];
 
 // Device address of g_noalloc_flags, looked up once per device (with that
 // device current) on the first call that needs it.

@@ -123,7 +123,6 @@ __device__ __forceinline__ GroupCarry resolve_group(uint32_t gmask, uint32_t pma
     return r;
 }
 
-// Raw limb op: returns s and sets g/p for the carry scan.
 // Same resolution for a group of n <= 32 members held in bits [0, n).  The
 // members are moved to the top bits and the free low bits are marked
 // "propagate", so cin still enters at bit 0 and the carry out is bit 32.
@@ -138,24 +137,12 @@ __device__ __forceinline__ GroupCarry resolve_group_n(uint32_t gmask, uint32_t p
     return r;
 }
 
-template <bool SUB>
-__device__ __forceinline__ uint32_t raw_limb(uint32_t x, uint32_t y, bool &g, bool &p) {
-    if (SUB) {
-        const uint32_t d = x - y;
-        g = x < y;
-        p = (d == 0u);
-        return d;
-    } else {
-        const uint32_t s = x + y;
-        g = s < x;
-        p = (s == 0xffffffffu);
-        return s;
-    }
-}
-
-template <bool SUB>
-__device__ __forceinline__ uint32_t apply_carry(uint32_t s, uint32_t c) {
-    return SUB ? s - c : s + c;
+// Raw limb sum: returns s and sets g/p for the carry scan.
+__device__ __forceinline__ uint32_t raw_limb_add(uint32_t x, uint32_t y, bool &g, bool &p) {
+    const uint32_t s = x + y;
+    g = s < x;
+    p = (s == 0xffffffffu);
+    return s;
 }
 
 }  // namespace gpupi

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(128) k_decimal_warp(const uint32_t *__restrict
                 if (lane == 0) y = prev_hi;
                 prev_hi = __shfl_sync(0xffffffffu, hi, 31);
                 bool gg, pp;
-                const uint32_t s = raw_limb<false>(lo, y, gg, pp);
+                const uint32_t s = raw_limb_add(lo, y, gg, pp);
                 const uint32_t gm = __ballot_sync(0xffffffffu, gg);
                 const uint32_t pm = __ballot_sync(0xffffffffu, pp);
                 const GroupCarry gc = resolve_group(gm, pm, cin);

@@ -891,7 +891,7 @@ __device__ __forceinline__ void crt_chunk(const uint32_t *F0, int log_k, uint32_
 }
 
 __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
-    __shared__ uint32_t sg[kThreads / 32], sp[kThreads / 32], spre[kThreads / 32];
+    __shared__ uint32_t sg[kThreads / 32], sp[kThreads / 32];
     __shared__ uint32_t spill[kThreads / 32][3];
     const uint32_t tile = blockIdx.x;
     const uint64_t row = tile / a.tiles;
@@ -941,14 +941,7 @@ __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
 #pragma unroll
     for (int v = 0; v < kCrtV; ++v)
         if (base + v < (int64_t)a.Lc) out[base + v] = X[v];
-    if (a.tiles > 1u) {
-        uint32_t local = kCrtV;
-#pragma unroll
-        for (int v = kCrtV - 1; v >= 0; --v)
-            if (X[v] != 0xffffffffu || base + v >= (int64_t)a.Lc) local = v;
-        const uint32_t pre = block_prefix<kThreads / 32, kCrtV>(local, spre);
-        if (threadIdx.x == 0) a.flags[tile] = bc.G | (bc.P << 1) | (pre << 2);
-    }
+    if (a.tiles > 1u && threadIdx.x == 0) a.flags[tile] = bc.G | (bc.P << 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1271,7 +1264,7 @@ static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32
     KernelTimed kt("ntt_crt_carry", 12.0 * (double)Lc * N + 4.0 * (double)Lc * N);
     k_crt<<<(unsigned)(N * tiles), kThreads, 0, st>>>(c);
     count_launch();
-    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, flags, st);
+    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, false, flags, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1378,7 +1371,7 @@ static void spectrum_inverse(const NttParams &P, Shape s, uint32_t N, int terms,
                                         (add ? 4.0 * (double)add->Ld * N : 0.0));
     k_crt<<<(unsigned)(N * tiles), kThreads, 0, st>>>(c);
     count_launch();
-    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, flags, st);
+    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, false, flags, st);
 }
 
 void build_tables(std::vector<uint32_t> &lv1, std::vector<uint32_t> &lv2, std::vector<uint32_t> &inv2n) {
