@@ -1,9 +1,9 @@
 // Batched schoolbook multiplication (gpupi batch_mul_naive.cu:8-273).
 //
 // Two shapes:
-//   * k_school_thread<MA, MB>: one thread per product for operands of at most
-//     MA x MB limbs (the bottom levels of the splitting tree: 3..16-limb rows
-//     in batches of millions).  Register arrays, fully unrolled MACs.
+//   * k_school_rows<MB>: one thread per product for operands of at most 16
+//     limbs each (the bottom levels of the splitting tree: 3..16-limb rows in
+//     batches of millions), staged through shared memory.
 //   * k_school_seg<G>: G = 8, 16 or 32 lanes per product for
 //     L_a + L_b <= 4 G (up to 128), carries resolved with one ballot pair.
 //   * k_school_cols: one CTA per product, 64-256 threads x 4 consecutive output
@@ -18,39 +18,266 @@
 
 namespace gpupi {
 
-template <int MA, int MB>
-__global__ void __launch_bounds__(128) k_school_thread(const uint32_t *__restrict__ A,
-                                                       const uint32_t *__restrict__ B,
-                                                       uint32_t *__restrict__ C, uint32_t N,
-                                                       uint32_t La, uint32_t Lb, uint64_t sA,
-                                                       uint64_t sB, uint64_t sC) {
-    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < N;
-         row += gridDim.x * blockDim.x) {
-        uint32_t a[MA], b[MB], o[MA + MB];
-        const uint32_t *ar = A + row * sA;
-        const uint32_t *br = B + row * sB;
-#pragma unroll
-        for (int i = 0; i < MA; ++i) a[i] = (i < (int)La) ? ar[i] : 0u;
-#pragma unroll
-        for (int j = 0; j < MB; ++j) b[j] = (j < (int)Lb) ? br[j] : 0u;
-#pragma unroll
-        for (int k = 0; k < MA + MB; ++k) o[k] = 0u;
-#pragma unroll
-        for (int i = 0; i < MA; ++i) {
-            uint32_t carry = 0u;
-#pragma unroll
-            for (int j = 0; j < MB; ++j) {
-                const uint64_t t = (uint64_t)a[i] * b[j] + o[i + j] + carry;
-                o[i + j] = (uint32_t)t;
-                carry = (uint32_t)(t >> 32);
-            }
-            o[i + MB] = carry;
+// d = c + a (b_0 + b_2 2^64 + b_4 2^128 + ...) over 2 P words, dtop = ctop +
+// carry: one carry chain of P 64-bit multiply-adds.  c and d may not overlap.
+template <int P>
+struct MadChain;
+template <>
+struct MadChain<2> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %5, %6, %8;\n\t"
+            "madc.hi.cc.u32 %1, %5, %6, %9;\n\t"
+            "madc.lo.cc.u32 %2, %5, %7, %10;\n\t"
+            "madc.hi.cc.u32 %3, %5, %7, %11;\n\t"
+            "addc.u32 %4, %12, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(ctop));
+    }
+};
+template <>
+struct MadChain<3> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %7, %8, %11;\n\t"
+            "madc.hi.cc.u32 %1, %7, %8, %12;\n\t"
+            "madc.lo.cc.u32 %2, %7, %9, %13;\n\t"
+            "madc.hi.cc.u32 %3, %7, %9, %14;\n\t"
+            "madc.lo.cc.u32 %4, %7, %10, %15;\n\t"
+            "madc.hi.cc.u32 %5, %7, %10, %16;\n\t"
+            "addc.u32 %6, %17, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]),
+              "r"(c[4]), "r"(c[5]), "r"(ctop));
+    }
+};
+template <>
+struct MadChain<4> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %9, %10, %14;\n\t"
+            "madc.hi.cc.u32 %1, %9, %10, %15;\n\t"
+            "madc.lo.cc.u32 %2, %9, %11, %16;\n\t"
+            "madc.hi.cc.u32 %3, %9, %11, %17;\n\t"
+            "madc.lo.cc.u32 %4, %9, %12, %18;\n\t"
+            "madc.hi.cc.u32 %5, %9, %12, %19;\n\t"
+            "madc.lo.cc.u32 %6, %9, %13, %20;\n\t"
+            "madc.hi.cc.u32 %7, %9, %13, %21;\n\t"
+            "addc.u32 %8, %22, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(d[6]), "=&r"(d[7]), "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(b[6]), "r"(c[0]), "r"(c[1]), "r"(c[2]),
+              "r"(c[3]), "r"(c[4]), "r"(c[5]), "r"(c[6]), "r"(c[7]), "r"(ctop));
+    }
+};
+template <>
+struct MadChain<5> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %11, %12, %17;\n\t"
+            "madc.hi.cc.u32 %1, %11, %12, %18;\n\t"
+            "madc.lo.cc.u32 %2, %11, %13, %19;\n\t"
+            "madc.hi.cc.u32 %3, %11, %13, %20;\n\t"
+            "madc.lo.cc.u32 %4, %11, %14, %21;\n\t"
+            "madc.hi.cc.u32 %5, %11, %14, %22;\n\t"
+            "madc.lo.cc.u32 %6, %11, %15, %23;\n\t"
+            "madc.hi.cc.u32 %7, %11, %15, %24;\n\t"
+            "madc.lo.cc.u32 %8, %11, %16, %25;\n\t"
+            "madc.hi.cc.u32 %9, %11, %16, %26;\n\t"
+            "addc.u32 %10, %27, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(d[6]), "=&r"(d[7]), "=&r"(d[8]), "=&r"(d[9]), "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(b[6]), "r"(b[8]), "r"(c[0]), "r"(c[1]),
+              "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(c[5]), "r"(c[6]), "r"(c[7]), "r"(c[8]), "r"(c[9]),
+              "r"(ctop));
+    }
+};
+template <>
+struct MadChain<6> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %13, %14, %20;\n\t"
+            "madc.hi.cc.u32 %1, %13, %14, %21;\n\t"
+            "madc.lo.cc.u32 %2, %13, %15, %22;\n\t"
+            "madc.hi.cc.u32 %3, %13, %15, %23;\n\t"
+            "madc.lo.cc.u32 %4, %13, %16, %24;\n\t"
+            "madc.hi.cc.u32 %5, %13, %16, %25;\n\t"
+            "madc.lo.cc.u32 %6, %13, %17, %26;\n\t"
+            "madc.hi.cc.u32 %7, %13, %17, %27;\n\t"
+            "madc.lo.cc.u32 %8, %13, %18, %28;\n\t"
+            "madc.hi.cc.u32 %9, %13, %18, %29;\n\t"
+            "madc.lo.cc.u32 %10, %13, %19, %30;\n\t"
+            "madc.hi.cc.u32 %11, %13, %19, %31;\n\t"
+            "addc.u32 %12, %32, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(d[6]), "=&r"(d[7]), "=&r"(d[8]), "=&r"(d[9]), "=&r"(d[10]), "=&r"(d[11]),
+              "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(b[6]), "r"(b[8]), "r"(b[10]), "r"(c[0]),
+              "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(c[5]), "r"(c[6]), "r"(c[7]), "r"(c[8]),
+              "r"(c[9]), "r"(c[10]), "r"(c[11]), "r"(ctop));
+    }
+};
+template <>
+struct MadChain<7> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %15, %16, %23;\n\t"
+            "madc.hi.cc.u32 %1, %15, %16, %24;\n\t"
+            "madc.lo.cc.u32 %2, %15, %17, %25;\n\t"
+            "madc.hi.cc.u32 %3, %15, %17, %26;\n\t"
+            "madc.lo.cc.u32 %4, %15, %18, %27;\n\t"
+            "madc.hi.cc.u32 %5, %15, %18, %28;\n\t"
+            "madc.lo.cc.u32 %6, %15, %19, %29;\n\t"
+            "madc.hi.cc.u32 %7, %15, %19, %30;\n\t"
+            "madc.lo.cc.u32 %8, %15, %20, %31;\n\t"
+            "madc.hi.cc.u32 %9, %15, %20, %32;\n\t"
+            "madc.lo.cc.u32 %10, %15, %21, %33;\n\t"
+            "madc.hi.cc.u32 %11, %15, %21, %34;\n\t"
+            "madc.lo.cc.u32 %12, %15, %22, %35;\n\t"
+            "madc.hi.cc.u32 %13, %15, %22, %36;\n\t"
+            "addc.u32 %14, %37, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(d[6]), "=&r"(d[7]), "=&r"(d[8]), "=&r"(d[9]), "=&r"(d[10]), "=&r"(d[11]),
+              "=&r"(d[12]), "=&r"(d[13]), "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(b[6]), "r"(b[8]), "r"(b[10]), "r"(b[12]),
+              "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(c[5]), "r"(c[6]), "r"(c[7]),
+              "r"(c[8]), "r"(c[9]), "r"(c[10]), "r"(c[11]), "r"(c[12]), "r"(c[13]), "r"(ctop));
+    }
+};
+template <>
+struct MadChain<8> {
+    static __device__ __forceinline__ void run(uint32_t a, const uint32_t *b, const uint32_t *c, uint32_t ctop,
+                                               uint32_t *d, uint32_t &dtop) {
+        asm("mad.lo.cc.u32 %0, %17, %18, %26;\n\t"
+            "madc.hi.cc.u32 %1, %17, %18, %27;\n\t"
+            "madc.lo.cc.u32 %2, %17, %19, %28;\n\t"
+            "madc.hi.cc.u32 %3, %17, %19, %29;\n\t"
+            "madc.lo.cc.u32 %4, %17, %20, %30;\n\t"
+            "madc.hi.cc.u32 %5, %17, %20, %31;\n\t"
+            "madc.lo.cc.u32 %6, %17, %21, %32;\n\t"
+            "madc.hi.cc.u32 %7, %17, %21, %33;\n\t"
+            "madc.lo.cc.u32 %8, %17, %22, %34;\n\t"
+            "madc.hi.cc.u32 %9, %17, %22, %35;\n\t"
+            "madc.lo.cc.u32 %10, %17, %23, %36;\n\t"
+            "madc.hi.cc.u32 %11, %17, %23, %37;\n\t"
+            "madc.lo.cc.u32 %12, %17, %24, %38;\n\t"
+            "madc.hi.cc.u32 %13, %17, %24, %39;\n\t"
+            "madc.lo.cc.u32 %14, %17, %25, %40;\n\t"
+            "madc.hi.cc.u32 %15, %17, %25, %41;\n\t"
+            "addc.u32 %16, %42, 0;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]),
+              "=&r"(d[6]), "=&r"(d[7]), "=&r"(d[8]), "=&r"(d[9]), "=&r"(d[10]), "=&r"(d[11]),
+              "=&r"(d[12]), "=&r"(d[13]), "=&r"(d[14]), "=&r"(d[15]), "=&r"(dtop)
+            : "r"(a), "r"(b[0]), "r"(b[2]), "r"(b[4]), "r"(b[6]), "r"(b[8]), "r"(b[10]), "r"(b[12]),
+              "r"(b[14]), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]), "r"(c[5]), "r"(c[6]),
+              "r"(c[7]), "r"(c[8]), "r"(c[9]), "r"(c[10]), "r"(c[11]), "r"(c[12]), "r"(c[13]),
+              "r"(c[14]), "r"(c[15]), "r"(ctop));
+    }
+};
+
+// One thread per product, L_a >= L_b, L_b <= MB (even), L_a <= 16.  The CTA's 128
+// rows are staged in shared memory: operands read and products written as
+// contiguous runs, each thread working on a row of its own (odd pitch: no bank
+// conflicts).  A row holds A, then B; B moves to registers and the product
+// replaces A and B from the bottom as A's limbs are used up.
+//
+// Two limbs of A per step, sums kept in two sets of 64-bit accumulators (E:
+// pairs of words at even positions from the step's base, O: at odd ones), so
+// that the 2 MB products of a step are four carry chains of 64-bit
+// multiply-adds (one instruction each) with no other carry handling; the two
+// lowest words are final after the step and the rest moves down by two words
+// as the second limb's chains write their results.
+// Bound by the multiply-adds (half rate: 4 cycles per warp and scheduler):
+// 262,144 products of 14 x 13 limbs 41.9 -> 26.6 us a call (the previous kernel read
+// and wrote one row per thread straight from memory and kept one serial carry
+// chain per limb of A).
+constexpr int kRowsCta = 128;
+constexpr uint32_t kDivShift = 20;   // e / d = e * ceil(2^20 / d) >> 20 for e < 4096, d <= 32
+
+__device__ __forceinline__ void copy_limb(uint32_t *shared, const uint32_t *global) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)),
+                 "l"(global)
+                 : "memory");
+}
+
+template <int MB>
+__global__ void __launch_bounds__(kRowsCta) k_school_rows(const uint32_t *__restrict__ A,
+                                                          const uint32_t *__restrict__ B, uint32_t *__restrict__ C,
+                                                          uint32_t N, uint32_t La, uint32_t Lb, uint64_t sA,
+                                                          uint64_t sB, uint64_t sC, uint32_t divA, uint32_t divB,
+                                                          uint32_t divC) {
+    __shared__ uint32_t sh[kRowsCta * 33];
+    const uint32_t Lc = La + Lb;
+    const uint32_t pitch = Lc | 1u;
+    const uint32_t t = threadIdx.x;
+    for (uint64_t r0 = (uint64_t)blockIdx.x * kRowsCta; r0 < N; r0 += (uint64_t)gridDim.x * kRowsCta) {
+        const uint32_t rows = (uint32_t)(N - r0 < kRowsCta ? N - r0 : kRowsCta);
+        // asynchronous copies: all in flight at once, without registers
+#pragma unroll 4
+        for (uint32_t e = t; e < rows * La; e += kRowsCta) {
+            const uint32_t r = (e * divA) >> kDivShift;
+            const uint32_t i = e - r * La;
+            copy_limb(sh + r * pitch + i, A + (r0 + r) * sA + i);
         }
-        uint32_t *cr = C + row * sC;
-        const uint32_t Lc = La + Lb;
+#pragma unroll 4
+        for (uint32_t e = t; e < rows * Lb; e += kRowsCta) {
+            const uint32_t r = (e * divB) >> kDivShift;
+            const uint32_t i = e - r * Lb;
+            copy_limb(sh + r * pitch + La + i, B + (r0 + r) * sB + i);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (t < rows) {
+            uint32_t *row = sh + t * pitch;
+            uint32_t b[MB];
 #pragma unroll
-        for (int k = 0; k < MA + MB; ++k)
-            if (k < (int)Lc) cr[k] = o[k];
+            for (int j = 0; j < MB; ++j) b[j] = (j < (int)Lb) ? row[La + j] : 0u;
+            uint32_t e[MB], o[MB];   // o[k] sits at position k + 1
+#pragma unroll
+            for (int k = 0; k < MB; ++k) e[k] = o[k] = 0u;
+            uint64_t cr = 0;
+#pragma unroll 1
+            for (uint32_t i = 0; i < La; i += 2) {
+                const uint32_t a0 = row[i];
+                const uint32_t a1 = (i + 1u < La) ? row[i + 1] : 0u;
+                uint32_t e1[MB], o1[MB], ec, oc;
+                MadChain<MB / 2>::run(a0, b, e, 0u, e1, ec);
+                MadChain<MB / 2>::run(a0, b + 1, o, 0u, o1, oc);
+                // a1: positions 1 + j; odd j on words 2 .. MB + 1 of E
+                uint32_t x[MB], o2[MB], top;
+#pragma unroll
+                for (int k = 0; k < MB - 2; ++k) x[k] = e1[k + 2];
+                x[MB - 2] = ec;
+                x[MB - 1] = 0u;
+                MadChain<MB / 2>::run(a1, b + 1, x, 0u, e, top);   // no carry out: the sum fits
+                MadChain<MB / 2>::run(a1, b, o1, oc, o2, oc);
+                uint64_t s = cr + e1[0];
+                row[i] = (uint32_t)s;
+                s = (s >> 32) + e1[1] + o2[0];
+                if (i + 1u < Lc) row[i + 1] = (uint32_t)s;
+                cr = (s >> 32) + o2[1];
+#pragma unroll
+                for (int k = 0; k < MB - 2; ++k) o[k] = o2[k + 2];
+                o[MB - 2] = oc;
+                o[MB - 1] = 0u;
+            }
+            const uint32_t base = (La + 1u) & ~1u;
+#pragma unroll
+            for (int k = 0; k < MB; ++k) {
+                const uint64_t s = cr + e[k] + (k ? o[k ? k - 1 : 0] : 0u);
+                if (base + k < Lc) row[base + k] = (uint32_t)s;
+                cr = s >> 32;
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t e = t; e < rows * Lc; e += kRowsCta) {
+            const uint32_t r = (e * divC) >> kDivShift;
+            const uint32_t i = e - r * Lc;
+            C[(r0 + r) * sC + i] = sh[r * pitch + i];
+        }
+        __syncthreads();
     }
 }
 
@@ -231,11 +458,12 @@ __global__ void __launch_bounds__(kSchoolThreads) k_school_cols(const uint32_t *
     }
 }
 
-// Thread-per-product size classes.
-template <int MA, int MB>
-static void launch_thread(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t N, uint32_t La,
-                          uint32_t Lb, uint64_t sA, uint64_t sB, uint64_t sC, cudaStream_t st) {
-    k_school_thread<MA, MB><<<grid_for(N, 128, kNumSMs * 32), 128, 0, st>>>(A, B, C, N, La, Lb, sA, sB, sC);
+template <int MB>
+static void launch_rows(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t N, uint32_t La, uint32_t Lb,
+                        uint64_t sA, uint64_t sB, uint64_t sC, cudaStream_t st) {
+    auto div = [](uint32_t d) { return ((1u << kDivShift) + d - 1u) / d; };
+    k_school_rows<MB><<<grid_for(N, kRowsCta, kNumSMs * 32), kRowsCta, 0, st>>>(A, B, C, N, La, Lb, sA, sB, sC,
+                                                                              div(La), div(Lb), div(La + Lb));
     count_launch();
 }
 
@@ -258,14 +486,17 @@ void school_mul(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t N, u
         std::swap(La, Lb);
         std::swap(sA, sB);
     }
-    if (La <= 4u && Lb <= 4u) {
-        launch_thread<4, 4>(A, B, C, N, La, Lb, sA, sB, sC, st);
-    } else if (La <= 8u && Lb <= 8u) {
-        launch_thread<8, 8>(A, B, C, N, La, Lb, sA, sB, sC, st);
-    } else if (La <= 16u && Lb <= 8u) {
-        launch_thread<16, 8>(A, B, C, N, La, Lb, sA, sB, sC, st);
-    } else if (La <= 16u && Lb <= 16u) {
-        launch_thread<16, 16>(A, B, C, N, La, Lb, sA, sB, sC, st);
+    if (La <= 16u) {   // one thread per product; B's registers in steps of two
+        switch ((Lb + 1u) / 2u) {
+            case 1:
+            case 2: launch_rows<4>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            case 3: launch_rows<6>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            case 4: launch_rows<8>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            case 5: launch_rows<10>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            case 6: launch_rows<12>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            case 7: launch_rows<14>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+            default: launch_rows<16>(A, B, C, N, La, Lb, sA, sB, sC, st); break;
+        }
     } else if (La + Lb <= 32u) {
         launch_seg<8>(A, B, C, N, La, Lb, sA, sB, sC, st);
     } else if (La + Lb <= 64u) {
