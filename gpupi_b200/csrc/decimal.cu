@@ -150,11 +150,19 @@ void decimal_rows(const uint32_t *A, char *B, uint32_t N, uint32_t L, uint64_t s
     KernelTimed kt("decimal_leaf", 4.0 * N * L + (double)N * L_dec);
     const unsigned gt = grid_for(N, 128, kNumSMs * 32);
     const unsigned gw = grid_for(N, 4, kNumSMs * 32);
-    if (L <= 8u) k_decimal_thread<8, NATURAL><<<gt, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
-    else if (L <= 16u) k_decimal_thread<16, NATURAL><<<gt, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
-    else if (L <= 32u) k_decimal_thread<32, NATURAL><<<gt, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
-    else if (L <= 64u) k_decimal_thread<64, NATURAL><<<gt, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
-    else if (L <= 256u) k_decimal_warp<8, NATURAL><<<gw, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
+    // One thread per row multiplies all MAXL limbs of its array every round, so
+    // the array is the row's length rounded up to four limbs (the conversion's
+    // leaves are 30 to 62 limbs long): 2^20 rows of 34 limbs to 308 digits took
+    // 974 us in an array of 64, 696 us in one of 36.
+    if (L <= 64u) {
+        switch ((L + 3u) / 4u) {
+#define LEAF(q) \
+    case q: k_decimal_thread<4 * q, NATURAL><<<gt, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB); break;
+            LEAF(1) LEAF(2) LEAF(3) LEAF(4) LEAF(5) LEAF(6) LEAF(7) LEAF(8) LEAF(9) LEAF(10) LEAF(11) LEAF(12)
+            LEAF(13) LEAF(14) LEAF(15) LEAF(16)
+#undef LEAF
+        }
+    } else if (L <= 256u) k_decimal_warp<8, NATURAL><<<gw, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
     else if (L <= 1024u) k_decimal_warp<32, NATURAL><<<gw, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
     else k_decimal_warp<64, NATURAL><<<gw, 128, 0, st>>>(A, B, N, L, sA, L_dec, sB);
     count_launch();
