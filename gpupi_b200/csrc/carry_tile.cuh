@@ -109,16 +109,18 @@ __device__ __forceinline__ void patch_rest(uint32_t *out, TileRange r, bool all)
     }
 }
 
+// rows non-null: a ragged batch, each row's place from its descriptor (tiles
+// above a shorter row's end hold zeros and receive no carry).
 // Cross-tile carry fix-up for rows of at most 32 tiles: one warp per row, one
 // lane per tile.
 template <bool SUB>
 __global__ void carry_fixup_kernel(uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc, uint32_t tiles_per_row,
-                                   uint32_t span, bool aligned, const uint32_t *flags) {
+                                   uint32_t span, bool aligned, const uint32_t *flags, const RaggedRow *rows) {
     const uint32_t lane = lane_id();
     const uint32_t gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t row = gwarp; row < N; row += nwarps) {
-        uint32_t *out = C + row * sC;
+        uint32_t *out = C + (rows ? rows[row].offC : row * sC);
         const uint32_t f = (lane < tiles_per_row) ? flags[(uint64_t)row * tiles_per_row + lane] : 0u;
         const uint32_t gm = __ballot_sync(0xffffffffu, (f & 1u) != 0u);
         const uint32_t pm = __ballot_sync(0xffffffffu, (f & 2u) != 0u);
@@ -149,12 +151,13 @@ template <bool SUB>
 __global__ void __launch_bounds__(kFixThreads) carry_fixup_rows_kernel(uint32_t *C, uint64_t sC, uint32_t Lc,
                                                                        uint32_t tiles_per_row, uint32_t blocks_per_row,
                                                                        uint32_t span, bool aligned,
-                                                                       const uint32_t *flags) {
+                                                                       const uint32_t *flags,
+                                                                       const RaggedRow *rows) {
     __shared__ uint32_t sg[kFixThreads / 32], sp[kFixThreads / 32];
     const uint32_t row = blockIdx.x / blocks_per_row;
     const uint32_t blk = blockIdx.x - row * blocks_per_row;
     const uint32_t *fr = flags + (uint64_t)row * tiles_per_row;
-    uint32_t *out = C + row * sC;
+    uint32_t *out = C + (rows ? rows[row].offC : row * sC);
     // generate / propagate bits of this thread's four tiles of group b
     auto load = [&](uint32_t b, uint32_t &g, uint32_t &p) {
         g = p = 0u;
@@ -200,21 +203,22 @@ __global__ void __launch_bounds__(kFixThreads) carry_fixup_rows_kernel(uint32_t 
 }
 
 inline void launch_carry_fixup(bool sub, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc, uint32_t tiles_per_row,
-                               uint32_t span, bool aligned, const uint32_t *flags, cudaStream_t st) {
+                               uint32_t span, bool aligned, const uint32_t *flags, cudaStream_t st,
+                               const RaggedRow *rows = nullptr) {
     if (tiles_per_row > 32u) {
         const uint32_t bpr = (tiles_per_row + kFixTiles - 1u) / kFixTiles;
         if (sub)
             carry_fixup_rows_kernel<true><<<N * bpr, kFixThreads, 0, st>>>(C, sC, Lc, tiles_per_row, bpr, span, aligned,
-                                                                         flags);
+                                                                         flags, rows);
         else
             carry_fixup_rows_kernel<false><<<N * bpr, kFixThreads, 0, st>>>(C, sC, Lc, tiles_per_row, bpr, span,
-                                                                          aligned, flags);
+                                                                          aligned, flags, rows);
     } else {
         const unsigned grid = grid_for(N, 4, kNumSMs * 8);
         if (sub)
-            carry_fixup_kernel<true><<<grid, 128, 0, st>>>(C, sC, N, Lc, tiles_per_row, span, aligned, flags);
+            carry_fixup_kernel<true><<<grid, 128, 0, st>>>(C, sC, N, Lc, tiles_per_row, span, aligned, flags, rows);
         else
-            carry_fixup_kernel<false><<<grid, 128, 0, st>>>(C, sC, N, Lc, tiles_per_row, span, aligned, flags);
+            carry_fixup_kernel<false><<<grid, 128, 0, st>>>(C, sC, N, Lc, tiles_per_row, span, aligned, flags, rows);
     }
     count_launch();
 }

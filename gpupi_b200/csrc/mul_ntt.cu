@@ -9,6 +9,11 @@
 // inputs (A mod (x^K - c_i))(g^i x), and the M blocks of K coefficients of
 // C = A B follow from C_i = sum_b C_b c_i^b by the inverse Vandermonde
 // matrix of the nodes c_i.
+// Where M has two bits set and its larger part fits one transform (M = 3, 5,
+// 6, ... with K 2^floor(log2 M) <= 2^25), the M K points are split instead into
+// a transform of K1 = K 2^floor(log2 M) points mod x^K1 - 1 and one of the
+// remaining K2 points mod x^K2 - g^K2 (twisted by g^i): with C = C1 +
+// (x^K1 - 1) T, deg T < K2, T = (C2 - C1) / (g^K1 - 1) mod x^K2 - g^K2.
 //
 // Workspace: F[vrow][q][K] residues (vrow = row * M + coset), one such array
 // for A (FA) and one for B (FB; none when B is A, one row when B is
@@ -36,6 +41,8 @@
 
 #include <stdio.h>
 #include <stdlib.h>
+
+#include <mutex>
 #include <vector>
 
 namespace gpupi {
@@ -47,6 +54,19 @@ static const uint32_t kGen[kPrimes] = {Prime<0>::g, Prime<1>::g, Prime<2>::g};
 struct NttParams {
     Tables tab;
 };
+
+// Row `row` of an operand: X + row * sX with Lx limbs, or in a ragged batch
+// the A (side 0) or B (side 1) of its descriptor.
+struct LimbRow {
+    const uint32_t *p;
+    uint32_t L;
+};
+__device__ __forceinline__ LimbRow limb_row(const RaggedRow *rows, int side, const uint32_t *X, uint64_t sX,
+                                            uint32_t Lx, uint64_t row) {
+    if (!rows) return {X + row * sX, Lx};
+    const RaggedRow &d = rows[row];
+    return side ? LimbRow{X + d.offB, d.Lb} : LimbRow{X + d.offA, d.La};
+}
 
 // ---------------------------------------------------------------------------
 // Host modular helpers (table construction, coset matrices)
@@ -101,12 +121,16 @@ struct ColsArgs {
     uint32_t *F;         // workspace of this operand: F[vrow][q][K]
     int log_k, log_s;
     int M;               // cosets per row
+    int coset0;          // the first of them (1 for the second part of a two-part product)
+    int scaled;          // inverse pass: times K^-1 R as well (the row pass leaves products x y R^-1)
     // second operand of a paired forward pass (same shape, same tile)
     const uint32_t *X2;
     uint64_t sX2;
     uint32_t Lx2;
     uint32_t nb2;
     uint32_t *F2;
+    const RaggedRow *rows;   // first pass of a ragged batch: per-row operands (nb, nb2 per row)
+    int side;                // of X; X2 is side 1
 };
 
 // Offset of element j from element 0 in a LO = 0 stage with 2^B-point groups
@@ -117,29 +141,40 @@ __host__ __device__ constexpr uint32_t stage_delta(int j, int B, int log_r) {
 }
 
 // Twist the 16 residues of stage S (the LO = 0 stage: last forward, first
-// inverse) by w_S^(col * bitrev(pos)) or its inverse, E = colsh * bitrev(pos)
-// with colsh = col << shift; with PAIR the same factors twist y as well.
+// inverse) by one * w_S^(col * bitrev(pos)) / R or with the inverse root (one =
+// R for the plain twist, K^-1 R^2 where the product's scale is folded in),
+// E = colsh * bitrev(pos) with colsh = col << shift; with PAIR the same factors
+// twist y as well.
 // For LOG_R >= 4 the column is the same for all 16 residues and
 // bitrev(pos_j) = bitrev(pos_0) + sum over the set bits i of j of
 // bitrev(delta_(2^i)), so the 16 factors are the subset products of w^(E_0)
-// and four D_i = w^(colsh bitrev(delta_(2^i))): five table lookups and
-// fifteen products instead of sixteen scattered lookup pairs.
+// and four D_i = w^(colsh bitrev(delta_(2^i))).  bitrev(delta_(2^i)) is a power
+// of two that doubles as i falls within a group's bits, so D_i = D_(i+1)^2
+// there: two or three table lookups, the squares and fifteen products instead
+// of sixteen scattered lookup pairs.
 template <class S, int LOG_R, int Q, bool PAIR>
 __device__ __forceinline__ void twist16(uint32_t (&x)[16], uint32_t (&y)[16], uint32_t t, uint32_t c0, int shift,
-                                        const uint2 *lo, const uint2 *hi) {
+                                        const uint2 *lo, const uint2 *hi, uint32_t one, bool scaled) {
     if constexpr (LOG_R >= 4) {
         constexpr int B = S::kB;
         static_assert(S::kLO == 0, "twist stage");
         uint32_t pos0, c;
         S::elem(t, 0, pos0, c);
         const uint32_t colsh = (c0 + c) << shift;
+        uint32_t D[4];
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {
+            const uint32_t r = crev(stage_delta(1 << i, B, LOG_R), LOG_R);
+            const uint32_t above = i < 3 ? crev(stage_delta(2 << i, B, LOG_R), LOG_R) : 0u;
+            D[i] = (i < 3 && r == 2u * above) ? norm<Q>(mont<Q>(D[i < 3 ? i + 1 : 3], D[i < 3 ? i + 1 : 3]))
+                                              : root_m<Q>(lo, hi, colsh * r);
+        }
         uint32_t F[16];
-        F[0] = root_m<Q>(lo, hi, colsh * bitrev(pos0, LOG_R));
+        F[0] = mul_root<Q>(one, lo, hi, colsh * bitrev(pos0, LOG_R));
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t D = root_m<Q>(lo, hi, colsh * crev(stage_delta(1 << i, B, LOG_R), LOG_R));
 #pragma unroll
-            for (int k = 0; k < (1 << i); ++k) F[(1 << i) + k] = mont<Q>(F[k], D);   // lazy, < 2p
+            for (int k = 0; k < (1 << i); ++k) F[(1 << i) + k] = mont<Q>(F[k], D[i]);   // lazy, < 2p
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -147,25 +182,75 @@ __device__ __forceinline__ void twist16(uint32_t (&x)[16], uint32_t (&y)[16], ui
             if (PAIR) y[j] = norm<Q>(mont<Q>(y[j], F[j]));
         }
     } else {
-        // short columns: the 16 residues span several columns
+        // short columns: R = 2, 4 or 8 positions of each of 16 / R columns 256
+        // apart; a column's factors are the powers of w^(col << shift), and
+        // consecutive columns differ by w^(256 << shift)
+        static_assert(S::kB == LOG_R && S::kLO == 0, "whole columns in registers");
+        uint32_t pos0, c;
+        S::elem(t, 0, pos0, c);
+        uint32_t A = root_m<Q>(lo, hi, (c0 + c) << shift);
+        const uint32_t step = LOG_R < 4 ? root_m<Q>(lo, hi, 256u << shift) : 0u;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            S::elem(t, j, pos, c);
-            const uint32_t E = ((c0 + c) << shift) * bitrev(pos, LOG_R);
-            x[j] = mul_root<Q>(x[j], lo, hi, E);
-            if (PAIR) y[j] = mul_root<Q>(y[j], lo, hi, E);
+        for (int g = 0; g < (16 >> LOG_R); ++g) {
+            if (g) A = norm<Q>(mont<Q>(A, step));
+            uint32_t F[1 << LOG_R];
+            F[0] = one;
+            F[1] = scaled ? mont<Q>(one, A) : A;
+#pragma unroll
+            for (int k = 2; k < (1 << LOG_R); ++k) F[k] = mont<Q>(F[k - 1], A);   // lazy, < 2p
+#pragma unroll
+            for (int v = 0; v < (1 << LOG_R); ++v) {
+                const uint32_t k = crev((uint32_t)v, LOG_R);
+                const int j = (g << LOG_R) + v;
+                if (k != 0u || scaled) {
+                    x[j] = norm<Q>(mont<Q>(x[j], F[k]));
+                    if (PAIR) y[j] = norm<Q>(mont<Q>(y[j], F[k]));
+                }
+            }
         }
     }
 }
 
-// The 16 first-pass residues of one operand (limbs, folded into coset
-// `coset` and twisted by g^(coset i) when the row is split into cosets).
+// The 16 first-pass residues of one operand: its limbs, or its residues mod
+// x^K - c, c = g^(coset K), twisted by g^(coset i) (coset 0: plain folding
+// mod x^K - 1 when the operand is longer than K).
+//
+// Residue j of a thread sits delta_j above its first one, i_0, and the bits of
+// j add up in delta_j (FirstDelta), so it is g^(coset i_0) sum_b X_(b, j) W[b][j]
+// over the K-limb blocks b, with W[b][j] = c^b g^(coset delta_j) the same for the
+// whole CTA (coset_weights, in shared memory).  The sum of 64-bit products is
+// kept below 2^32 p by reducing its upper word only, and reduced once at the
+// end: per block one wide multiply-add and one reduction instead of a modular
+// product, a sum and their reductions, and no chain of powers.
+template <class First, int LOG_R>
+__device__ __forceinline__ uint32_t first_delta(int bit, int log_cols) {   // of j = 2^bit
+    if constexpr (LOG_R >= 4) {
+        static_assert(First::kB == 4, "one group per thread");
+        return 1u << (First::kLO + log_cols + bit);
+    } else {   // 2^LOG_R positions of each of 16 / 2^LOG_R columns, 256 apart
+        return bit < LOG_R ? 1u << (log_cols + bit) : 256u << (bit - LOG_R);
+    }
+}
+
 template <class First, int LOG_R, int Q>
-__device__ __forceinline__ void load_limbs(const ColsArgs &a, uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx,
-                                           uint32_t nb, uint64_t K, int log_cols, uint32_t c0, uint32_t t,
-                                           int coset, uint32_t cm, const uint32_t *clo, const uint32_t *chi) {
-    if (a.M == 1) {
+__device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int coset, int log_k, int log_cols,
+                                              const uint32_t *clo, const uint32_t *chi) {
+    const uint32_t c = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset << log_k);
+    for (uint32_t e = threadIdx.x; e < 16u * blocks; e += kThreads) {
+        uint32_t w = PrimeC<Q>::r1;
+        for (uint32_t k = 0; k < (e >> 4); ++k) w = norm<Q>(mont<Q>(w, c));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if ((e >> k) & 1u) w = mul_coset<Q, 0>(w, clo, chi, (uint32_t)coset * first_delta<First, LOG_R>(k, log_cols));
+        W[e] = w;
+    }
+}
+
+template <class First, int LOG_R, int Q>
+__device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx, uint32_t nb,
+                                           uint64_t K, int log_cols, uint32_t c0, uint32_t t, int coset,
+                                           const uint32_t *W, uint32_t f) {
+    if (nb == 1u && coset == 0) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             uint32_t pos, c;
@@ -175,48 +260,33 @@ __device__ __forceinline__ void load_limbs(const ColsArgs &a, uint32_t (&x)[16],
         }
         return;
     }
-    // X mod (x^K - c): Horner over the K-limb blocks, top block first, the
-    // 16 loads of a block issued together
+    // two halves of eight residues: their sums and loads fit the registers
 #pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = 0u;
-    for (int blk = (int)nb - 1; blk >= 0; --blk) {
-        uint32_t v[16];
+    for (int h = 0; h < 2; ++h) {
+        uint32_t lo[8], hi[8];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            First::elem(t, j, pos, c);
-            const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c + (uint64_t)blk * K;
-            v[j] = (i < Lx) ? __ldg(xr + i) : 0u;
+        for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0u;
+#pragma unroll 1
+        for (uint32_t blk = 0; blk < nb; ++blk) {
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                uint32_t pos, c;
+                First::elem(t, 8 * h + j, pos, c);
+                const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c + (uint64_t)blk * K;
+                v[j] = (i < Lx) ? __ldg(xr + i) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint64_t s = (uint64_t)v[j] * W[16u * blk + 8u * h + j] + (((uint64_t)hi[j] << 32) | lo[j]);
+                lo[j] = (uint32_t)s;
+                hi[j] = norm<Q>((uint32_t)(s >> 32));   // < p again
+            }
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-            x[j] = add_n<Q>(coset ? norm<Q>(mont<Q>(x[j], cm)) : x[j], reduce_limb<Q>(v[j]));
-    }
-    if (coset) {
-        // twist by g^(coset i).  For LOG_R >= 4 the 16 residues of a thread sit
-        // at i_0 + v 2^(LO + log_cols) (one group), so the factors are
-        // g^(coset i_0) D^v with D = g^(coset 2^(LO + log_cols)), the same for
-        // the whole CTA: two lookup pairs and fifteen products.
-        if constexpr (LOG_R >= 4) {
-            static_assert(First::kB == 4, "one group per thread");
-            uint32_t pos, c;
-            First::elem(t, 0, pos, c);
-            const uint32_t i0 = (uint32_t)(((uint64_t)pos << log_cols) + c0 + c);
-            uint32_t f = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * i0);
-            const uint32_t d = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset << (First::kLO + log_cols));
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                x[j] = norm<Q>(mont<Q>(x[j], f));
-                f = mont<Q>(f, d);   // lazy, < 2p
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                uint32_t pos, c;
-                First::elem(t, j, pos, c);
-                const uint32_t i = (uint32_t)(((uint64_t)pos << log_cols) + c0 + c);
-                x[j] = mul_coset<Q, 0>(x[j], clo, chi, (uint32_t)coset * i);
-            }
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t r = redc<Q>(lo[j], hi[j]);   // < 2p
+            x[8 * h + j] = norm<Q>(mont<Q>(r, f));
         }
     }
 }
@@ -264,15 +334,31 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
     uint32_t x[16], y[16];
     if constexpr (FROM_LIMBS) {
         const uint64_t row = vrow / (uint32_t)a.M;
-        const int coset = (int)(vrow - row * (uint32_t)a.M);
-        const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q);
-        const uint32_t *chi = coset_hi_ptr(P.tab, 0, Q);
-        // coset node c = g^(coset K), Montgomery form
-        const uint32_t cm = (a.M > 1) ? mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset << a.log_k) : 0u;
-        load_limbs<First, LOG_R, Q>(a, x, a.X + row * a.sX, a.Lx, a.nb, K, log_cols, c0, t, coset, cm, clo, chi);
+        const int coset = a.coset0 + (int)(vrow - row * (uint32_t)a.M);
+        const LimbRow X = limb_row(a.rows, a.side, a.X, a.sX, a.Lx, row);
+        LimbRow Y = X;
+        uint32_t nb = a.nb, nb2 = a.nb2;
+        if constexpr (PAIR) Y = limb_row(a.rows, 1, a.X2, a.sX2, a.Lx2, row);
+        if (a.rows) {
+            nb = (uint32_t)((X.L + K - 1) >> a.log_k);
+            nb2 = (uint32_t)((Y.L + K - 1) >> a.log_k);
+        }
+        const uint32_t blocks = PAIR ? max(nb, nb2) : nb;
+        uint32_t f = 0u;    // g^(coset i_0), Montgomery form
+        uint32_t *W = Sm;   // weights in the tile, before its first use
+        if (coset || blocks > 1u) {
+            const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q);
+            const uint32_t *chi = coset_hi_ptr(P.tab, 0, Q);
+            uint32_t pos, c;
+            First::elem(t, 0, pos, c);
+            const uint32_t i0 = (uint32_t)(((uint64_t)pos << log_cols) + c0 + c);
+            f = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * i0);
+            coset_weights<First, LOG_R, Q>(W, blocks, coset, a.log_k, log_cols, clo, chi);
+            __syncthreads();
+        }
+        load_limbs<First, LOG_R, Q>(x, X.p, X.L, nb, K, log_cols, c0, t, coset, W, f);
         if constexpr (PAIR)
-            load_limbs<First, LOG_R, Q>(a, y, a.X2 + row * a.sX2, a.Lx2, a.nb2, K, log_cols, c0, t, coset, cm, clo,
-                                        chi);
+            load_limbs<First, LOG_R, Q>(y, Y.p, Y.L, nb2, K, log_cols, c0, t, coset, W, f);
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -282,11 +368,14 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
             x[j] = F[i];
             if constexpr (PAIR) y[j] = F2[i];
         }
-        if constexpr (INVERSE) twist16<First, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi);
+        if constexpr (INVERSE) {
+            const uint32_t one = a.scaled ? __ldg(P.tab.inv2n + a.log_k * kPrimes + Q) : PrimeC<Q>::r1;
+            twist16<First, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, one, a.scaled != 0);
+        }
     }
-    __syncthreads();   // twiddle table ready
-    run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR>(x, y, Sm, Sm2, t, tw);
-    if constexpr (!INVERSE) twist16<Last, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi);
+    __syncthreads();   // twiddle table ready (and the weights read)
+    run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR>(x, y, Sm, Sm2, t, tw, CtaSync{});
+    if constexpr (!INVERSE) twist16<Last, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, PrimeC<Q>::r1, false);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         uint32_t pos, c;
@@ -322,8 +411,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a)
         cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, 2>(P, a, b, Sm, Sm2, tw);
 }
 
+__device__ __forceinline__ void swap16(uint32_t (&x)[16], uint32_t (&y)[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const uint32_t v = x[j];
+        x[j] = y[j];
+        y[j] = v;
+    }
+}
+
 struct RowsArgs {
-    const uint32_t *A;   // limbs (FROM_LIMBS)
+    const uint32_t *A;   // limbs (whole products of at most 4096 points)
     uint64_t sA;
     uint32_t La;
     const uint32_t *B;
@@ -335,80 +433,64 @@ struct RowsArgs {
     int M;               // cosets per row
     int b_bcast;         // B row 0 serves every row
     int square;          // B is A
+    const RaggedRow *rows;   // whole products of a ragged batch: per-row operands
+    __device__ __forceinline__ LimbRow a_row(uint64_t row) const { return limb_row(rows, 0, A, sA, La, row); }
+    __device__ __forceinline__ LimbRow b_row(uint64_t row) const {
+        return limb_row(rows, 1, B, b_bcast ? 0u : sB, square ? 0u : Lb, row);
+    }
 };
 
-// Fused row pass on C = 2^LOG_C points (T = C/16 threads): forward stages of
-// A then B (A stays in registers while B reuses the shared tile), pointwise
-// product * scale, inverse stages.  The last forward and the first inverse
-// stage share one thread mapping, so the product never leaves registers.
-// The forward twiddle levels are replaced by the inverse ones in the same
-// shared buffer once the forward stages are done.
-template <int LOG_C, bool FROM_LIMBS, int Q>
-__device__ __forceinline__ void rows_body(const NttParams &P, const RowsArgs &a, uint64_t b, uint32_t *Sm,
+// Whole product of C = 2^LOG_C points (512 .. 2048, T = C/16 threads) from
+// limbs: forward stages of A then B (A stays in registers while B reuses the
+// shared tile), pointwise product * C^-1, inverse stages.  The last forward
+// and the first inverse stage share one thread mapping, so the product never
+// leaves registers.  The forward twiddle levels are replaced by the inverse
+// ones in the same shared buffer once the forward stages are done.
+template <int LOG_C, int Q>
+__device__ __forceinline__ void rows_body(const NttParams &P, const RowsArgs &a, uint64_t row, uint32_t *Sm,
                                           uint2 *tw) {
     constexpr int C = 1 << LOG_C;
     constexpr int T = C / 16;
     constexpr int NS = StagePlan<LOG_C>::n;
     using First = typename ExecStage<LOG_C, 0, false, 0>::S;
     using Out = typename ExecStage<LOG_C, 0, true, NS - 1>::S;
-    const uint32_t nseg = 1u << (a.log_k - LOG_C);
-    const uint32_t seg = (uint32_t)(b % nseg);
-    const uint64_t vrow = b / nseg;
-    const uint64_t brow = a.b_bcast ? (vrow % (uint32_t)a.M) : vrow;
-    const uint64_t K = 1ull << a.log_k;
-    const uint32_t scale = __ldg(P.tab.inv2n + a.log_k * kPrimes + Q);
+    const LimbRow A = a.a_row(row), B = a.b_row(row);   // B empty for squares
+    const uint32_t scale = __ldg(P.tab.inv2n + LOG_C * kPrimes + Q);
     const uint2 *levf = level_ptr(P.tab, 0, Q);
     const uint2 *levi = level_ptr(P.tab, 1, Q);
     for (uint32_t e = threadIdx.x; e < C - 1; e += T) tw[e] = __ldg(levf + e);
-    const uint64_t offA = vrow * 3 * K + (uint64_t)Q * K + ((uint64_t)seg << LOG_C);
-    const uint64_t offB = brow * 3 * K + (uint64_t)Q * K + ((uint64_t)seg << LOG_C);
     const uint32_t t = threadIdx.x;
     uint32_t xa[16], xb[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         uint32_t pos, c;
         First::elem(t, j, pos, c);
-        if (FROM_LIMBS) {
-            xa[j] = (pos < a.La) ? reduce_limb<Q>(__ldg(a.A + vrow * a.sA + pos)) : 0u;
-            xb[j] = (!a.square && pos < a.Lb) ? reduce_limb<Q>(__ldg(a.B + brow * a.sB + pos)) : 0u;
-        } else {
-            xa[j] = a.FA[offA + pos];
-            xb[j] = a.square ? 0u : a.FB[offB + pos];
-        }
+        xa[j] = (pos < A.L) ? reduce_limb<Q>(__ldg(A.p + pos)) : 0u;
+        xb[j] = (pos < B.L) ? reduce_limb<Q>(__ldg(B.p + pos)) : 0u;
     }
     __syncthreads();
-    // A then B through one copy of the forward stages (a loop, not two
-    // copies: smaller code for the instruction cache); B waits in xb and
-    // trades places with the transformed A between the passes.  A and B one
-    // after the other: a second tile would cost a CTA per SM.
 #pragma unroll 1
     for (int op = 0; op < (a.square ? 1 : 2); ++op) {
         if (op) {
-            // the tile is free again: every thread has passed the last stage's loads
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const uint32_t v = xa[j];
-                xa[j] = xb[j];
-                xb[j] = v;
-            }
+            __syncthreads();   // A's last hand-off has been read
+            swap16(xa, xb);
         }
-        run_stages<LOG_C, 0, false, Q, 0>(xa, Sm, t, tw);
+        run_stages<LOG_C, 0, false, Q, 0>(xa, Sm, t, tw, CtaSync{});
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         const uint32_t y = a.square ? xa[j] : xb[j];
-        xa[j] = norm<Q>(mont<Q>(mont<Q>(xa[j], y), scale));   // x y K^-1
+        xa[j] = norm<Q>(mont<Q>(mont<Q>(xa[j], y), scale));   // x y C^-1
     }
-    __syncthreads();   // forward twiddles and tile no longer read
+    __syncthreads();   // forward twiddles no longer read
     for (uint32_t e = threadIdx.x; e < C - 1; e += T) tw[e] = __ldg(levi + e);
     __syncthreads();
-    run_stages<LOG_C, 0, true, Q, 0>(xa, Sm, t, tw);
+    run_stages<LOG_C, 0, true, Q, 0>(xa, Sm, t, tw, CtaSync{});
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         uint32_t pos, c;
         Out::elem(t, j, pos, c);
-        a.FA[offA + pos] = xa[j];
+        a.FA[(row * 3 + Q) * C + pos] = xa[j];
     }
 }
 
@@ -417,8 +499,8 @@ constexpr size_t rows_smem_bytes() {   // the padded tile + the twiddle levels
     return (size_t)((1 << LOG_C) + (1 << LOG_C) / 32) * 4u + (size_t)((1 << LOG_C) - 1) * 8u;
 }
 
-template <int LOG_C, bool FROM_LIMBS>
-__global__ void __launch_bounds__((1 << LOG_C) / 16, LOG_C == 12 ? 4 : 1) k_rows_r(NttParams P, RowsArgs a) {
+template <int LOG_C>
+__global__ void __launch_bounds__((1 << LOG_C) / 16) k_rows_r(NttParams P, RowsArgs a) {
     extern __shared__ uint4 rows_smem[];
     constexpr int C = 1 << LOG_C;
     uint32_t *Sm = reinterpret_cast<uint32_t *>(rows_smem);
@@ -426,11 +508,190 @@ __global__ void __launch_bounds__((1 << LOG_C) / 16, LOG_C == 12 ? 4 : 1) k_rows
     uint64_t b;
     const int q = grid_prime(b);
     if (q == 0)
-        rows_body<LOG_C, FROM_LIMBS, 0>(P, a, b, Sm, tw);
+        rows_body<LOG_C, 0>(P, a, b, Sm, tw);
     else if (q == 1)
-        rows_body<LOG_C, FROM_LIMBS, 1>(P, a, b, Sm, tw);
+        rows_body<LOG_C, 1>(P, a, b, Sm, tw);
     else
-        rows_body<LOG_C, FROM_LIMBS, 2>(P, a, b, Sm, tw);
+        rows_body<LOG_C, 2>(P, a, b, Sm, tw);
+}
+
+// ---------------------------------------------------------------------------
+// 4096-point row passes: persistent CTAs of two 256-thread groups.  A group
+// has a tile and a named barrier of its own; the CTA's forward and inverse
+// twiddle levels (2 x 32 KiB) stay in shared memory while its groups work
+// through a contiguous run of segments (at most two or three runs: one per
+// prime).  With one CTA per segment the tables were loaded afresh for every
+// product, two to four times, each with two barriers: as much shared-memory
+// traffic as the transforms' own hand-offs.
+// ---------------------------------------------------------------------------
+constexpr int kRowLog = 12;
+constexpr int kRowPoints = 1 << kRowLog;
+constexpr int kRowGroups = 2;
+constexpr int kRowThreads = 256 * kRowGroups;
+constexpr int kRowCtas = 2;   // per SM: 64 registers a thread, 2 x 97 KiB shared memory
+static_assert(kRowPoints == 16 * 256, "a group holds one segment in registers");
+
+constexpr size_t row_smem_bytes() { return (size_t)kRowGroups * kTilePad * 4u + 2u * kRowPoints * 8u; }
+inline unsigned row_grid(uint64_t segments) {   // all primes' segments
+    return (unsigned)std::min<uint64_t>((segments + kRowGroups - 1) / kRowGroups, (uint64_t)kNumSMs * kRowCtas);
+}
+
+struct RowShared {
+    uint32_t *tile;   // this group's
+    uint2 *twf, *twi;
+};
+
+__device__ __forceinline__ RowShared row_shared(uint4 *smem) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(smem);
+    RowShared s;
+    s.twf = reinterpret_cast<uint2 *>(w);
+    s.twi = s.twf + kRowPoints;
+    s.tile = reinterpret_cast<uint32_t *>(s.twi + kRowPoints) + (threadIdx.x >> 8) * kTilePad;
+    return s;
+}
+
+__device__ __forceinline__ void row_tables(const NttParams &P, int q, const RowShared &s) {
+    __syncthreads();   // the previous prime's stages are done
+    const uint2 *f = level_ptr(P.tab, 0, q), *i = level_ptr(P.tab, 1, q);
+    for (uint32_t e = threadIdx.x; e < (uint32_t)kRowPoints - 1u; e += kRowThreads) {
+        s.twf[e] = __ldg(f + e);
+        s.twi[e] = __ldg(i + e);
+    }
+    __syncthreads();
+}
+
+// This CTA's share [first, last) of prime q's `segs` segments (2^30 segments
+// would be 12 TB of residues).
+__device__ __forceinline__ bool row_share(uint32_t segs, uint32_t q, uint32_t &first, uint32_t &last) {
+    const uint64_t total = (uint64_t)segs * kPrimes;
+    const uint32_t lo = (uint32_t)(total * blockIdx.x / gridDim.x), hi = (uint32_t)(total * (blockIdx.x + 1u) / gridDim.x);
+    const uint32_t a = segs * q;
+    first = max(lo, a) - a;
+    last = min(hi, a + segs);
+    if (last <= a + first) return false;
+    last -= a;
+    return true;
+}
+
+// 16 KiB segments are 16-byte aligned (K >= 4096 residues from the workspace's
+// base): bulk prefetch to L2 by the copy engine.
+__device__ __forceinline__ void prefetch_segment(const uint32_t *p) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((uint32_t)kRowPoints * 4u) : "memory");
+}
+
+using RowFirst = typename ExecStage<kRowLog, 0, false, 0>::S;
+using RowOut = typename ExecStage<kRowLog, 0, true, StagePlan<kRowLog>::n - 1>::S;
+using RowLast = typename ExecStage<kRowLog, 0, false, StagePlan<kRowLog>::n - 1>::S;
+static_assert(RowLast::kLO == 0 && RowLast::kB == 4, "last row stage holds 16 consecutive positions");
+
+// Fused row pass of one product: forward stages of A then B through one copy
+// of the code (a loop: smaller code for the instruction cache), pointwise
+// product / R, inverse stages; the first inverse column pass multiplies by
+// K^-1 R with its twist.  The loads between the transforms come from L2, where
+// the group's next segment is sent while it transforms the one before.
+// One 2^28-point product (196,608 segments): 6.88 -> 5.45 ms.
+template <int Q>
+__device__ __forceinline__ void rows_run(const RowsArgs &a, uint32_t first, uint32_t last, const RowShared &s) {
+    const uint32_t t = threadIdx.x & 255u;
+    const uint32_t grp = threadIdx.x >> 8;
+    const GroupSync sync{1u + grp};
+    const int log_seg = a.log_k - kRowLog;
+    auto offset = [&](uint32_t vrow, uint32_t b) {
+        return ((uint64_t)(((vrow * 3u + Q) << log_seg) + (b & ((1u << log_seg) - 1u)))) << kRowLog;
+    };
+    auto prefetch = [&](uint32_t b) {
+        if (t < 2u && b < last) {
+            const uint32_t v = b >> log_seg;
+            if (t == 0u)
+                prefetch_segment(a.FA + offset(v, b));
+            else if (!a.square)
+                prefetch_segment(a.FB + offset(a.b_bcast ? v % (uint32_t)a.M : v, b));
+        }
+    };
+    prefetch(first + grp);
+#pragma unroll 1
+    for (uint32_t b = first + grp; b < last; b += kRowGroups) {
+        const uint32_t vrow = b >> log_seg;
+        const uint32_t brow = a.b_bcast ? (vrow % (uint32_t)a.M) : vrow;
+        uint32_t *FA = a.FA + offset(vrow, b) + t;
+        prefetch(b + kRowGroups);
+        uint32_t k[16], x[16];   // the transform of A, the operand at hand
+#pragma unroll 1
+        for (int op = a.square ? 1 : 0; op < 2; ++op) {
+            const uint32_t *X = op && !a.square ? a.FB + offset(brow, b) + t : FA;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = X[256u * j];
+            if (op && !a.square) sync();   // A's last hand-off has been read
+            run_stages<kRowLog, 0, false, Q, 0>(x, s.tile, t, s.twf, sync);
+            if (!op || a.square) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) k[j] = x[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = norm<Q>(mont<Q>(k[j], x[j]));
+        run_stages<kRowLog, 0, true, Q, 0>(x, s.tile, t, s.twi, sync);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) FA[256u * j] = x[j];
+    }
+}
+
+// Whole products of 4096 points, from limbs: both operands' limbs are loaded
+// at once (their HBM latency overlaps), the product is scaled by K^-1 here.
+// 1024 products of 2001 x 1903 limbs: 125 -> 108 us.
+template <int Q>
+__device__ __forceinline__ void rows_limbs_run(const NttParams &P, const RowsArgs &a, uint32_t first, uint32_t last,
+                                               const RowShared &s) {
+    const uint32_t t = threadIdx.x & 255u;
+    const uint32_t grp = threadIdx.x >> 8;
+    const GroupSync sync{1u + grp};
+#pragma unroll 1
+    for (uint32_t row = first + grp; row < last; row += kRowGroups) {
+        const LimbRow A = a.a_row(row), B = a.b_row(row);   // B empty for squares
+        uint32_t xa[16], xb[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const uint32_t pos = t + 256u * j;
+            xa[j] = (pos < A.L) ? reduce_limb<Q>(__ldg(A.p + pos)) : 0u;
+            xb[j] = (pos < B.L) ? reduce_limb<Q>(__ldg(B.p + pos)) : 0u;
+        }
+#pragma unroll 1
+        for (int op = 0; op < (a.square ? 1 : 2); ++op) {
+            if (op) {
+                sync();   // A's last hand-off has been read
+                swap16(xa, xb);
+            }
+            run_stages<kRowLog, 0, false, Q, 0>(xa, s.tile, t, s.twf, sync);
+        }
+        const uint32_t scale = __ldg(P.tab.inv2n + kRowLog * kPrimes + Q);
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            xa[j] = norm<Q>(mont<Q>(mont<Q>(xa[j], a.square ? xa[j] : xb[j]), scale));
+        run_stages<kRowLog, 0, true, Q, 0>(xa, s.tile, t, s.twi, sync);
+        uint32_t *out = a.FA + (((uint64_t)row * 3u + Q) << kRowLog) + t;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) out[256u * j] = xa[j];
+    }
+}
+
+template <bool LIMBS, int Q>
+__device__ __forceinline__ void rows_prime(const NttParams &P, const RowsArgs &a, uint32_t segs, const RowShared &s) {
+    uint32_t first, last;
+    if (!row_share(segs, Q, first, last)) return;
+    row_tables(P, Q, s);
+    if constexpr (LIMBS)
+        rows_limbs_run<Q>(P, a, first, last, s);
+    else
+        rows_run<Q>(a, first, last, s);
+}
+
+template <bool LIMBS>
+__global__ void __launch_bounds__(kRowThreads, kRowCtas) k_rows(NttParams P, RowsArgs a, uint32_t segs) {
+    extern __shared__ uint4 rows_smem[];
+    const RowShared s = row_shared(rows_smem);
+    rows_prime<LIMBS, 0>(P, a, segs, s);
+    rows_prime<LIMBS, 1>(P, a, segs, s);
+    rows_prime<LIMBS, 2>(P, a, segs, s);
 }
 
 // Whole product of K <= 2^8 points per CTA (one prime, one row), radix-2
@@ -442,7 +703,7 @@ __device__ __forceinline__ void rows_small_body(const NttParams &P, const RowsAr
                                                 uint32_t *SA, uint32_t *SB, uint2 *twf, uint2 *twi) {
     const int log_k = a.log_k;
     const uint32_t K = 1u << log_k;
-    const uint64_t brow = a.b_bcast ? 0u : row;
+    const LimbRow A = a.a_row(row), B = a.b_row(row);
     const uint32_t scale = __ldg(P.tab.inv2n + log_k * kPrimes + Q);
     const uint2 *levf = level_ptr(P.tab, 0, Q) + (K / 2 - 1u);   // top level: w_K^e, e < K/2
     const uint2 *levi = level_ptr(P.tab, 1, Q) + (K / 2 - 1u);
@@ -451,8 +712,8 @@ __device__ __forceinline__ void rows_small_body(const NttParams &P, const RowsAr
         twi[e] = __ldg(levi + e);
     }
     for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
-        SA[i] = (i < a.La) ? reduce_limb<Q>(__ldg(a.A + row * a.sA + i)) : 0u;
-        SB[i] = (!a.square && i < a.Lb) ? reduce_limb<Q>(__ldg(a.B + brow * a.sB + i)) : 0u;
+        SA[i] = (i < A.L) ? reduce_limb<Q>(__ldg(A.p + i)) : 0u;
+        SB[i] = (i < B.L) ? reduce_limb<Q>(__ldg(B.p + i)) : 0u;
     }
     __syncthreads();
     tile_transform<Q, false>(SA, log_k, 0, twf);
@@ -488,15 +749,14 @@ __global__ void __launch_bounds__(128) k_rows_small(NttParams P, RowsArgs a) {
 // positions 16t .. 16t + 15) go through the shared tile to the first
 // stage's order (thread t holds t + 256 j), so the spectrum is stored with
 // coalesced 128-byte warp accesses.  k_rows_inv loads T pairs of spectra in
-// that order, forms sum_t X_t Y_t K^-1 (mod p), moves the result back to
+// that order, forms sum_t X_t Y_t / R (mod p), moves the result back to
 // the last stage's order through the tile and runs the inverse stages,
 // leaving the segment in the order the inverse column passes expect, as the
 // fused k_rows_r does.  So a transform computed once serves every product
 // it takes part in, and a sum of products costs one inverse transform.
 // ---------------------------------------------------------------------------
-constexpr int kSplitLogC = 12;
-using SplitLast = ExecStage<kSplitLogC, 0, false, StagePlan<kSplitLogC>::n - 1>::S;
-static_assert(SplitLast::kLO == 0 && SplitLast::kB == 4, "last row stage holds 16 consecutive positions");
+constexpr int kSplitLogC = kRowLog;
+using SplitLast = RowLast;
 
 struct RowsFwdArgs {
     uint32_t *F0;   // spectra [vrow][q][K], column passes done
@@ -523,7 +783,7 @@ __device__ __forceinline__ void rows_fwd_body(const RowsFwdArgs &a, uint64_t b, 
             x[j] = F[pos];
         }
         __syncthreads();   // twiddles loaded; the previous operand has left the tile
-        run_stages<kSplitLogC, 0, false, Q, 0>(x, Sm, t, tw);
+        run_stages<kSplitLogC, 0, false, Q, 0>(x, Sm, t, tw, CtaSync{});
         SplitLast::store(Sm, x, t);   // every thread passed the last stage's tile loads
         __syncthreads();
 #pragma unroll
@@ -571,7 +831,6 @@ __device__ __forceinline__ void rows_inv_body(const NttParams &P, const RowsInvA
     const uint64_t K = 1ull << a.log_k;
     const uint64_t off = (b / nseg) * 3 * K + (uint64_t)Q * K + ((uint64_t)(b % nseg) << kSplitLogC);
     const uint32_t t = threadIdx.x;
-    const uint32_t scale = __ldg(P.tab.inv2n + a.log_k * kPrimes + Q);
     using First = typename ExecStage<kSplitLogC, 0, false, 0>::S;
     uint32_t x[16];
 #pragma unroll
@@ -586,13 +845,10 @@ __device__ __forceinline__ void rows_inv_body(const NttParams &P, const RowsInvA
             x[j] = add_n<Q>(x[j], norm<Q>(mont<Q>(__ldg(X + pos), __ldg(Y + pos))));
         }
     }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = norm<Q>(mont<Q>(x[j], scale));   // sum K^-1
     First::store(Sm, x, t);
     __syncthreads();   // tile written, inverse twiddles loaded
     SplitLast::load(Sm, x, t);
-    __syncthreads();
-    run_stages<kSplitLogC, 0, true, Q, 0>(x, Sm, t, tw);
+    run_stages<kSplitLogC, 0, true, Q, 0>(x, Sm, t, tw, CtaSync{});
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         uint32_t pos, c;
@@ -620,135 +876,113 @@ __global__ void __launch_bounds__((1 << kSplitLogC) / 16, 4) k_rows_inv(NttParam
             rows_inv_body<TERMS, 1>(P, a, s, Sm, tw);
         else
             rows_inv_body<TERMS, 2>(P, a, s, Sm, tw);
-        __syncthreads();   // the tile is free for the next segment
+        // the next segment's first store goes where this thread's last loads came from
     }
 }
 
 // One merge level's four row products in one pass (the tuned form's level):
-// from the column-transformed segments of P_e, P_o, R_o, Q_o, Q_e, R_e the
-// CTA forms P' = P_e P_o, R2 = P_e R_o, Q' = Q_e Q_o, R1 = R_e Q_o (each
-// x K^-1) and runs their inverse row stages, writing them over P_o, R_o, Q_e
-// and R_e: six forward and four inverse row transforms, the kept operand
-// (P_e, then Q_o) and one product in registers, no spectrum stored.  With
-// Fpo null (the tree's root) P' is not formed: five and three.
+// from the column-transformed segments of P_e, P_o, R_o, Q_o, Q_e, R_e a group
+// forms P' = P_e P_o, R2 = P_e R_o, Q' = Q_e Q_o, R1 = R_e Q_o (each / R; the
+// first inverse column pass scales them by K^-1 R) and runs their inverse row
+// stages, writing them over P_o, R_o, Q_e and R_e: six forward and four
+// inverse row transforms, the kept operand (P_e, then Q_o) and one product in
+// registers, no spectrum stored.  With Fpo null (the tree's root) P' is not
+// formed: five and three.
 struct RowsLevelArgs {
     uint32_t *Fpe, *Fpo, *Fro, *Fqo, *Fqe, *Fre;
     int log_k;
 };
 
 template <int Q>
-__device__ __forceinline__ void rows_level_body(const NttParams &P, const RowsLevelArgs &a, uint64_t b,
-                                                uint32_t *Sm, uint2 *tw) {
-    constexpr int C = 1 << kSplitLogC;
-    constexpr int T = C / 16;
-    using First = typename ExecStage<kSplitLogC, 0, false, 0>::S;
-    using Out = typename ExecStage<kSplitLogC, 0, true, StagePlan<kSplitLogC>::n - 1>::S;
-    const uint32_t nseg = 1u << (a.log_k - kSplitLogC);
-    const uint64_t K = 1ull << a.log_k;
-    const uint64_t off = (b / nseg) * 3 * K + (uint64_t)Q * K + ((uint64_t)(b % nseg) << kSplitLogC);
-    const uint32_t t = threadIdx.x;
-    const uint32_t scale = __ldg(P.tab.inv2n + a.log_k * kPrimes + Q);
-    const uint2 *levf = level_ptr(P.tab, 0, Q);
-    const uint2 *levi = level_ptr(P.tab, 1, Q);
-    auto load = [&](const uint32_t *F, uint32_t (&x)[16]) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            First::elem(t, j, pos, c);
-            x[j] = __ldg(F + off + pos);
+__device__ __forceinline__ void level_run(const RowsLevelArgs &a, uint32_t first, uint32_t last, const RowShared &s) {
+    const uint32_t t = threadIdx.x & 255u;
+    const uint32_t grp = threadIdx.x >> 8;
+    const GroupSync sync{1u + grp};
+    const int log_seg = a.log_k - kRowLog;
+    auto offset = [&](uint32_t b) {
+        return ((uint64_t)((((b >> log_seg) * 3u + Q) << log_seg) + (b & ((1u << log_seg) - 1u)))) << kRowLog;
+    };
+    // The next segment's six operand segments go to L2 while this one is
+    // transformed, so the loads between its transforms find them there.
+    auto prefetch = [&](uint32_t b) {
+        if (t < 6u && b < last) {
+            const uint32_t *F = t == 0u ? a.Fpe : t == 1u ? a.Fpo : t == 2u ? a.Fro : t == 3u ? a.Fqo
+                                                                          : t == 4u ? a.Fqe : a.Fre;
+            if (F) prefetch_segment(F + offset(b));
         }
     };
-    auto store = [&](uint32_t *F, const uint32_t (&x)[16]) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            Out::elem(t, j, pos, c);
-            F[off + pos] = x[j];
-        }
-    };
-    auto table = [&](const uint2 *lev) {
-        __syncthreads();   // the previous stages have left the tile and the table
-        for (uint32_t e = t; e < C - 1; e += T) tw[e] = __ldg(lev + e);
-        __syncthreads();
-    };
-    // The six operand segments (16 KiB each, contiguous, 16-byte aligned) go
-    // to L2 by bulk prefetch (the copy engine, no registers or shared memory)
-    // as the CTA starts, so the later loads, issued between transforms, find
-    // them in L2 instead of waiting on HBM.
-    if (t < 6u) {
-        const uint32_t *F = t == 0u ? a.Fpe : t == 1u ? a.Fpo : t == 2u ? a.Fro : t == 3u ? a.Fqo
-                                                                      : t == 4u ? a.Fqe : a.Fre;
-        if (F)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(F + off), "r"((uint32_t)C * 4u)
-                         : "memory");
-    }
+    prefetch(first + grp);
     // One copy of the forward and one of the inverse stages per prime, run
     // in loops (the ten transforms written out would not fit the instruction
     // cache).  Per half: the kept operand F_keep, then F0 (its product with
-    // F_keep waits in F0's own segment: word j of thread t at j * T + t,
+    // F_keep waits in F0's own segment: word j of thread t at j * 256 + t,
     // coalesced; every thread has loaded F0 before the next barrier and reads
     // back only its own words; the segment is rewritten by the product's
-    // inverse anyway, and keeping the product out of shared memory leaves
-    // room for a fourth CTA per SM), then F1 (its product stays in registers);
-    // the inverse of F_keep F1 goes to F1, that of the held product to F0.
+    // inverse anyway), then F1 (its product stays in registers); the inverse of
+    // F_keep F1 goes to F1, that of the held product to F0.
     // F0 null (the tree's root, uniform over the grid): no P' product.
-    uint32_t k[16], x[16];
 #pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t *Fk = h ? a.Fqo : a.Fpe;
-        uint32_t *F0 = h ? a.Fqe : a.Fpo;
-        uint32_t *F1 = h ? a.Fre : a.Fro;
-        uint32_t *held = F0 ? F0 + off : nullptr;
-        table(levf);
+    for (uint32_t b = first + grp; b < last; b += kRowGroups) {
+        const uint64_t off = offset(b) + t;
+        prefetch(b + kRowGroups);
+        uint32_t k[16], x[16];
 #pragma unroll 1
-        for (int step = 0; step < 3; ++step) {
-            const uint32_t *src = step == 0 ? Fk : (step == 1 ? F0 : F1);
-            if (!src) continue;
-            if (step) __syncthreads();   // the previous transform has left the tile
-            load(src, x);
-            run_stages<kSplitLogC, 0, false, Q, 0>(x, Sm, t, tw);
-            if (step == 0) {
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t *Fk = h ? a.Fqo : a.Fpe;
+            uint32_t *F0 = h ? a.Fqe : a.Fpo;
+            uint32_t *F1 = h ? a.Fre : a.Fro;
+#pragma unroll 1
+            for (int step = 0; step < 3; ++step) {
+                const uint32_t *src = step == 0 ? Fk : (step == 1 ? F0 : F1);
+                if (!src) continue;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) k[j] = x[j];
-            } else if (step == 1) {
+                for (int j = 0; j < 16; ++j) x[j] = __ldg(src + off + 256u * j);
+                if (step) sync();   // the previous forward transform's last hand-off has been read
+                run_stages<kRowLog, 0, false, Q, 0>(x, s.tile, t, s.twf, sync);
+                if (step == 0) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) held[j * T + t] = norm<Q>(mont<Q>(mont<Q>(k[j], x[j]), scale));
-            } else {
+                    for (int j = 0; j < 16; ++j) k[j] = x[j];
+                } else if (step == 1) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] = norm<Q>(mont<Q>(mont<Q>(k[j], x[j]), scale));
+                    for (int j = 0; j < 16; ++j) F0[off + 256u * j] = norm<Q>(mont<Q>(k[j], x[j]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) x[j] = norm<Q>(mont<Q>(k[j], x[j]));
+                }
             }
-        }
-        table(levi);
 #pragma unroll 1
-        for (int step = 0; step < 2; ++step) {
-            if (step == 1) {
-                if (!held) break;
-                __syncthreads();
+            for (int step = 0; step < 2; ++step) {
+                uint32_t *dst = step ? F0 : F1;
+                if (step == 1) {
+                    if (!F0) break;
+                    sync();   // the previous inverse transform's last hand-off has been read
 #pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] = held[j * T + t];
+                    for (int j = 0; j < 16; ++j) x[j] = F0[off + 256u * j];
+                }
+                run_stages<kRowLog, 0, true, Q, 0>(x, s.tile, t, s.twi, sync);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) dst[off + 256u * j] = x[j];
             }
-            run_stages<kSplitLogC, 0, true, Q, 0>(x, Sm, t, tw);
-            store(step ? F0 : F1, x);
         }
     }
 }
 
-// the padded tile and the twiddle levels
-constexpr size_t rows_level_smem_bytes() { return rows_smem_bytes<kSplitLogC>(); }
-
-__global__ void __launch_bounds__((1 << kSplitLogC) / 16, 4) k_rows_level(NttParams P, RowsLevelArgs a) {
+__global__ void __launch_bounds__(kRowThreads, kRowCtas) k_rows_level(NttParams P, RowsLevelArgs a, uint32_t segs) {
     extern __shared__ uint4 rows_smem[];
-    constexpr int C = 1 << kSplitLogC;
-    uint32_t *Sm = reinterpret_cast<uint32_t *>(rows_smem);
-    uint2 *tw = reinterpret_cast<uint2 *>(Sm + C + C / 32);
-    uint64_t b;
-    const int q = grid_prime(b);
-    if (q == 0)
-        rows_level_body<0>(P, a, b, Sm, tw);
-    else if (q == 1)
-        rows_level_body<1>(P, a, b, Sm, tw);
-    else
-        rows_level_body<2>(P, a, b, Sm, tw);
+    const RowShared s = row_shared(rows_smem);
+    uint32_t first, last;
+    if (row_share(segs, 0, first, last)) {
+        row_tables(P, 0, s);
+        level_run<0>(a, first, last, s);
+    }
+    if (row_share(segs, 1, first, last)) {
+        row_tables(P, 1, s);
+        level_run<1>(a, first, last, s);
+    }
+    if (row_share(segs, 2, first, last)) {
+        row_tables(P, 2, s);
+        level_run<2>(a, first, last, s);
+    }
 }
 
 // Coset recombination.  Row r holds z_i[j] = C_i[j] g^(ij) for cosets i < M;
@@ -760,22 +994,34 @@ struct CombineArgs {
     uint32_t vinv[kPrimes][kMaxCosets][kMaxCosets];   // Montgomery form, [q][b][i]
 };
 
+// The untwist factors of position j are the powers of g^-j (one table lookup);
+// each output sums 64-bit products, reducing the upper word only after each
+// (as the first pass's coset sums) and fully once.  Eight cosets of 2^25
+// points: 3.22 -> 1.85 ms.
 template <int M, int Q>
 __device__ __forceinline__ void combine_body(const NttParams &P, const CombineArgs &a, uint64_t row, uint32_t j) {
     const uint64_t K = 1ull << a.log_k;
     uint32_t *F0 = a.F + row * M * 3 * K + (uint64_t)Q * K + j;
-    const uint32_t *clo = coset_lo_ptr(P.tab, 1, Q);
-    const uint32_t *chi = coset_hi_ptr(P.tab, 1, Q);
+    const uint32_t h = mul_coset<Q, 1>(PrimeC<Q>::r1, coset_lo_ptr(P.tab, 1, Q), coset_hi_ptr(P.tab, 1, Q), j);
     uint32_t u[M];
-    u[0] = F0[0];
 #pragma unroll
-    for (int i = 1; i < M; ++i) u[i] = mul_coset<Q, 1>(F0[(uint64_t)i * 3 * K], clo, chi, (uint32_t)i * j);
+    for (int i = 0; i < M; ++i) u[i] = F0[(uint64_t)i * 3 * K];
+    uint32_t f = h;   // g^(-ij), < 2p
+#pragma unroll
+    for (int i = 1; i < M; ++i) {
+        u[i] = norm<Q>(mont<Q>(u[i], f));
+        if (i + 1 < M) f = mont<Q>(f, h);
+    }
 #pragma unroll
     for (int b = 0; b < M; ++b) {
-        uint32_t acc = 0u;
+        uint32_t lo = 0u, hi = 0u;   // hi < p after each term
 #pragma unroll
-        for (int i = 0; i < M; ++i) acc = add_n<Q>(acc, norm<Q>(mont<Q>(u[i], a.vinv[Q][b][i])));
-        F0[(uint64_t)b * 3 * K] = acc;
+        for (int i = 0; i < M; ++i) {
+            const uint64_t s = (uint64_t)u[i] * a.vinv[Q][b][i] + (((uint64_t)hi << 32) | lo);
+            lo = (uint32_t)s;
+            hi = norm<Q>((uint32_t)(s >> 32));
+        }
+        F0[(uint64_t)b * 3 * K] = norm<Q>(redc<Q>(lo, hi));
     }
 }
 
@@ -792,6 +1038,57 @@ __global__ void __launch_bounds__(kThreads) k_combine(NttParams P, CombineArgs a
         combine_body<M, 1>(P, a, row, j);
     else
         combine_body<M, 2>(P, a, row, j);
+}
+
+// Two-part recombination: C1 mod x^K1 - 1 in F1[row][q][K1], z[j] = C2[j] g^j
+// in F2[row][q][K2] -> T in F2 and C's coefficients below K2, C1 - T, in F1
+// (those from K2 to K1 are C1's own).  C1 folds mod x^K2 - c, c = g^K2, as
+// sum_b C1[j + b K2] c^b; w[q][b] holds -c^b / (g^K1 - 1) and w[q][parts] its
+// reciprocal factor 1 / (g^K1 - 1), Montgomery form.  One read of both parts and
+// one write of 2 K2 points: HBM-bound, against M^2 products per M points for
+// equal cosets (five cosets of 2^13 points x 96 rows: 42 us, this 20 us).
+constexpr int kMaxFold = 16;   // K1 / K2
+struct Combine2Args {
+    uint32_t *F1, *F2;
+    int log_k1, log_k2;
+    uint32_t w[kPrimes][kMaxFold + 1];
+};
+
+template <int Q>
+__device__ __forceinline__ void combine2_body(const NttParams &P, const Combine2Args &a, uint64_t row, uint32_t j) {
+    const uint64_t base = row * 3 + Q;
+    uint32_t *F1 = a.F1 + (base << a.log_k1) + j;
+    uint32_t *F2 = a.F2 + (base << a.log_k2) + j;
+    const uint32_t parts = 1u << (a.log_k1 - a.log_k2);
+    const uint32_t first = F1[0];
+    const uint32_t h = mul_coset<Q, 1>(PrimeC<Q>::r1, coset_lo_ptr(P.tab, 1, Q), coset_hi_ptr(P.tab, 1, Q), j);
+    uint64_t s = (uint64_t)norm<Q>(mont<Q>(F2[0], h)) * a.w[Q][parts];
+    uint32_t lo = (uint32_t)s, hi = (uint32_t)(s >> 32);   // hi < p, after each term
+    uint32_t v = first;
+    for (uint32_t b = 0; b < parts; ++b) {
+        const uint32_t next = b + 1u < parts ? F1[(uint64_t)(b + 1u) << a.log_k2] : 0u;
+        s = (uint64_t)v * a.w[Q][b] + (((uint64_t)hi << 32) | lo);
+        lo = (uint32_t)s;
+        hi = norm<Q>((uint32_t)(s >> 32));
+        v = next;
+    }
+    const uint32_t T = norm<Q>(redc<Q>(lo, hi));
+    F2[0] = T;
+    F1[0] = sub_n<Q>(first, T);
+}
+
+__global__ void __launch_bounds__(kThreads) k_combine2(NttParams P, Combine2Args a) {
+    uint64_t rest;
+    const int q = grid_prime(rest);
+    const uint32_t jblocks = (1u << a.log_k2) / kThreads;
+    const uint64_t row = rest / jblocks;
+    const uint32_t j = (uint32_t)(rest - row * jblocks) * kThreads + threadIdx.x;
+    if (q == 0)
+        combine2_body<0>(P, a, row, j);
+    else if (q == 1)
+        combine2_body<1>(P, a, row, j);
+    else
+        combine2_body<2>(P, a, row, j);
 }
 
 // Garner: residues (r0, r1, r2) -> coefficient < p0 p1 p2 as 3 limbs.
@@ -822,6 +1119,8 @@ struct CrtArgs {
     const uint32_t *F;
     int log_k;
     int M;
+    const uint32_t *F2;   // coefficients from K on, of a two-part product, or null
+    int log_k2;
     uint32_t *C;
     uint64_t sC;
     uint32_t Lc;
@@ -834,6 +1133,7 @@ struct CrtArgs {
     uint64_t sD;
     uint32_t Ld;
     uint32_t dshift;
+    const RaggedRow *rows;   // ragged batch: each row's output place and length
 };
 
 // Adds limbs base .. base + kCrtV - 1 of (D << dshift) to the chunk sum S
@@ -858,18 +1158,33 @@ __device__ __forceinline__ void crt_add_shifted(const CrtArgs &a, const uint32_t
     }
 }
 
-// Coefficient n of a row lives in block b = n / K at F0[(b * 3 + q) * K + n mod K];
-// there are ncoef = L_c - 1 <= M K of them (the top limb only receives carries).
-__device__ __forceinline__ void crt_chunk(const uint32_t *F0, int log_k, uint32_t ncoef, int64_t base,
-                                          uint32_t (&S)[kCrtV + 3]) {
+// A row's coefficients: n < M K lives in block b = n / K at F[(b * 3 + q) * K +
+// n mod K], those of a two-part product from K on at F2[q * K2 + n - K].  There
+// are ncoef = L_c - 1 of them (the top limb only receives carries).
+struct CrtRow {
+    const uint32_t *F, *F2;
+    int log_k, log_k2;
+    uint32_t ncoef;
+    // the word of prime 0 for coefficient n, and the distance to the next prime's
+    __device__ __forceinline__ const uint32_t *at(uint64_t n, uint64_t &next) const {
+        if (F2 && (n >> log_k)) {
+            next = 1ull << log_k2;
+            return F2 + (n - (1ull << log_k));
+        }
+        next = 1ull << log_k;
+        return F + (((n >> log_k) * 3) << log_k) + (n & (next - 1ull));
+    }
+};
+
+__device__ __forceinline__ void crt_chunk(const CrtRow &r, int64_t base, uint32_t (&S)[kCrtV + 3]) {
     uint32_t c[kCrtV][3];
-    const uint64_t K = 1ull << log_k;
-    if (base >= 0 && base + kCrtV <= (int64_t)ncoef && K >= (uint64_t)kCrtV) {
+    uint64_t K;
+    if (base >= 0 && base + kCrtV <= (int64_t)r.ncoef && (1 << r.log_k) >= kCrtV) {
         // the chunk lies in one block: one 128-bit load per prime (K and base are multiples of 4)
-        const uint64_t off = (((uint64_t)base >> log_k) * 3) * K + ((uint64_t)base & (K - 1));
-        const uint4 r0 = *reinterpret_cast<const uint4 *>(F0 + off);
-        const uint4 r1 = *reinterpret_cast<const uint4 *>(F0 + off + K);
-        const uint4 r2 = *reinterpret_cast<const uint4 *>(F0 + off + 2 * K);
+        const uint32_t *f = r.at((uint64_t)base, K);
+        const uint4 r0 = *reinterpret_cast<const uint4 *>(f);
+        const uint4 r1 = *reinterpret_cast<const uint4 *>(f + K);
+        const uint4 r2 = *reinterpret_cast<const uint4 *>(f + 2 * K);
         garner(r0.x, r1.x, r2.x, c[0]);
         garner(r0.y, r1.y, r2.y, c[1]);
         garner(r0.z, r1.z, r2.z, c[2]);
@@ -880,9 +1195,9 @@ __device__ __forceinline__ void crt_chunk(const uint32_t *F0, int log_k, uint32_
 #pragma unroll
     for (int v = 0; v < kCrtV; ++v) {
         const int64_t i = base + v;
-        if (i >= 0 && i < (int64_t)ncoef) {
-            const uint64_t off = (((uint64_t)i >> log_k) * 3) * K + ((uint64_t)i & (K - 1));
-            garner(F0[off], F0[off + K], F0[off + 2 * K], c[v]);
+        if (i >= 0 && i < (int64_t)r.ncoef) {
+            const uint32_t *f = r.at((uint64_t)i, K);
+            garner(f[0], f[K], f[2 * K], c[v]);
         } else {
             c[v][0] = c[v][1] = c[v][2] = 0u;
         }
@@ -896,13 +1211,14 @@ __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
     const uint32_t tile = blockIdx.x;
     const uint64_t row = tile / a.tiles;
     const uint32_t t = tile - (uint32_t)row * a.tiles;
-    const uint64_t K = 1ull << a.log_k;
-    const uint32_t *F0 = a.F + row * (uint64_t)a.M * 3 * K;
+    const uint32_t Lc = a.rows ? a.rows[row].La + a.rows[row].Lb : a.Lc;
+    const CrtRow cr{a.F + ((row * (uint64_t)a.M * 3) << a.log_k), a.F2 ? a.F2 + ((row * 3) << a.log_k2) : nullptr,
+                    a.log_k, a.log_k2, a.rows ? Lc - 1u : a.ncoef};
     const int64_t base = (int64_t)t * kCrtSpan + threadIdx.x * kCrtV;
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     uint32_t S[kCrtV + 3];
     const uint32_t *Dr = a.D ? a.D + row * a.sD : nullptr;
-    crt_chunk(F0, a.log_k, a.ncoef, base, S);
+    crt_chunk(cr, base, S);
     if (Dr) crt_add_shifted(a, Dr, base, S);
     // words of the previous chunk's sum that land in this chunk: from the
     // previous lane, from the previous warp's last lane, and for the tile's
@@ -918,7 +1234,7 @@ __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
     }
     if (threadIdx.x == 0) {
         uint32_t Sp[kCrtV + 3];
-        crt_chunk(F0, a.log_k, a.ncoef, base - kCrtV, Sp);
+        crt_chunk(cr, base - kCrtV, Sp);
         if (Dr) crt_add_shifted(a, Dr, base - kCrtV, Sp);
         H[0] = Sp[kCrtV];
         H[1] = Sp[kCrtV + 1];
@@ -934,13 +1250,13 @@ __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
     const uint32_t g = chunk_add_spill<kCrtV>(S, H, X);
     bool p = true;
 #pragma unroll
-    for (int v = 0; v < kCrtV; ++v) p = p && (X[v] == 0xffffffffu) && (base + v < (int64_t)a.Lc);
+    for (int v = 0; v < kCrtV; ++v) p = p && (X[v] == 0xffffffffu) && (base + v < (int64_t)Lc);
     const BlockCarry bc = block_resolve<kThreads / 32>(g != 0u, p, sg, sp);
     chunk_increment<kCrtV>(X, bc.cin);
-    uint32_t *out = a.C + row * a.sC;
+    uint32_t *out = a.C + (a.rows ? a.rows[row].offC : row * a.sC);
 #pragma unroll
     for (int v = 0; v < kCrtV; ++v)
-        if (base + v < (int64_t)a.Lc) out[base + v] = X[v];
+        if (base + v < (int64_t)Lc) out[base + v] = X[v];
     if (a.tiles > 1u && threadIdx.x == 0) a.flags[tile] = bc.G | (bc.P << 1);
 }
 
@@ -971,7 +1287,12 @@ static Shape shape_for(uint32_t La, uint32_t Lb);
 // tuned splitting tree's spectra keep the built-in rule.
 static Shape shape_tuned(uint32_t La, uint32_t Lb) {
     int lk = 0, M = 0;
-    if (ntt_shape_override((uint64_t)La + Lb - 1u, &lk, &M)) return Shape{lk, M};
+    const uint64_t need = (uint64_t)La + Lb - 1u;
+    if (ntt_shape_override(need, &lk, &M)) return Shape{lk, M};
+    // just above one transform: 2^25 points and a second part instead of two
+    // cosets of 2^25
+    if (need > (1ull << kMaxLog) && need <= (5ull << (kMaxLog - 2))) return Shape{kMaxLog - 2, 5};
+    if (need > (1ull << kMaxLog) && need <= (3ull << (kMaxLog - 1))) return Shape{kMaxLog - 1, 3};
     return shape_for(La, Lb);
 }
 
@@ -1055,32 +1376,49 @@ static void launch_cols_r(bool from_limbs, bool inverse, bool pair, int log_r, c
             cols_r_dispatch<false, false, true>(log_r, blocks, P, a, st);
         else
             cols_r_dispatch<false, false, false>(log_r, blocks, P, a, st);
+    } else if (pair) {
+        cols_r_dispatch<false, true, true>(log_r, blocks, P, a, st);
     } else {
         cols_r_dispatch<false, true, false>(log_r, blocks, P, a, st);
     }
     count_launch();
 }
 
-template <int LOG_C, bool FL>
+template <int LOG_C>
 static void rows_launch(unsigned blocks, const NttParams &P, const RowsArgs &r, cudaStream_t st) {
     constexpr size_t smem = rows_smem_bytes<LOG_C>();
-    static bool attr = false;
-    if (!attr) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_rows_r<LOG_C, FL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
-    k_rows_r<LOG_C, FL><<<blocks, (1 << LOG_C) / 16, smem, st>>>(P, r);
+    static_assert(smem <= 48 * 1024, "within the default limit");
+    k_rows_r<LOG_C><<<blocks, (1 << LOG_C) / 16, smem, st>>>(P, r);
 }
 
-template <bool FL>
-static void rows_r_dispatch(int log_c, unsigned blocks, const NttParams &P, const RowsArgs &r, cudaStream_t st) {
-    switch (log_c) {
-        case 9: rows_launch<9, FL>(blocks, P, r, st); break;
-        case 10: rows_launch<10, FL>(blocks, P, r, st); break;
-        case 11: rows_launch<11, FL>(blocks, P, r, st); break;
-        default: rows_launch<12, FL>(blocks, P, r, st); break;
+// Shared-memory limit of the 4096-point row kernels, set once per device.
+static void row_attr() {
+    static std::mutex mu;
+    static uint64_t done = 0;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> l(mu);
+    if ((done >> (dev & 63)) & 1u) return;
+    cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    cudaFuncSetAttribute(k_rows_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    done |= 1ull << (dev & 63);
+}
+
+// Row pass of `segs` segments per prime.
+static void launch_rows(int log_k, bool limbs, uint32_t segs, const NttParams &P, const RowsArgs &r, cudaStream_t st) {
+    switch (limbs ? log_k : kRowLog) {
+        case 9: rows_launch<9>((unsigned)(segs * kPrimes), P, r, st); break;
+        case 10: rows_launch<10>((unsigned)(segs * kPrimes), P, r, st); break;
+        case 11: rows_launch<11>((unsigned)(segs * kPrimes), P, r, st); break;
+        default:
+            row_attr();
+            if (limbs)
+                k_rows<true><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r, segs);
+            else
+                k_rows<false><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r, segs);
     }
+    count_launch();
 }
 
 // Inverse of the Vandermonde matrix V[i][b] = c_i^b (c_i = g^(i 2^log_k)) mod
@@ -1180,8 +1518,109 @@ size_t workspace_bytes(uint32_t N, uint32_t La, uint32_t Lb) {
     return (size_t)(2ull * N * s.M * 3 * K * 4 + N * tiles * 4 + 256);
 }
 
+// The two-part split of a shape of M K points (M with two bits set, the larger
+// part within one transform).
+static bool two_parts(Shape s, int *log_k1, int *log_k2) {
+    if (s.log_k <= 12 || __builtin_popcount((unsigned)s.M) != 2) return false;
+    const int hi = 31 - __builtin_clz((unsigned)s.M), lo = __builtin_ctz((unsigned)s.M);
+    if (s.log_k + hi > kMaxLog || (1 << (hi - lo)) > kMaxFold) return false;
+    *log_k1 = s.log_k + hi;
+    *log_k2 = s.log_k + lo;
+    return true;
+}
+
+// Inverse column passes of vrows virtual rows of F, innermost first (the
+// first one scales by K^-1 R); of F2 as well, in the same launches where the
+// columns are long enough to pair.
+static void inverse_columns(const NttParams &P, int log_k, int M, uint64_t vrows, uint32_t *F, uint32_t *F2,
+                            cudaStream_t st) {
+    int passes[2];
+    const int npass = column_passes(log_k, passes);
+    const bool pair = F2 && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
+    for (int op = 0; op < (F2 && !pair ? 2 : 1); ++op) {
+        int log_s = kRowLog;
+        for (int ps = npass - 1; ps >= 0; --ps) {
+            log_s += passes[ps];
+            ColsArgs a{nullptr, 0, 0, 0, op ? F2 : F, log_k, log_s, M, 0, ps == npass - 1, nullptr, 0, 0, 0,
+                       pair ? F2 : nullptr, nullptr, 0};
+            launch_cols_r(false, true, pair, passes[ps], P, a, vrows, st);
+        }
+    }
+}
+
+struct Operands {
+    const uint32_t *A, *B;
+    uint32_t N, La, Lb;
+    uint64_t sA, sB;
+    bool square, bcast;   // B is A / one row of B serves every row
+    const RaggedRow *rows;
+};
+
+// Residues of the products mod x^K - g^(iK) twisted by g^(ij), for the cosets
+// i = coset0 .. coset0 + M - 1 of each row, left in FA.
+static void cyclic_product(const NttParams &P, const Operands &o, int log_k, int M, int coset0, uint32_t *FA,
+                           uint32_t *FB, cudaStream_t st) {
+    const uint64_t K = 1ull << log_k;
+    const uint64_t VR = (uint64_t)o.N * M;   // virtual rows (row, coset)
+    int passes[2];
+    const int npass = column_passes(log_k, passes);
+    // forward column passes: A and B together (one launch per pass) unless
+    // B is A or a broadcast row
+    const bool pair = !o.square && !o.bcast && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
+    for (int op = 0; op < (pair || o.square ? 1 : 2); ++op) {
+        const uint32_t *X = op == 0 ? o.A : o.B;
+        const uint64_t sX = op == 0 ? o.sA : o.sB;
+        const uint32_t Lx = op == 0 ? o.La : o.Lb;
+        uint32_t *F = op == 0 ? FA : FB;
+        const uint64_t vrows = (op == 1 && o.bcast) ? (uint64_t)M : VR;
+        const uint32_t nb = (uint32_t)((Lx + K - 1) / K);
+        const uint32_t nb2 = (uint32_t)((o.Lb + K - 1) / K);
+        int log_s = log_k;
+        for (int ps = 0; ps < npass; ++ps) {
+            ColsArgs a{X, sX, Lx, nb, F, log_k, log_s, M, coset0, 0, pair ? o.B : nullptr, o.sB, o.Lb, nb2,
+                       pair ? FB : nullptr, o.rows, op};
+            launch_cols_r(ps == 0, false, pair, passes[ps], P, a, vrows, st);
+            log_s -= passes[ps];
+        }
+    }
+    RowsArgs r{o.A, o.sA, o.La, o.B, o.sB, o.Lb, FA, FB, log_k, M, o.bcast ? 1 : 0, o.square ? 1 : 0, nullptr};
+    {
+        KernelTimed kt("ntt_rows_fused", 12.0 * (double)K * ((o.square ? 2.0 : 3.0) * (double)VR));
+        launch_rows(log_k, false, (uint32_t)(VR * (K >> kRowLog)), P, r, st);
+    }
+    inverse_columns(P, log_k, M, VR, FA, nullptr, st);
+}
+
+static void launch_combine2(const NttParams &P, uint32_t *F1, int log_k1, uint32_t *F2, int log_k2, uint32_t N,
+                            cudaStream_t st) {
+    Combine2Args a{};
+    a.F1 = F1;
+    a.F2 = F2;
+    a.log_k1 = log_k1;
+    a.log_k2 = log_k2;
+    const int parts = 1 << (log_k1 - log_k2);
+    for (int q = 0; q < kPrimes; ++q) {
+        const uint32_t p = kP[q];
+        const uint32_t c = h_pow(kGen[q], 1ull << log_k2, p);
+        const uint32_t d = h_inv((h_pow(c, (uint64_t)parts, p) + p - 1u) % p, p);   // g^K1 != 1: p - 1 is no power of 2
+        uint32_t x = p - d;
+        for (int b = 0; b < parts; ++b) {
+            a.w[q][b] = h_mont(x, p);
+            x = h_mul(x, c, p);
+        }
+        a.w[q][parts] = h_mont(d, p);
+    }
+    KernelTimed kt("ntt_coset_combine", 12.0 * N * ((double)(1ull << log_k1) + 3.0 * (double)(1ull << log_k2)));
+    k_combine2<<<(unsigned)((uint64_t)N * kPrimes * ((1ull << log_k2) / kThreads)), kThreads, 0, st>>>(P, a);
+    count_launch();
+}
+
+// rows (device) non-null: a ragged batch, each product's operands and output
+// from its descriptor; L_a + L_b is then the largest product's length (the
+// workspace's too) and the strides are unused.
 static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t *ws,
-                uint32_t N, uint32_t La, uint32_t Lb, uint64_t sA, uint64_t sB, uint64_t sC) {
+                uint32_t N, uint32_t La, uint32_t Lb, uint64_t sA, uint64_t sB, uint64_t sC,
+                const RaggedRow *rows = nullptr) {
     cudaStream_t st = current_stream();
     const uint32_t Lc = La + Lb;
     if (N == 0u || Lc == 0u) return;
@@ -1198,73 +1637,47 @@ static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32
         fprintf(stderr, "gpupi_b200: min(L_a, L_b) = %u exceeds the three-prime CRT capacity\n", La < Lb ? La : Lb);
         return;
     }
-    const int log_k = s.log_k, M = s.M;
-    const uint64_t K = 1ull << log_k;
-    const uint64_t VR = (uint64_t)N * M;   // virtual rows (row, coset)
-    const bool square = (A == B && La == Lb && sA == sB);
-    const bool bcast = (!square && sB == 0u && N > 1u);
-    uint32_t *FA = ws;
-    uint32_t *FB = square ? FA : ws + VR * 3 * K;
+    const bool square = (!rows && A == B && La == Lb && sA == sB);
+    const bool bcast = (!rows && !square && sB == 0u && N > 1u);
+    const uint64_t points = (uint64_t)N * s.M * 3 << s.log_k;
     const uint64_t tiles = ((uint64_t)Lc + kCrtSpan - 1) / kCrtSpan;
-    uint32_t *flags = ws + 2ull * VR * 3 * K;
-
-    if (log_k <= 12) {
-        RowsArgs r{A, sA, La, B, sB, Lb, FA, FB, log_k, 1, bcast ? 1 : 0, square ? 1 : 0};
-        KernelTimed kt("ntt_local", 4.0 * N * ((double)La + (square ? 0 : Lb)) + 12.0 * K * N);
-        if (log_k >= 9)
-            rows_r_dispatch<true>(log_k, (unsigned)(N * kPrimes), P, r, st);
-        else
+    uint32_t *FA = ws;
+    uint32_t *FB = square ? FA : ws + points;
+    uint32_t *flags = ws + 2ull * points;
+    CrtArgs c{FA, s.log_k, s.M, nullptr, 0, C, sC, Lc, (uint32_t)tiles, flags, Lc - 1u, nullptr, 0, 0, 0, rows};
+    int log_k2 = 0;
+    if (s.log_k <= 12) {
+        RowsArgs r{A, sA, La, B, sB, Lb, FA, FB, s.log_k, 1, bcast ? 1 : 0, square ? 1 : 0, rows};
+        KernelTimed kt("ntt_local", 4.0 * N * ((double)La + (square ? 0 : Lb)) + 12.0 * (double)(1ull << s.log_k) * N);
+        if (s.log_k >= 9) {
+            launch_rows(s.log_k, true, N, P, r, st);
+        } else {
             k_rows_small<<<(unsigned)(N * kPrimes), 128, 0, st>>>(P, r);
-        count_launch();
-    } else {
-        const int log_c = 12;
-        int passes[2];
-        const int npass = column_passes(log_k, passes);
-        // forward column passes: A and B together (one launch per pass) unless
-        // B is A or a broadcast row
-        const bool pair = !square && !bcast && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
-        for (int op = 0; op < (pair || square ? 1 : 2); ++op) {
-            const uint32_t *X = op == 0 ? A : B;
-            const uint64_t sX = op == 0 ? sA : sB;
-            const uint32_t Lx = op == 0 ? La : Lb;
-            uint32_t *F = op == 0 ? FA : FB;
-            const uint64_t vrows = (op == 1 && bcast) ? (uint64_t)M : VR;
-            const uint32_t nb = (uint32_t)((Lx + K - 1) / K);
-            const uint32_t nb2 = (uint32_t)((Lb + K - 1) / K);
-            int log_s = log_k;
-            for (int ps = 0; ps < npass; ++ps) {
-                ColsArgs a{X, sX, Lx, nb, F, log_k, log_s, M, pair ? B : nullptr, sB, Lb, nb2, pair ? FB : nullptr};
-                launch_cols_r(ps == 0, false, pair, passes[ps], P, a, vrows, st);
-                log_s -= passes[ps];
-            }
-        }
-        RowsArgs r{A, sA, La, B, sB, Lb, FA, FB, log_k, M, bcast ? 1 : 0, square ? 1 : 0};
-        const uint64_t blocks = VR * kPrimes * (K >> log_c);
-        {
-            KernelTimed kt("ntt_rows_fused", 12.0 * (double)K * ((square ? 2.0 : 3.0) * (double)VR));
-            rows_r_dispatch<false>(log_c, (unsigned)blocks, P, r, st);
             count_launch();
         }
-        // inverse column passes, innermost first
-        int log_s = log_c;
-        for (int ps = npass - 1; ps >= 0; --ps) {
-            log_s += passes[ps];
-            ColsArgs a{nullptr, 0, 0, 0, FA, log_k, log_s, M, nullptr, 0, 0, 0, nullptr};
-            launch_cols_r(false, true, false, passes[ps], P, a, VR, st);
-        }
-        if (M > 1) {
-            CombineArgs c{};
-            c.F = FA;
-            c.log_k = log_k;
-            coset_matrix(M, log_k, c.vinv);
-            launch_combine(M, P, c, N, st);
+    } else if (two_parts(s, &c.log_k, &log_k2)) {
+        const uint64_t p1 = (uint64_t)N * 3 << c.log_k;
+        c.M = 1;
+        c.F2 = FA + p1;
+        c.log_k2 = log_k2;
+        const Operands o{A, B, N, La, Lb, sA, sB, square, bcast, rows};
+        cyclic_product(P, o, c.log_k, 1, 0, FA, FB, st);
+        cyclic_product(P, o, log_k2, 1, 1, FA + p1, square ? FA + p1 : FB + p1, st);
+        launch_combine2(P, FA, c.log_k, FA + p1, log_k2, N, st);
+    } else {
+        cyclic_product(P, Operands{A, B, N, La, Lb, sA, sB, square, bcast, rows}, s.log_k, s.M, 0, FA, FB, st);
+        if (s.M > 1) {
+            CombineArgs m{};
+            m.F = FA;
+            m.log_k = s.log_k;
+            coset_matrix(s.M, s.log_k, m.vinv);
+            launch_combine(s.M, P, m, N, st);
         }
     }
-    CrtArgs c{FA, log_k, M, C, sC, Lc, (uint32_t)tiles, flags, Lc - 1u, nullptr, 0, 0, 0};
     KernelTimed kt("ntt_crt_carry", 12.0 * (double)Lc * N + 4.0 * (double)Lc * N);
     k_crt<<<(unsigned)(N * tiles), kThreads, 0, st>>>(c);
     count_launch();
-    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, false, flags, st);
+    if (tiles > 1) launch_carry_fixup(false, C, sC, N, Lc, (uint32_t)tiles, kCrtSpan, false, flags, st, rows);
 }
 
 // ---------------------------------------------------------------------------
@@ -1279,8 +1692,6 @@ static void rows_split_attr() {
         cudaFuncSetAttribute(k_rows_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         cudaFuncSetAttribute(k_rows_inv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         cudaFuncSetAttribute(k_rows_inv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        cudaFuncSetAttribute(k_rows_level, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)rows_level_smem_bytes());
         done = true;
     }
 }
@@ -1303,7 +1714,7 @@ static void spectrum_forward(const NttParams &P, Shape s, uint32_t N, const uint
         const uint32_t nb2 = (uint32_t)((Ly + K - 1) / K);
         int log_s = log_k;
         for (int ps = 0; ps < npass; ++ps) {
-            ColsArgs a{Z, sZ, Lz, nb, F, log_k, log_s, M, pair ? Y : nullptr, sY, Ly, nb2, pair ? FY : nullptr};
+            ColsArgs a{Z, sZ, Lz, nb, F, log_k, log_s, M, 0, 0, pair ? Y : nullptr, sY, Ly, nb2, pair ? FY : nullptr, nullptr, 0};
             launch_cols_r(ps == 0, false, pair, passes[ps], P, a, VR, st);
             log_s -= passes[ps];
         }
@@ -1319,7 +1730,8 @@ static void spectrum_forward(const NttParams &P, Shape s, uint32_t N, const uint
 
 static void spectrum_inverse(const NttParams &P, Shape s, uint32_t N, int terms, const uint32_t *const *X,
                              const uint32_t *const *Y, uint32_t *Fout, uint32_t *C, uint64_t sC, uint32_t Lc,
-                             uint32_t *flags, cudaStream_t st, bool rows, const SpectrumAddend *add) {
+                             uint32_t *flags, cudaStream_t st, bool rows, bool cols,
+                             const SpectrumAddend *add) {
     const int log_k = s.log_k, M = s.M;
     const uint64_t K = 1ull << log_k;
     const uint64_t VR = (uint64_t)N * M;
@@ -1343,14 +1755,7 @@ static void spectrum_inverse(const NttParams &P, Shape s, uint32_t N, int terms,
         count_launch();
     }
     }
-    int passes[2];
-    const int npass = column_passes(log_k, passes);
-    int log_s = kSplitLogC;
-    for (int ps = npass - 1; ps >= 0; --ps) {
-        log_s += passes[ps];
-        ColsArgs a{nullptr, 0, 0, 0, Fout, log_k, log_s, M, nullptr, 0, 0, 0, nullptr};
-        launch_cols_r(false, true, false, passes[ps], P, a, VR, st);
-    }
+    if (cols) inverse_columns(P, log_k, M, VR, Fout, nullptr, st);
     if (M > 1) {
         CombineArgs c{};
         c.F = Fout;
@@ -1359,7 +1764,7 @@ static void spectrum_inverse(const NttParams &P, Shape s, uint32_t N, int terms,
         launch_combine(M, P, c, N, st);
     }
     const uint64_t tiles = ((uint64_t)Lc + kCrtSpan - 1) / kCrtSpan;
-    CrtArgs c{Fout, log_k, M, C, sC, Lc, (uint32_t)tiles, flags, Lc - 1u, nullptr, 0, 0, 0};
+    CrtArgs c{Fout, log_k, M, nullptr, 0, C, sC, Lc, (uint32_t)tiles, flags, Lc - 1u, nullptr, 0, 0, 0, nullptr};
     if (add) {
         c.ncoef = add->ncoef;
         c.D = add->D;
@@ -1455,6 +1860,14 @@ size_t batch_mul_ntt_workspace_size(uint32_t N, uint32_t L_a, uint32_t L_b) {
 
 namespace gpupi {
 
+// A ragged batch of products of at most Lc limbs in all at one transform
+// shape, the largest product's (Lc >= 2); workspace: batch_mul_ntt_workspace_size(N,
+// Lc - 1, 1).
+void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint32_t *A, const uint32_t *B,
+                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc) {
+    ntt::mul(ntt::make_params(tables), A, B, C, ws, N, Lc - 1u, 1u, 0, 0, 0, rows);
+}
+
 // Transform shape a product of La x Lb limbs gets (tune table or built-in rule).
 void ntt_shape_of(uint32_t La, uint32_t Lb, int *log_k, int *M) {
     const ntt::Shape s = ntt::shape_tuned(La, Lb);
@@ -1497,23 +1910,29 @@ void spectrum_forward(const NTTPrecomputedTables &tables, SpectrumShape s, uint3
 
 void spectrum_inverse(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, int terms,
                       const uint32_t *const *X, const uint32_t *const *Y, uint32_t *Fout, uint32_t *C, uint64_t sC,
-                      uint32_t Lc, uint32_t *flags, bool rows, const SpectrumAddend *add) {
+                      uint32_t Lc, uint32_t *flags, bool rows, bool cols, const SpectrumAddend *add) {
     const ntt::NttParams P = ntt::make_params(tables);
     ntt::spectrum_inverse(P, ntt::Shape{s.log_k, s.M}, N, terms, X, Y, Fout, C, sC, Lc, flags, current_stream(),
-                          rows, add);
+                          rows, cols, add);
+}
+
+void spectrum_inverse_columns(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *F0,
+                              uint32_t *F1) {
+    ntt::inverse_columns(ntt::make_params(tables), s.log_k, s.M, (uint64_t)N * s.M, F0, F1, current_stream());
 }
 
 void spectrum_level_rows(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *Fpe,
                          uint32_t *Fpo, uint32_t *Fro, uint32_t *Fqo, uint32_t *Fqe, uint32_t *Fre) {
     const ntt::NttParams P = ntt::make_params(tables);
     cudaStream_t st = current_stream();
-    ntt::rows_split_attr();
+    ntt::row_attr();
     const uint64_t VR = (uint64_t)N * s.M;
-    const unsigned blocks = (unsigned)(VR * ntt::kPrimes * ((1ull << s.log_k) >> ntt::kSplitLogC));
+    const uint64_t segs = VR * ((1ull << s.log_k) >> ntt::kRowLog);
     ntt::RowsLevelArgs a{Fpe, Fpo, Fro, Fqo, Fqe, Fre, s.log_k};
     // six residues read and four written per point, or five and three
     KernelTimed kt("ntt_rows_level", (Fpo ? 40.0 : 32.0) * (double)(1ull << s.log_k) * (double)VR * ntt::kPrimes);
-    ntt::k_rows_level<<<blocks, (1 << ntt::kSplitLogC) / 16, ntt::rows_level_smem_bytes(), st>>>(P, a);
+    ntt::k_rows_level<<<ntt::row_grid(segs * ntt::kPrimes), ntt::kRowThreads, ntt::row_smem_bytes(), st>>>(
+        P, a, (uint32_t)segs);
     count_launch();
 }
 

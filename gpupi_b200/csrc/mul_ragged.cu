@@ -2,24 +2,26 @@
 // lengths, one call (no counterpart in the reference, whose batches share one
 // L_a / L_b; gpupi's callers with uneven pairs issue one call per pair).
 //
-// Products are bucketed on the host:
+// Products are bucketed on the host; every kernel reads its products' offsets
+// and lengths from one descriptor array, so operands and products are read and
+// written in place:
 //   * L_a = 0 or L_b = 0: the L_a + L_b output limbs are zeroed;
 //   * products the tune table gives to the CUDA-core schoolbook: one
-//     k_school_cols launch reading every product's offsets and lengths from a
-//     descriptor array; those it gives to the tensor-core schoolbook: one
-//     k_mul_tc launch over their descriptors;
-//   * otherwise by transform size 2^ceil(log2(L_a + L_b - 1)): each bucket's
-//     operands are gathered into zero-padded rows (longer operand first: the
-//     product commutes), multiplied as one uniform batch (mul_tuned), and
-//     the L_a + L_b limbs of each row scattered to the product's output.
-//     Zeros above an operand leave the low L_a + L_b limbs of the product
-//     unchanged.
-// Device scratch comes from the stream's scratch arena.
+//     k_school_cols launch; those it gives to the tensor-core schoolbook:
+//     up to four k_mul_tc launches by length, longest products first (a
+//     launch's shared memory is sized for its largest product, so short ones
+//     in a launch of their own get several CTAs per SM);
+//   * otherwise by transform size (powers of two up to 2^13 points, quarters of
+//     an octave above): one NTT batch per bucket at its largest product's shape.
+// 4096 products of 8..4096 limbs per operand: gathering the NTT products into
+// padded rows and scattering them back took 104 of 503 us and gave rows of
+// 3073..4096 limbs transforms of twice the size.
+// The descriptors' device memory comes from the stream's scratch arena.
 #include "common.cuh"
 #include "batch_arith.h"
+#include "batch_mul_ntt.h"
 
 #include <algorithm>
-#include <map>
 #include <vector>
 
 namespace gpupi {
@@ -29,36 +31,13 @@ void school_mul_ragged(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32
 cudaError_t tc_mul_ragged(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t n, const RaggedRow *rows,
                           uint32_t maxQ, uint32_t maxN, uint64_t limbs_moved);
 void tc_shape(uint32_t La, uint32_t Lb, uint32_t *Q, uint32_t *N);
-int mul_kind(uint32_t La, uint32_t Lb, bool public_api);
-cudaError_t mul_tuned(BatchMPContext *ctx, BatchMPArray A, BatchMPArray B, BatchMPArray C);
+void mul_kinds(uint32_t n, const uint32_t *La, const uint32_t *Lb, uint8_t *kinds);
+void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint32_t *A, const uint32_t *B,
+                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc);
+const NTTPrecomputedTables &context_tables(const BatchMPContext *ctx);
+const void *context_workspace(const BatchMPContext *ctx);
 
 namespace {
-
-// dst row r (stride limbs) = src[off_r .. off_r + len_r) zero-padded; which
-// selects the A (0) or B (1) side of the descriptor.
-__global__ void __launch_bounds__(256) k_gather_rows(uint32_t *__restrict__ dst, uint64_t stride,
-                                                     const uint32_t *__restrict__ src,
-                                                     const RaggedRow *__restrict__ rows, uint32_t n, int which) {
-    for (uint32_t r = blockIdx.x; r < n; r += gridDim.x) {
-        const RaggedRow d = rows[r];
-        const uint64_t off = which ? d.offB : d.offA;
-        const uint32_t len = which ? d.Lb : d.La;
-        uint32_t *out = dst + r * stride;
-        for (uint64_t i = threadIdx.x; i < stride; i += blockDim.x) out[i] = (i < len) ? src[off + i] : 0u;
-    }
-}
-
-// C[offC_r .. + La_r + Lb_r) = the low limbs of padded product row r.
-__global__ void __launch_bounds__(256) k_scatter_rows(uint32_t *__restrict__ C, const uint32_t *__restrict__ src,
-                                                      uint64_t stride, const RaggedRow *__restrict__ rows,
-                                                      uint32_t n) {
-    for (uint32_t r = blockIdx.x; r < n; r += gridDim.x) {
-        const RaggedRow d = rows[r];
-        const uint32_t *in = src + r * stride;
-        const uint64_t len = (uint64_t)d.La + d.Lb;
-        for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) C[d.offC + i] = in[i];
-    }
-}
 
 __global__ void __launch_bounds__(256) k_zero_rows(uint32_t *__restrict__ C, const RaggedRow *__restrict__ rows,
                                                    uint32_t n) {
@@ -69,72 +48,24 @@ __global__ void __launch_bounds__(256) k_zero_rows(uint32_t *__restrict__ C, con
     }
 }
 
-int ceil_log2_u64(uint64_t x) {
-    int k = 0;
-    while ((1ull << k) < x) ++k;
-    return k;
-}
-
 unsigned grid_rows(uint32_t n) { return (unsigned)std::max<uint32_t>(1u, std::min<uint32_t>(n, kNumSMs * 16)); }
 
-// One NTT bucket: rows with La >= Lb come first (sources A, B), rows with
-// La < Lb follow with their operands exchanged (sources B, A).
-cudaError_t ntt_bucket(BatchMPContext *ctx, const std::vector<RaggedRow> &rows, const uint32_t *A,
-                       const uint32_t *B, uint32_t *C, cudaStream_t st) {
-    std::vector<RaggedRow> ord;
-    ord.reserve(rows.size());
-    for (const RaggedRow &d : rows)
-        if (d.La >= d.Lb) ord.push_back(d);
-    const uint32_t nk = (uint32_t)ord.size();
-    for (RaggedRow d : rows)
-        if (d.La < d.Lb) {
-            std::swap(d.La, d.Lb);
-            std::swap(d.offA, d.offB);
-            ord.push_back(d);
-        }
-    const uint32_t n = (uint32_t)ord.size(), ns = n - nk;
-    uint32_t ma = 0, mb = 0;
-    for (const RaggedRow &d : ord) {
-        ma = std::max(ma, d.La);
-        mb = std::max(mb, d.Lb);
-    }
-    const uint64_t lc = (uint64_t)ma + mb;
-    uint32_t *pa = nullptr, *pb = nullptr, *pc = nullptr;
-    RaggedRow *dr = nullptr;
-    cudaError_t err = scratch_alloc((void **)&pa, (size_t)n * ma * 4);
-    if (err == cudaSuccess) err = scratch_alloc((void **)&pb, (size_t)n * mb * 4);
-    if (err == cudaSuccess) err = scratch_alloc((void **)&pc, (size_t)n * lc * 4);
-    if (err == cudaSuccess) err = scratch_alloc((void **)&dr, (size_t)n * sizeof(RaggedRow));
-    if (err == cudaSuccess) {
-        err = cudaMemcpyAsync(dr, ord.data(), (size_t)n * sizeof(RaggedRow), cudaMemcpyHostToDevice, st);
-        note_h2d((size_t)n * sizeof(RaggedRow));
-    }
-    if (err == cudaSuccess && nk) {
-        k_gather_rows<<<grid_rows(nk), 256, 0, st>>>(pa, ma, A, dr, nk, 0);
-        k_gather_rows<<<grid_rows(nk), 256, 0, st>>>(pb, mb, B, dr, nk, 1);
-        count_launch();
-        count_launch();
-    }
-    if (err == cudaSuccess && ns) {
-        k_gather_rows<<<grid_rows(ns), 256, 0, st>>>(pa + (size_t)nk * ma, ma, B, dr + nk, ns, 0);
-        k_gather_rows<<<grid_rows(ns), 256, 0, st>>>(pb + (size_t)nk * mb, mb, A, dr + nk, ns, 1);
-        count_launch();
-        count_launch();
-    }
-    if (err == cudaSuccess) {
-        const BatchMPArray a{pa, ma, n, ma}, b{pb, mb, n, mb}, c{pc, (uint32_t)lc, n, (uint32_t)lc};
-        err = mul_tuned(ctx, a, b, c);
-    }
-    if (err == cudaSuccess) {
-        k_scatter_rows<<<grid_rows(n), 256, 0, st>>>(C, pc, lc, dr, n);
-        count_launch();
-        err = cudaGetLastError();
-    }
-    scratch_free(pa);
-    scratch_free(pb);
-    scratch_free(pc);
-    scratch_free(dr);
-    return err;
+// Group numbers: zero products, schoolbook, tensor-core length steps from the
+// longest (32 limbs each), NTT buckets.
+constexpr uint32_t kZero = 0u, kSchoolGroup = 1u, kTensorGroup = 2u;
+constexpr uint32_t kTensorStep = 32u;
+constexpr uint32_t kTensorGroups = 8192u / kTensorStep + 1u;
+constexpr uint32_t kNttGroup = kTensorGroup + kTensorGroups;
+constexpr uint32_t kNttGroups = 4u * 32u;
+constexpr uint32_t kGroups = kNttGroup + kNttGroups;
+
+uint32_t ntt_bucket(uint64_t need) {   // 4 ceil(log2 need), less the quarter octaves below above 2^13
+    uint32_t k = 0;
+    while ((1ull << k) < need) ++k;
+    if (k <= 13u) return 4u * k;
+    const uint64_t q = 1ull << (k - 3u);   // an eighth of 2^k: quarters of its octave
+    const uint32_t below = (uint32_t)(((1ull << k) - need) / q);   // 0 .. 3
+    return 4u * k - below;
 }
 
 }  // namespace
@@ -145,57 +76,76 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
     if (N == 0u) return cudaSuccess;
     if (!ctx || !A || !B || !C || !offA || !La || !offB || !Lb || !offC) return cudaErrorInvalidValue;
     cudaStream_t st = current_stream();
-    std::vector<RaggedRow> zero, school, tensor;
-    std::map<int, std::vector<RaggedRow>> ntt;   // by log2 of the transform size
-    uint64_t school_work = 0, tc_limbs = 0;
-    uint32_t tcQ = 0, tcN = 0;
+    // counting sort into groups
+    std::vector<uint8_t> kind(N);
+    mul_kinds(N, La, Lb, kind.data());
+    std::vector<uint16_t> group(N);
+    std::vector<uint32_t> start(kGroups + 1u, 0u);
     for (uint32_t i = 0; i < N; ++i) {
-        const RaggedRow d{offA[i], offB[i], offC[i], La[i], Lb[i]};
-        const uint64_t Lc = (uint64_t)d.La + d.Lb;
-        if (Lc > (20ull << 25) || std::min(d.La, d.Lb) > (1u << 28)) return cudaErrorInvalidValue;
-        if (d.La == 0u || d.Lb == 0u) {
-            zero.push_back(d);
-        } else if (const int kind = mul_kind(d.La, d.Lb, false); kind == 0) {
-            school.push_back(d);
-            school_work += (uint64_t)d.La * d.Lb;
-        } else if (kind == 1) {
-            tensor.push_back(d);
+        const uint64_t Lc = (uint64_t)La[i] + Lb[i];
+        if (Lc > (20ull << 25) || std::min(La[i], Lb[i]) > (1u << 28)) return cudaErrorInvalidValue;
+        uint32_t g;
+        if (La[i] == 0u || Lb[i] == 0u)
+            g = kZero;
+        else if (kind[i] == 0u)
+            g = kSchoolGroup;
+        else if (kind[i] == 1u)
+            g = kTensorGroup + (kTensorGroups - 1u - (uint32_t)Lc / kTensorStep);
+        else
+            g = kNttGroup + ntt_bucket(Lc - 1u);
+        group[i] = (uint16_t)g;
+        ++start[g + 1u];
+    }
+    for (uint32_t g = 0; g < kGroups; ++g) start[g + 1u] += start[g];
+    std::vector<RaggedRow> rows(N);
+    {
+        std::vector<uint32_t> at(start.begin(), start.end() - 1);
+        for (uint32_t i = 0; i < N; ++i) rows[at[group[i]]++] = RaggedRow{offA[i], offB[i], offC[i], La[i], Lb[i]};
+    }
+    RaggedRow *dr = nullptr;
+    cudaError_t err = scratch_alloc((void **)&dr, (size_t)N * sizeof(RaggedRow));
+    if (err == cudaSuccess) {
+        err = cudaMemcpyAsync(dr, rows.data(), (size_t)N * sizeof(RaggedRow), cudaMemcpyHostToDevice, st);
+        note_h2d((size_t)N * sizeof(RaggedRow));
+    }
+    const uint32_t nz = start[1], ns = start[2] - start[1];
+    if (err == cudaSuccess && nz) {
+        k_zero_rows<<<grid_rows(nz), 256, 0, st>>>(C, dr, nz);
+        count_launch();
+    }
+    if (err == cudaSuccess && ns) {
+        uint64_t work = 0;
+        for (uint32_t i = start[1]; i < start[2]; ++i) work += (uint64_t)rows[i].La * rows[i].Lb;
+        school_mul_ragged(A, B, C, ns, dr + start[1], work);
+    }
+    // tensor-core launches: products above 2048, 1024 and 512 limbs, the rest
+    for (uint32_t first = start[kTensorGroup], end = start[kNttGroup]; err == cudaSuccess && first < end;) {
+        const uint32_t longest = rows[first].La + rows[first].Lb;
+        const uint32_t least = longest >= 2048u ? 2048u : longest >= 1024u ? 1024u : longest >= 512u ? 512u : 0u;
+        uint32_t last = first, maxQ = 0, maxN = 0;
+        uint64_t limbs = 0;
+        // 32-limb groups: a group never spans one of the limits
+        for (; last < end && rows[last].La + rows[last].Lb >= least; ++last) {
             uint32_t q = 0, n = 0;
-            tc_shape(d.La, d.Lb, &q, &n);
-            tcQ = std::max(tcQ, q);
-            tcN = std::max(tcN, n);
-            tc_limbs += 2ull * Lc;
-        } else {
-            ntt[ceil_log2_u64(Lc - 1)].push_back(d);
+            tc_shape(rows[last].La, rows[last].Lb, &q, &n);
+            maxQ = std::max(maxQ, q);
+            maxN = std::max(maxN, n);
+            limbs += 2ull * (rows[last].La + rows[last].Lb);
         }
+        err = tc_mul_ragged(A, B, C, last - first, dr + first, maxQ, maxN, limbs);
+        first = last;
     }
-    cudaError_t err = cudaSuccess;
-    if (!zero.empty() || !school.empty() || !tensor.empty()) {
-        std::vector<RaggedRow> both(zero);
-        both.insert(both.end(), school.begin(), school.end());
-        both.insert(both.end(), tensor.begin(), tensor.end());
-        RaggedRow *dr = nullptr;
-        err = scratch_alloc((void **)&dr, both.size() * sizeof(RaggedRow));
-        if (err == cudaSuccess) {
-            err = cudaMemcpyAsync(dr, both.data(), both.size() * sizeof(RaggedRow), cudaMemcpyHostToDevice, st);
-            note_h2d(both.size() * sizeof(RaggedRow));
-        }
-        if (err == cudaSuccess && !zero.empty()) {
-            k_zero_rows<<<grid_rows((uint32_t)zero.size()), 256, 0, st>>>(C, dr, (uint32_t)zero.size());
-            count_launch();
-        }
-        if (err == cudaSuccess && !school.empty())
-            school_mul_ragged(A, B, C, (uint32_t)school.size(), dr + zero.size(), school_work);
-        if (err == cudaSuccess && !tensor.empty())
-            err = tc_mul_ragged(A, B, C, (uint32_t)tensor.size(), dr + zero.size() + school.size(), tcQ, tcN,
-                                tc_limbs);
-        if (err == cudaSuccess) err = cudaGetLastError();
-        scratch_free(dr);
+    for (uint32_t g = kNttGroup; err == cudaSuccess && g < kGroups; ++g) {
+        const uint32_t n = start[g + 1u] - start[g];
+        if (!n) continue;
+        uint32_t most = 0;
+        for (uint32_t i = start[g]; i < start[g + 1u]; ++i) most = std::max(most, rows[i].La + rows[i].Lb);
+        err = batch_mp_ensure_workspace(ctx, batch_mul_ntt_workspace_size(n, most - 1u, 1u));
+        if (err == cudaSuccess)
+            ntt_mul_ragged(context_tables(ctx), (uint32_t *)context_workspace(ctx), A, B, C, n, dr + start[g], most);
     }
-    for (auto &kv : ntt) {
-        if (err != cudaSuccess) break;
-        err = ntt_bucket(ctx, kv.second, A, B, C, st);
-    }
+    if (err == cudaSuccess) err = cudaGetLastError();
+    scratch_free(dr);
     return err;
 }
 

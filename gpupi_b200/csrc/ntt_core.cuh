@@ -121,12 +121,16 @@ __device__ __forceinline__ uint32_t shoup(uint32_t x, uint32_t w, uint32_t wq) {
     const uint32_t q = __umulhi(x, wq);
     return x * w - q * Prime<Q>::p;
 }
+// (hi 2^32 + lo) / 2^32 mod p in (0, 2p), hi < p
+template <int Q>
+__device__ __forceinline__ uint32_t redc(uint32_t lo, uint32_t hi) {
+    return hi - __umulhi(lo * PrimeC<Q>::pinv, Prime<Q>::p) + Prime<Q>::p;
+}
 // a * b / 2^32 mod p in (0, 2p); requires a * b < 2^32 * p
 template <int Q>
 __device__ __forceinline__ uint32_t mont(uint32_t a, uint32_t b) {
     const uint64_t t = (uint64_t)a * b;
-    const uint32_t m = (uint32_t)t * PrimeC<Q>::pinv;
-    return (uint32_t)(t >> 32) - __umulhi(m, Prime<Q>::p) + Prime<Q>::p;
+    return redc<Q>((uint32_t)t, (uint32_t)(t >> 32));
 }
 
 // Table layout inside NTTPrecomputedTables (raw u32 views of the uint3 buffers).
@@ -322,6 +326,10 @@ struct Stage {
     // loaded once each from the contiguous table of that level, so the lanes
     // of a warp read consecutive entries or one broadcast entry.  The
     // half-span-1 level (LO = 0, lm = 0) has twiddle 1 and needs no product.
+    // Forward levels keep residues in [0, p).  Inverse levels leave them in
+    // [0, 2p) (the next level reduces one operand and multiplies the other, so
+    // a butterfly reduces twice instead of three times: 11.1 -> 10.5 issue
+    // cycles per warp); run_stages reduces once after the last one.
     template <bool INV, int Q>
     __device__ static __forceinline__ void bfly(uint32_t (&x)[16], int j, int mm, uint2 w, bool trivial) {
         constexpr uint32_t P = Prime<Q>::p;
@@ -330,10 +338,14 @@ struct Stage {
         if (!INV) {
             x[j] = add_n<Q>(a, b);
             x[j + mm] = trivial ? sub_n<Q>(a, b) : norm<Q>(shoup<Q>(a - b + P, w.x, w.y));
-        } else {
-            const uint32_t y = trivial ? b : norm<Q>(shoup<Q>(b, w.x, w.y));
-            x[j] = add_n<Q>(a, y);
-            x[j + mm] = sub_n<Q>(a, y);
+        } else if (trivial) {   // the first inverse level: a, b in [0, p)
+            x[j] = a + b;
+            x[j + mm] = a - b + P;
+        } else {   // a, b in [0, 2p), results too
+            const uint32_t y = norm<Q>(shoup<Q>(b, w.x, w.y));
+            const uint32_t z = norm<Q>(a);
+            x[j] = z + y;
+            x[j + mm] = z - y + P;
         }
     }
     template <bool INV, int Q>
@@ -380,11 +392,29 @@ struct ExecStage {
     using S = Stage<LOG_R, LOG_TC, I::LO, I::B>;
 };
 
+// Barrier of the threads that share a tile: the whole CTA, or one of several
+// groups of 256 threads with a named barrier of its own.
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+struct GroupSync {
+    uint32_t id;   // 1 .. 15 (0 is the CTA's)
+    __device__ __forceinline__ void operator()() const {
+        asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory");
+    }
+};
+
 // Runs execution stages K .. n-1 on x (and, with PAIR, in lockstep on y);
-// Sx / Sy are the shared tiles of the stage hand-offs.
-template <int LOG_R, int LOG_TC, bool INV, int Q, int K, bool PAIR>
+// Sx / Sy are the shared tiles of the stage hand-offs.  A stage's results go
+// back to the tile positions that the thread itself loaded, so one barrier
+// per hand-off is enough: between a thread's load and its next store no other
+// thread touches those positions.  On entry the tile must be free at the
+// positions of the first stage's mapping: a forward transform leaves it free
+// only at the last stage's (the inverse may follow at once, another forward
+// transform needs a barrier first), and the reverse.
+template <int LOG_R, int LOG_TC, bool INV, int Q, int K, bool PAIR, class Sync>
 __device__ __forceinline__ void run_stages_pair(uint32_t (&x)[16], uint32_t (&y)[16], uint32_t *Sx, uint32_t *Sy,
-                                                uint32_t t, const uint2 *tw) {
+                                                uint32_t t, const uint2 *tw, Sync sync) {
     constexpr int n = StagePlan<LOG_R>::n;
     if constexpr (K < n) {
         using Cur = typename ExecStage<LOG_R, LOG_TC, INV, K>::S;
@@ -392,19 +422,24 @@ __device__ __forceinline__ void run_stages_pair(uint32_t (&x)[16], uint32_t (&y)
             using Prev = typename ExecStage<LOG_R, LOG_TC, INV, K - 1>::S;
             Prev::store(Sx, x, t);
             if (PAIR) Prev::store(Sy, y, t);
-            __syncthreads();
+            sync();
             Cur::load(Sx, x, t);
             if (PAIR) Cur::load(Sy, y, t);
-            __syncthreads();
         }
         Cur::template levels_pair<INV, Q, PAIR>(x, y, t, tw);
-        run_stages_pair<LOG_R, LOG_TC, INV, Q, K + 1, PAIR>(x, y, Sx, Sy, t, tw);
+        run_stages_pair<LOG_R, LOG_TC, INV, Q, K + 1, PAIR>(x, y, Sx, Sy, t, tw, sync);
+    } else if constexpr (INV) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            x[j] = norm<Q>(x[j]);
+            if (PAIR) y[j] = norm<Q>(y[j]);
+        }
     }
 }
 
-template <int LOG_R, int LOG_TC, bool INV, int Q, int K>
-__device__ __forceinline__ void run_stages(uint32_t (&x)[16], uint32_t *Sm, uint32_t t, const uint2 *tw) {
-    run_stages_pair<LOG_R, LOG_TC, INV, Q, K, false>(x, x, Sm, Sm, t, tw);
+template <int LOG_R, int LOG_TC, bool INV, int Q, int K, class Sync>
+__device__ __forceinline__ void run_stages(uint32_t (&x)[16], uint32_t *Sm, uint32_t t, const uint2 *tw, Sync sync) {
+    run_stages_pair<LOG_R, LOG_TC, INV, Q, K, false>(x, x, Sm, Sm, t, tw, sync);
 }
 
 }  // namespace ntt

@@ -302,8 +302,8 @@ static cudaError_t plain_level(BatchMPContext *ctx, Profiler *pr, uint32_t n, ui
 // serves P' = P_e P_o and R2 = P_e R_o, so the level's four products take
 // six forward transforms instead of eight (four inverse either way): the
 // six operands' column passes, then one row kernel for the four products
-// (spectrum_level_rows), then each product's inverse column passes and
-// CRT; R' = (R1 << s) +- R2 as in the plain level.  All products run at the
+// (spectrum_level_rows), then the products' inverse column passes, two per
+// launch, and each one's CRT; R' = (R1 << s) +- R2 as in the plain level.  All products run at the
 // largest one's transform shape; used when that costs less than the plain
 // level (summing R' in the transform domain would need room for R1 << s,
 // about 6 % longer than R1, which sits just below a power of two at every
@@ -375,12 +375,17 @@ static cudaError_t tuned_level(BatchMPContext *ctx, Profiler *pr, uint32_t n, ui
         spectrum_level_rows(tab, S, half, fpe.p, pb ? fpo.p : nullptr, fro.p, fqo.p, fqe.p, fre.p);
         fpe.reset();
         fqo.reset();
+        // inverse column passes, two products per launch (P' has pb rows)
+        spectrum_inverse_columns(tab, S, half, fqe.p, fre.p);
+        if (pb) spectrum_inverse_columns(tab, S, pb, fpo.p, fro.p);
+        if (pb < half)
+            spectrum_inverse_columns(tab, S, half - pb, fro.p + spectrum_words(S, pb), nullptr);
         return cudaGetLastError();
     }));
     auto finish = [&](const char *label, uint32_t rows, Buf &f, uint32_t *C, uint32_t Lc, uint32_t la,
                       uint32_t lb) {
         return stage(pr, "mul", label, n1, rows, la, lb, true, [&]() {
-            spectrum_inverse(tab, S, rows, 1, nullptr, nullptr, f.p, C, Lc, Lc, flags.p, false);
+            spectrum_inverse(tab, S, rows, 1, nullptr, nullptr, f.p, C, Lc, Lc, flags.p, false, false);
             f.reset();
             return cudaGetLastError();
         });
@@ -412,7 +417,8 @@ static cudaError_t tuned_level(BatchMPContext *ctx, Profiler *pr, uint32_t n, ui
         // separate addition pass runs (same integers as the plain level)
         const SpectrumAddend add{r1b.p, R1.stride, R1.length, shift, lr + lp - 1u};
         TRY(stage(pr, "mul", "P*R+(R*Q<<15n)", n1, half, lp, lr, true, [&]() {
-            spectrum_inverse(tab, S, half, 1, nullptr, nullptr, fro.p, Rn.data, rlen, rlen, flags.p, false, &add);
+            spectrum_inverse(tab, S, half, 1, nullptr, nullptr, fro.p, Rn.data, rlen, rlen, flags.p, false, false,
+                             &add);
             fro.reset();
             return cudaGetLastError();
         }));

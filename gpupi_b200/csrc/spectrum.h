@@ -52,10 +52,12 @@ struct SpectrumAddend {
 // addend when add is not null).  Fout receives the intermediate residues and
 // may be one of the X_t / Y_t; flags: spectrum_flag_words(N, Lc) words.
 // rows = false: Fout already holds the product after its inverse row pass
-// (spectrum_level_rows); X and Y are not read.
+// (spectrum_level_rows); X and Y are not read.  cols = false: also after its
+// inverse column passes (spectrum_inverse_columns).
 void spectrum_inverse(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, int terms,
                       const uint32_t *const *X, const uint32_t *const *Y, uint32_t *Fout, uint32_t *C, uint64_t sC,
-                      uint32_t Lc, uint32_t *flags, bool rows = true, const SpectrumAddend *add = nullptr);
+                      uint32_t Lc, uint32_t *flags, bool rows = true, bool cols = true,
+                      const SpectrumAddend *add = nullptr);
 
 // One merge level's row products from six column-transformed operands
 // (spectrum_forward with rows = false): P' = P_e P_o into Fpo, R2 = P_e R_o
@@ -63,5 +65,10 @@ void spectrum_inverse(const NTTPrecomputedTables &tables, SpectrumShape s, uint3
 // inverse row pass; N rows of shape s.  Fpo null: no P' (five operands).
 void spectrum_level_rows(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *Fpe,
                          uint32_t *Fpo, uint32_t *Fro, uint32_t *Fqo, uint32_t *Fqe, uint32_t *Fre);
+
+// The inverse column passes of N rows of two products at once (F1 null: of
+// one), sharing the stages' twiddles and twist factors.
+void spectrum_inverse_columns(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *F0,
+                              uint32_t *F1);
 
 }  // namespace gpupi

@@ -160,22 +160,18 @@ std::string default_table_path() {
 
 // Kernel for a product of La x Lb limbs.  public_api: gpupi's batch_mp_mul
 // contract (no product above 1024 limbs avoids the NTT, none at or below
-// it uses the NTT's workspace).
-int mul_kind(uint32_t La, uint32_t Lb, bool public_api) {
+// it uses the NTT's workspace).  t.mu held.
+static int mul_kind_locked(const Table &t, uint32_t La, uint32_t Lb, bool public_api) {
     const uint64_t L = (uint64_t)La + Lb;
     if (La == 0u || Lb == 0u || school_thread_fits(La, Lb)) return kSchool;
     int k = -1;
-    {
-        Table &t = table();
-        std::lock_guard<std::mutex> g(t.mu);
-        if (t.loaded) {
-            k = kNtt;
-            for (const MulEntry &e : t.mul)
-                if (L <= e.max_sum) {
-                    k = e.kind;
-                    break;
-                }
-        }
+    if (t.loaded) {
+        k = kNtt;
+        for (const MulEntry &e : t.mul)
+            if (L <= e.max_sum) {
+                k = e.kind;
+                break;
+            }
     }
     if (k < 0) k = (L <= school_max() && L <= 1024u) ? kSchool : kNtt;
     if (public_api) {
@@ -185,6 +181,19 @@ int mul_kind(uint32_t La, uint32_t Lb, bool public_api) {
     if (k == kTensor && !tc_fits(La, Lb)) k = (L <= 1024u) ? kSchool : kNtt;
     if (k == kSchool && L > 1024u) k = kNtt;
     return k;
+}
+
+int mul_kind(uint32_t La, uint32_t Lb, bool public_api) {
+    Table &t = table();
+    std::lock_guard<std::mutex> g(t.mu);
+    return mul_kind_locked(t, La, Lb, public_api);
+}
+
+// The library's own choice for each product of a ragged batch.
+void mul_kinds(uint32_t n, const uint32_t *La, const uint32_t *Lb, uint8_t *kinds) {
+    Table &t = table();
+    std::lock_guard<std::mutex> g(t.mu);
+    for (uint32_t i = 0; i < n; ++i) kinds[i] = (uint8_t)mul_kind_locked(t, La[i], Lb[i], false);
 }
 
 // NTT shape for `need` points from the table (or the tuner's forced
