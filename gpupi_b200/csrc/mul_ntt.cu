@@ -246,47 +246,50 @@ __device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int 
     }
 }
 
-template <class First, int LOG_R, int Q>
+template <class First, int LOG_R, int Q, bool HALF>
 __device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx, uint32_t nb,
                                            uint64_t K, int log_cols, uint32_t c0, uint32_t t, int coset,
                                            const uint32_t *W, uint32_t f) {
-    if (nb == 1u && coset == 0) {
+    if (HALF || (nb == 1u && coset == 0)) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             uint32_t pos, c;
             First::elem(t, j, pos, c);
             const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c;
-            x[j] = (i < Lx) ? reduce_limb<Q>(__ldg(xr + i)) : 0u;
+            const bool upper = HALF && ((j >> (First::kB - 1)) & 1);   // positions R / 2 .. R - 1
+            x[j] = (!upper && i < Lx) ? reduce_limb<Q>(__ldg(xr + i)) : 0u;
         }
         return;
     }
-    // two halves of eight residues: their sums and loads fit the registers
+    if constexpr (!HALF) {
+        // two halves of eight residues: their sums and loads fit the registers
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t lo[8], hi[8];
+        for (int h = 0; h < 2; ++h) {
+            uint32_t lo[8], hi[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0u;
+            for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0u;
 #pragma unroll 1
-        for (uint32_t blk = 0; blk < nb; ++blk) {
-            uint32_t v[8];
+            for (uint32_t blk = 0; blk < nb; ++blk) {
+                uint32_t v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                uint32_t pos, c;
-                First::elem(t, 8 * h + j, pos, c);
-                const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c + (uint64_t)blk * K;
-                v[j] = (i < Lx) ? __ldg(xr + i) : 0u;
+                for (int j = 0; j < 8; ++j) {
+                    uint32_t pos, c;
+                    First::elem(t, 8 * h + j, pos, c);
+                    const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c + (uint64_t)blk * K;
+                    v[j] = (i < Lx) ? __ldg(xr + i) : 0u;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint64_t s = (uint64_t)v[j] * W[16u * blk + 8u * h + j] + (((uint64_t)hi[j] << 32) | lo[j]);
+                    lo[j] = (uint32_t)s;
+                    hi[j] = norm<Q>((uint32_t)(s >> 32));   // < p again
+                }
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const uint64_t s = (uint64_t)v[j] * W[16u * blk + 8u * h + j] + (((uint64_t)hi[j] << 32) | lo[j]);
-                lo[j] = (uint32_t)s;
-                hi[j] = norm<Q>((uint32_t)(s >> 32));   // < p again
+                const uint32_t r = redc<Q>(lo[j], hi[j]);   // < 2p
+                x[8 * h + j] = norm<Q>(mont<Q>(r, f));
             }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t r = redc<Q>(lo[j], hi[j]);   // < 2p
-            x[8 * h + j] = norm<Q>(mont<Q>(r, f));
         }
     }
 }
@@ -294,7 +297,10 @@ __device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr
 // Column pass: R = 2^LOG_R (<= 512) points per column, TC = 4096 / R columns
 // per CTA; segment of S = 2^log_s points viewed as [R][S/R].  PAIR: the
 // forward pass of A and B together (same tile, shared twiddles and twists).
-template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, int Q>
+// HALF (first pass): each operand fills at most the lower half of its K points
+// (a balanced product at one power-of-two transform): half the loads, and the
+// first level multiplies without adding.
+template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, bool HALF, int Q>
 __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a, uint64_t b, uint32_t *Sm,
                                           uint32_t *Sm2, uint2 *tw) {
     constexpr int LOG_TC = 12 - LOG_R;
@@ -346,7 +352,7 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
         const uint32_t blocks = PAIR ? max(nb, nb2) : nb;
         uint32_t f = 0u;    // g^(coset i_0), Montgomery form
         uint32_t *W = Sm;   // weights in the tile, before its first use
-        if (coset || blocks > 1u) {
+        if (!HALF && (coset || blocks > 1u)) {
             const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q);
             const uint32_t *chi = coset_hi_ptr(P.tab, 0, Q);
             uint32_t pos, c;
@@ -356,9 +362,9 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
             coset_weights<First, LOG_R, Q>(W, blocks, coset, a.log_k, log_cols, clo, chi);
             __syncthreads();
         }
-        load_limbs<First, LOG_R, Q>(x, X.p, X.L, nb, K, log_cols, c0, t, coset, W, f);
+        load_limbs<First, LOG_R, Q, HALF>(x, X.p, X.L, nb, K, log_cols, c0, t, coset, W, f);
         if constexpr (PAIR)
-            load_limbs<First, LOG_R, Q>(y, Y.p, Y.L, nb2, K, log_cols, c0, t, coset, W, f);
+            load_limbs<First, LOG_R, Q, HALF>(y, Y.p, Y.L, nb2, K, log_cols, c0, t, coset, W, f);
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -374,7 +380,7 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
         }
     }
     __syncthreads();   // twiddle table ready (and the weights read)
-    run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR>(x, y, Sm, Sm2, t, tw, CtaSync{});
+    run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR, CtaSync, HALF>(x, y, Sm, Sm2, t, tw, CtaSync{});
     if constexpr (!INVERSE) twist16<Last, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, PrimeC<Q>::r1, false);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -395,7 +401,7 @@ constexpr size_t cols_smem_bytes() {   // one or two padded tiles + the twiddle 
 // operands' residues, and for the first of them a few words spill, but the
 // extra resident warps hide more of the limb and tile latency (first pass of
 // a 2^24 x 2^24-limb product 0.589 -> 0.541 ms against three CTAs per SM).
-template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR>
+template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, bool HALF>
 __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a) {
     extern __shared__ uint4 cols_smem[];
     uint32_t *Sm = reinterpret_cast<uint32_t *>(cols_smem);
@@ -404,11 +410,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a)
     uint64_t b;
     const int q = grid_prime(b);
     if (q == 0)
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, 0>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 0>(P, a, b, Sm, Sm2, tw);
     else if (q == 1)
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, 1>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 1>(P, a, b, Sm, Sm2, tw);
     else
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, 2>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 2>(P, a, b, Sm, Sm2, tw);
 }
 
 __device__ __forceinline__ void swap16(uint32_t (&x)[16], uint32_t (&y)[16]) {
@@ -639,7 +645,7 @@ __device__ __forceinline__ void rows_run(const RowsArgs &a, uint32_t first, uint
 // Whole products of 4096 points, from limbs: both operands' limbs are loaded
 // at once (their HBM latency overlaps), the product is scaled by K^-1 here.
 // 1024 products of 2001 x 1903 limbs: 125 -> 108 us.
-template <int Q>
+template <bool HALF, int Q>
 __device__ __forceinline__ void rows_limbs_run(const NttParams &P, const RowsArgs &a, uint32_t first, uint32_t last,
                                                const RowShared &s) {
     const uint32_t t = threadIdx.x & 255u;
@@ -652,8 +658,9 @@ __device__ __forceinline__ void rows_limbs_run(const NttParams &P, const RowsArg
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const uint32_t pos = t + 256u * j;
-            xa[j] = (pos < A.L) ? reduce_limb<Q>(__ldg(A.p + pos)) : 0u;
-            xb[j] = (pos < B.L) ? reduce_limb<Q>(__ldg(B.p + pos)) : 0u;
+            const bool upper = HALF && j >= 8;
+            xa[j] = (!upper && pos < A.L) ? reduce_limb<Q>(__ldg(A.p + pos)) : 0u;
+            xb[j] = (!upper && pos < B.L) ? reduce_limb<Q>(__ldg(B.p + pos)) : 0u;
         }
 #pragma unroll 1
         for (int op = 0; op < (a.square ? 1 : 2); ++op) {
@@ -661,7 +668,7 @@ __device__ __forceinline__ void rows_limbs_run(const NttParams &P, const RowsArg
                 sync();   // A's last hand-off has been read
                 swap16(xa, xb);
             }
-            run_stages<kRowLog, 0, false, Q, 0>(xa, s.tile, t, s.twf, sync);
+            run_stages<kRowLog, 0, false, Q, 0, HALF>(xa, s.tile, t, s.twf, sync);
         }
         const uint32_t scale = __ldg(P.tab.inv2n + kRowLog * kPrimes + Q);
 #pragma unroll
@@ -674,24 +681,25 @@ __device__ __forceinline__ void rows_limbs_run(const NttParams &P, const RowsArg
     }
 }
 
-template <bool LIMBS, int Q>
+template <bool LIMBS, bool HALF, int Q>
 __device__ __forceinline__ void rows_prime(const NttParams &P, const RowsArgs &a, uint32_t segs, const RowShared &s) {
     uint32_t first, last;
     if (!row_share(segs, Q, first, last)) return;
     row_tables(P, Q, s);
     if constexpr (LIMBS)
-        rows_limbs_run<Q>(P, a, first, last, s);
+        rows_limbs_run<HALF, Q>(P, a, first, last, s);
     else
         rows_run<Q>(a, first, last, s);
 }
 
-template <bool LIMBS>
+// HALF (with LIMBS): operands of at most 2048 limbs
+template <bool LIMBS, bool HALF>
 __global__ void __launch_bounds__(kRowThreads, kRowCtas) k_rows(NttParams P, RowsArgs a, uint32_t segs) {
     extern __shared__ uint4 rows_smem[];
     const RowShared s = row_shared(rows_smem);
-    rows_prime<LIMBS, 0>(P, a, segs, s);
-    rows_prime<LIMBS, 1>(P, a, segs, s);
-    rows_prime<LIMBS, 2>(P, a, segs, s);
+    rows_prime<LIMBS, HALF, 0>(P, a, segs, s);
+    rows_prime<LIMBS, HALF, 1>(P, a, segs, s);
+    rows_prime<LIMBS, HALF, 2>(P, a, segs, s);
 }
 
 // Whole product of K <= 2^8 points per CTA (one prime, one row), radix-2
@@ -1318,37 +1326,37 @@ constexpr int kPairMinLogR = 5;
 // pass against 0.41 ms in two.
 constexpr int kOnePassMaxLog = 10;
 
-template <int LOG_R, bool FL, bool INV, bool PAIR>
+template <int LOG_R, bool FL, bool INV, bool PAIR, bool HALF>
 static void cols_launch(unsigned blocks, const NttParams &P, const ColsArgs &a, cudaStream_t st) {
     constexpr size_t smem = cols_smem_bytes<LOG_R, PAIR>();
     static bool attr = false;
     if (!attr) {
         if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_cols_r<LOG_R, FL, INV, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(k_cols_r<LOG_R, FL, INV, PAIR, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         attr = true;
     }
-    k_cols_r<LOG_R, FL, INV, PAIR><<<blocks, kThreads, smem, st>>>(P, a);
+    k_cols_r<LOG_R, FL, INV, PAIR, HALF><<<blocks, kThreads, smem, st>>>(P, a);
 }
 
-template <bool FL, bool INV, bool PAIR>
+template <bool FL, bool INV, bool PAIR, bool HALF = false>
 static void cols_r_dispatch(int log_r, unsigned blocks, const NttParams &P, const ColsArgs &a, cudaStream_t st) {
     if constexpr (!PAIR) {
         switch (log_r) {
-            case 1: cols_launch<1, FL, INV, false>(blocks, P, a, st); return;
-            case 2: cols_launch<2, FL, INV, false>(blocks, P, a, st); return;
-            case 3: cols_launch<3, FL, INV, false>(blocks, P, a, st); return;
-            case 4: cols_launch<4, FL, INV, false>(blocks, P, a, st); return;
+            case 1: cols_launch<1, FL, INV, false, HALF>(blocks, P, a, st); return;
+            case 2: cols_launch<2, FL, INV, false, HALF>(blocks, P, a, st); return;
+            case 3: cols_launch<3, FL, INV, false, HALF>(blocks, P, a, st); return;
+            case 4: cols_launch<4, FL, INV, false, HALF>(blocks, P, a, st); return;
             default: break;
         }
     }
     switch (log_r) {
-        case 5: cols_launch<5, FL, INV, PAIR>(blocks, P, a, st); break;
-        case 6: cols_launch<6, FL, INV, PAIR>(blocks, P, a, st); break;
-        case 7: cols_launch<7, FL, INV, PAIR>(blocks, P, a, st); break;
-        case 8: cols_launch<8, FL, INV, PAIR>(blocks, P, a, st); break;
-        case 9: cols_launch<9, FL, INV, PAIR>(blocks, P, a, st); break;
-        default: cols_launch<10, FL, INV, PAIR>(blocks, P, a, st); break;
+        case 5: cols_launch<5, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        case 6: cols_launch<6, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        case 7: cols_launch<7, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        case 8: cols_launch<8, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        case 9: cols_launch<9, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        default: cols_launch<10, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
     }
 }
 
@@ -1367,8 +1375,14 @@ static void launch_cols_r(bool from_limbs, bool inverse, bool pair, int log_r, c
                                     : 24.0 * K * (double)vrows * ops;
     KernelTimed kt(from_limbs ? "ntt_cols_fwd_first" : (inverse ? "ntt_cols_inv" : "ntt_cols_fwd"), bytes);
     if (from_limbs) {
-        if (pair)
+        const uint64_t half = 1ull << (a.log_k - 1);
+        const bool lower = a.M == 1 && !a.coset0 && !a.rows && a.Lx <= half && (!pair || a.Lx2 <= half);
+        if (pair && lower)
+            cols_r_dispatch<true, false, true, true>(log_r, blocks, P, a, st);
+        else if (pair)
             cols_r_dispatch<true, false, true>(log_r, blocks, P, a, st);
+        else if (lower)
+            cols_r_dispatch<true, false, false, true>(log_r, blocks, P, a, st);
         else
             cols_r_dispatch<true, false, false>(log_r, blocks, P, a, st);
     } else if (!inverse) {
@@ -1399,8 +1413,9 @@ static void row_attr() {
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> l(mu);
     if ((done >> (dev & 63)) & 1u) return;
-    cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
-    cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    cudaFuncSetAttribute(k_rows<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    cudaFuncSetAttribute(k_rows<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
+    cudaFuncSetAttribute(k_rows<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
     cudaFuncSetAttribute(k_rows_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes());
     done |= 1ull << (dev & 63);
 }
@@ -1413,10 +1428,14 @@ static void launch_rows(int log_k, bool limbs, uint32_t segs, const NttParams &P
         case 11: rows_launch<11>((unsigned)(segs * kPrimes), P, r, st); break;
         default:
             row_attr();
-            if (limbs)
-                k_rows<true><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r, segs);
+            if (limbs && !r.rows && r.La <= kRowPoints / 2 && r.Lb <= kRowPoints / 2)
+                k_rows<true, true><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r,
+                                                                                                            segs);
+            else if (limbs)
+                k_rows<true, false><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(
+                    P, r, segs);
             else
-                k_rows<false><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r, segs);
+                k_rows<false, false><<<row_grid((uint64_t)segs * kPrimes), kRowThreads, row_smem_bytes(), st>>>(P, r, segs);
     }
     count_launch();
 }

@@ -353,8 +353,9 @@ struct Stage {
         levels_pair<INV, Q, false>(x, x, t, tw);
     }
     // Two independent transforms of the same shape (PAIR): every twiddle is
-    // loaded once and serves both.
-    template <bool INV, int Q, bool PAIR>
+    // loaded once and serves both.  HALF (forward, first stage): the upper half
+    // of every group is zero, so the first level only multiplies.
+    template <bool INV, int Q, bool PAIR, bool HALF = false>
     __device__ static __forceinline__ void levels_pair(uint32_t (&x)[16], uint32_t (&y)[16], uint32_t t,
                                                        const uint2 *tw) {
         constexpr int G = 16 >> B;
@@ -375,8 +376,14 @@ struct Stage {
                     const uint2 w = trivial ? make_uint2(1u, 0u) : tw[lbase + low + ((uint32_t)u << LO)];
 #pragma unroll
                     for (int v = u; v < (1 << B); v += 2 * mm) {
-                        bfly<INV, Q>(x, (g << B) + v, mm, w, trivial);
-                        if (PAIR) bfly<INV, Q>(y, (g << B) + v, mm, w, trivial);
+                        const int j = (g << B) + v;
+                        if (HALF && step == 0) {
+                            x[j + mm] = trivial ? x[j] : norm<Q>(shoup<Q>(x[j], w.x, w.y));
+                            if (PAIR) y[j + mm] = trivial ? y[j] : norm<Q>(shoup<Q>(y[j], w.x, w.y));
+                            continue;
+                        }
+                        bfly<INV, Q>(x, j, mm, w, trivial);
+                        if (PAIR) bfly<INV, Q>(y, j, mm, w, trivial);
                     }
                 }
             }
@@ -408,11 +415,12 @@ struct GroupSync {
 // Sx / Sy are the shared tiles of the stage hand-offs.  A stage's results go
 // back to the tile positions that the thread itself loaded, so one barrier
 // per hand-off is enough: between a thread's load and its next store no other
-// thread touches those positions.  On entry the tile must be free at the
+// thread touches those positions.  HALF: the upper half of every transform's
+// points is zero (forward only).  On entry the tile must be free at the
 // positions of the first stage's mapping: a forward transform leaves it free
 // only at the last stage's (the inverse may follow at once, another forward
 // transform needs a barrier first), and the reverse.
-template <int LOG_R, int LOG_TC, bool INV, int Q, int K, bool PAIR, class Sync>
+template <int LOG_R, int LOG_TC, bool INV, int Q, int K, bool PAIR, class Sync, bool HALF = false>
 __device__ __forceinline__ void run_stages_pair(uint32_t (&x)[16], uint32_t (&y)[16], uint32_t *Sx, uint32_t *Sy,
                                                 uint32_t t, const uint2 *tw, Sync sync) {
     constexpr int n = StagePlan<LOG_R>::n;
@@ -426,8 +434,8 @@ __device__ __forceinline__ void run_stages_pair(uint32_t (&x)[16], uint32_t (&y)
             Cur::load(Sx, x, t);
             if (PAIR) Cur::load(Sy, y, t);
         }
-        Cur::template levels_pair<INV, Q, PAIR>(x, y, t, tw);
-        run_stages_pair<LOG_R, LOG_TC, INV, Q, K + 1, PAIR>(x, y, Sx, Sy, t, tw, sync);
+        Cur::template levels_pair<INV, Q, PAIR, HALF && K == 0>(x, y, t, tw);
+        run_stages_pair<LOG_R, LOG_TC, INV, Q, K + 1, PAIR, Sync, HALF>(x, y, Sx, Sy, t, tw, sync);
     } else if constexpr (INV) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -437,9 +445,9 @@ __device__ __forceinline__ void run_stages_pair(uint32_t (&x)[16], uint32_t (&y)
     }
 }
 
-template <int LOG_R, int LOG_TC, bool INV, int Q, int K, class Sync>
+template <int LOG_R, int LOG_TC, bool INV, int Q, int K, bool HALF = false, class Sync>
 __device__ __forceinline__ void run_stages(uint32_t (&x)[16], uint32_t *Sm, uint32_t t, const uint2 *tw, Sync sync) {
-    run_stages_pair<LOG_R, LOG_TC, INV, Q, K, false>(x, x, Sm, Sm, t, tw, sync);
+    run_stages_pair<LOG_R, LOG_TC, INV, Q, K, false, Sync, HALF>(x, x, Sm, Sm, t, tw, sync);
 }
 
 }  // namespace ntt
