@@ -140,6 +140,31 @@ __host__ __device__ constexpr uint32_t stage_delta(int j, int B, int log_r) {
     return ((uint32_t)j & ((1u << B) - 1u)) + (((uint32_t)j >> B) << (log_r - 4 + B));
 }
 
+// Distance of residue j of a thread from its residue 0 in stage S, in limbs of
+// a tile row pitch of 2^log_cols: positions and columns of j occupy bits that
+// those of residue 0 leave free, so it is the same for every thread.
+template <class S, int LOG_R>
+__device__ __forceinline__ uint32_t elem_delta(int j, int log_cols) {
+    constexpr int B = S::kB;
+    const uint32_t v = (uint32_t)j & ((1u << B) - 1u), g = (uint32_t)j >> B;
+    if constexpr (LOG_R >= 4)
+        return ((v << S::kLO) + (g << (LOG_R - 4 + B))) << log_cols;
+    else   // whole columns, 256 apart
+        return (v << log_cols) + 256u * g;
+}
+
+// Word i of an array by a 32-bit byte offset from a base that is the same for
+// the whole CTA: the offsets of a thread's residues differ by uniform amounts
+// (elem_delta), one 32-bit add each, where 64-bit indexing cost a wide
+// multiply-add (four cycles of the pipe that bounds these passes) per access.
+// i < 2^30: an operand has at most 20 * 2^25 limbs, a transform 2^25 points.
+__device__ __forceinline__ const uint32_t *word_at(const uint32_t *base, uint32_t i) {
+    return reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(base) + (uint64_t)(i * 4u));
+}
+__device__ __forceinline__ uint32_t *word_at(uint32_t *base, uint32_t i) {
+    return reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(base) + (uint64_t)(i * 4u));
+}
+
 // Twist the 16 residues of stage S (the LO = 0 stage: last forward, first
 // inverse) by one * w_S^(col * bitrev(pos)) / R or with the inverse root (one =
 // R for the plain twist, K^-1 R^2 where the product's scale is folded in),
@@ -216,22 +241,12 @@ __device__ __forceinline__ void twist16(uint32_t (&x)[16], uint32_t (&y)[16], ui
 // mod x^K - 1 when the operand is longer than K).
 //
 // Residue j of a thread sits delta_j above its first one, i_0, and the bits of
-// j add up in delta_j (FirstDelta), so it is g^(coset i_0) sum_b X_(b, j) W[b][j]
+// j add up in delta_j (elem_delta), so it is g^(coset i_0) sum_b X_(b, j) W[b][j]
 // over the K-limb blocks b, with W[b][j] = c^b g^(coset delta_j) the same for the
 // whole CTA (coset_weights, in shared memory).  The sum of 64-bit products is
 // kept below 2^32 p by reducing its upper word only, and reduced once at the
 // end: per block one wide multiply-add and one reduction instead of a modular
 // product, a sum and their reductions, and no chain of powers.
-template <class First, int LOG_R>
-__device__ __forceinline__ uint32_t first_delta(int bit, int log_cols) {   // of j = 2^bit
-    if constexpr (LOG_R >= 4) {
-        static_assert(First::kB == 4, "one group per thread");
-        return 1u << (First::kLO + log_cols + bit);
-    } else {   // 2^LOG_R positions of each of 16 / 2^LOG_R columns, 256 apart
-        return bit < LOG_R ? 1u << (log_cols + bit) : 256u << (bit - LOG_R);
-    }
-}
-
 template <class First, int LOG_R, int Q>
 __device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int coset, int log_k, int log_cols,
                                               const uint32_t *clo, const uint32_t *chi) {
@@ -241,23 +256,21 @@ __device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int 
         for (uint32_t k = 0; k < (e >> 4); ++k) w = norm<Q>(mont<Q>(w, c));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if ((e >> k) & 1u) w = mul_coset<Q, 0>(w, clo, chi, (uint32_t)coset * first_delta<First, LOG_R>(k, log_cols));
+            if ((e >> k) & 1u) w = mul_coset<Q, 0>(w, clo, chi, (uint32_t)coset * elem_delta<First, LOG_R>(1 << k, log_cols));
         W[e] = w;
     }
 }
 
 template <class First, int LOG_R, int Q, bool HALF>
 __device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx, uint32_t nb,
-                                           uint64_t K, int log_cols, uint32_t c0, uint32_t t, int coset,
-                                           const uint32_t *W, uint32_t f) {
+                                           uint64_t K, int log_cols, uint32_t i0, int coset, const uint32_t *W,
+                                           uint32_t f) {
     if (HALF || (nb == 1u && coset == 0)) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            First::elem(t, j, pos, c);
-            const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c;
+            const uint32_t i = i0 + elem_delta<First, LOG_R>(j, log_cols);
             const bool upper = HALF && ((j >> (First::kB - 1)) & 1);   // positions R / 2 .. R - 1
-            x[j] = (!upper && i < Lx) ? reduce_limb<Q>(__ldg(xr + i)) : 0u;
+            x[j] = (!upper && i < Lx) ? reduce_limb<Q>(__ldg(word_at(xr, i))) : 0u;
         }
         return;
     }
@@ -270,17 +283,20 @@ __device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr
             for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0u;
 #pragma unroll 1
             for (uint32_t blk = 0; blk < nb; ++blk) {
+                const uint32_t *xb = xr + blk * K;
+                const uint32_t left = Lx - blk * (uint32_t)K;   // > 0
+                const uint4 wa = *reinterpret_cast<const uint4 *>(W + 16u * blk + 8u * h);
+                const uint4 wb = *reinterpret_cast<const uint4 *>(W + 16u * blk + 8u * h + 4u);
+                const uint32_t w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
                 uint32_t v[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    uint32_t pos, c;
-                    First::elem(t, 8 * h + j, pos, c);
-                    const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c + (uint64_t)blk * K;
-                    v[j] = (i < Lx) ? __ldg(xr + i) : 0u;
+                    const uint32_t i = i0 + elem_delta<First, LOG_R>(8 * h + j, log_cols);
+                    v[j] = (i < left) ? __ldg(word_at(xb, i)) : 0u;
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const uint64_t s = (uint64_t)v[j] * W[16u * blk + 8u * h + j] + (((uint64_t)hi[j] << 32) | lo[j]);
+                    const uint64_t s = (uint64_t)v[j] * w[j] + (((uint64_t)hi[j] << 32) | lo[j]);
                     lo[j] = (uint32_t)s;
                     hi[j] = norm<Q>((uint32_t)(s >> 32));   // < p again
                 }
@@ -337,6 +353,9 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
     const uint32_t c0 = ct << LOG_TC;
     const int twist_shift = kMaxLog - a.log_s;
     const uint32_t t = threadIdx.x;
+    uint32_t pos0, col0;
+    First::elem(t, 0, pos0, col0);
+    const uint32_t i0 = (pos0 << log_cols) + c0 + col0;   // this thread's first residue
     uint32_t x[16], y[16];
     if constexpr (FROM_LIMBS) {
         const uint64_t row = vrow / (uint32_t)a.M;
@@ -355,24 +374,18 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
         if (!HALF && (coset || blocks > 1u)) {
             const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q);
             const uint32_t *chi = coset_hi_ptr(P.tab, 0, Q);
-            uint32_t pos, c;
-            First::elem(t, 0, pos, c);
-            const uint32_t i0 = (uint32_t)(((uint64_t)pos << log_cols) + c0 + c);
             f = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * i0);
             coset_weights<First, LOG_R, Q>(W, blocks, coset, a.log_k, log_cols, clo, chi);
             __syncthreads();
         }
-        load_limbs<First, LOG_R, Q, HALF>(x, X.p, X.L, nb, K, log_cols, c0, t, coset, W, f);
-        if constexpr (PAIR)
-            load_limbs<First, LOG_R, Q, HALF>(y, Y.p, Y.L, nb2, K, log_cols, c0, t, coset, W, f);
+        load_limbs<First, LOG_R, Q, HALF>(x, X.p, X.L, nb, K, log_cols, i0, coset, W, f);
+        if constexpr (PAIR) load_limbs<First, LOG_R, Q, HALF>(y, Y.p, Y.L, nb2, K, log_cols, i0, coset, W, f);
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            First::elem(t, j, pos, c);
-            const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c;
-            x[j] = F[i];
-            if constexpr (PAIR) y[j] = F2[i];
+            const uint32_t i = i0 + elem_delta<First, LOG_R>(j, log_cols);
+            x[j] = *word_at(F, i);
+            if constexpr (PAIR) y[j] = *word_at(F2, i);
         }
         if constexpr (INVERSE) {
             const uint32_t one = a.scaled ? __ldg(P.tab.inv2n + a.log_k * kPrimes + Q) : PrimeC<Q>::r1;
@@ -382,13 +395,14 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
     __syncthreads();   // twiddle table ready (and the weights read)
     run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR, CtaSync, HALF>(x, y, Sm, Sm2, t, tw, CtaSync{});
     if constexpr (!INVERSE) twist16<Last, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, PrimeC<Q>::r1, false);
+    uint32_t pos1, c1;
+    Last::elem(t, 0, pos1, c1);
+    const uint32_t i1 = (pos1 << log_cols) + c0 + c1;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        uint32_t pos, c;
-        Last::elem(t, j, pos, c);
-        const uint64_t i = ((uint64_t)pos << log_cols) + c0 + c;
-        F[i] = x[j];
-        if constexpr (PAIR) F2[i] = y[j];
+        const uint32_t i = i1 + elem_delta<Last, LOG_R>(j, log_cols);
+        *word_at(F, i) = x[j];
+        if constexpr (PAIR) *word_at(F2, i) = y[j];
     }
 }
 

@@ -304,21 +304,27 @@ struct Stage {
         const uint32_t i = (pos << LOG_TC) + c;
         return i + (i >> 5);   // one pad word per 32 avoids bank conflicts
     }
+    // Tile distance of element j from element 0: its bits are free in element
+    // 0's index, so the padded address moves by a compile-time amount too.
+    __host__ __device__ static constexpr uint32_t offset(int j) {
+        const uint32_t d = ((((uint32_t)j & ((1u << B) - 1u)) << LO) + (((uint32_t)j >> B) << (LOG_R - 4 + B)))
+                           << LOG_TC;
+        return d + (d >> 5);
+    }
     __device__ static __forceinline__ void store(uint32_t *S, const uint32_t (&x)[16], uint32_t t) {
+        static_assert(LOG_R >= 4, "stages of shorter columns have no hand-off");
+        uint32_t pos, c;
+        elem(t, 0, pos, c);
+        uint32_t *p = S + addr(pos, c);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            elem(t, j, pos, c);
-            S[addr(pos, c)] = x[j];
-        }
+        for (int j = 0; j < 16; ++j) p[offset(j)] = x[j];
     }
     __device__ static __forceinline__ void load(const uint32_t *S, uint32_t (&x)[16], uint32_t t) {
+        uint32_t pos, c;
+        elem(t, 0, pos, c);
+        const uint32_t *p = S + addr(pos, c);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            uint32_t pos, c;
-            elem(t, j, pos, c);
-            x[j] = S[addr(pos, c)];
-        }
+        for (int j = 0; j < 16; ++j) x[j] = p[offset(j)];
     }
     // tw = the LEVEL table (levels 0 .. LOG_R - 1).
     // In a level of half-span h = s*2^lm the butterfly of group element v uses
