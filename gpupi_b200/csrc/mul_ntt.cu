@@ -251,12 +251,16 @@ template <class First, int LOG_R, int Q>
 __device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int coset, int log_k, int log_cols,
                                               const uint32_t *clo, const uint32_t *chi) {
     const uint32_t c = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset << log_k);
+    uint32_t d[4];   // independent lookups
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        d[k] = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * elem_delta<First, LOG_R>(1 << k, log_cols));
     for (uint32_t e = threadIdx.x; e < 16u * blocks; e += kThreads) {
         uint32_t w = PrimeC<Q>::r1;
         for (uint32_t k = 0; k < (e >> 4); ++k) w = norm<Q>(mont<Q>(w, c));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if ((e >> k) & 1u) w = mul_coset<Q, 0>(w, clo, chi, (uint32_t)coset * elem_delta<First, LOG_R>(1 << k, log_cols));
+            if ((e >> k) & 1u) w = norm<Q>(mont<Q>(w, d[k]));
         W[e] = w;
     }
 }
@@ -1124,18 +1128,49 @@ constexpr uint32_t kI02q = shoup_of(kI02, Prime<2>::p);
 constexpr uint32_t kI12q = shoup_of(kI12, Prime<2>::p);
 constexpr uint64_t kP0P1 = (uint64_t)Prime<0>::p * Prime<1>::p;
 
+// x = r0 + p0 t1 + p0 p1 t2 as three wide multiply-adds: none overflows
+// 64 bits (p0 t1 + r0 < 2^62, its sum with lo(p0 p1) t2 < 2^64).
 __device__ __forceinline__ void garner(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t (&out)[3]) {
     const uint32_t t1 = norm<1>(shoup<1>(sub_n<1>(r1, r0), kI01, kI01q));   // r0 < p0 < p1
     const uint32_t u = norm<2>(shoup<2>(sub_n<2>(r2, r0), kI02, kI02q));
     const uint32_t t2 = norm<2>(shoup<2>(sub_n<2>(u, t1), kI12, kI12q));    // t1 < p1 < p2
-    const unsigned __int128 x = (unsigned __int128)kP0P1 * t2 + (uint64_t)Prime<0>::p * t1 + r0;
-    out[0] = (uint32_t)x;
-    out[1] = (uint32_t)(x >> 32);
-    out[2] = (uint32_t)(x >> 64);
+    const uint64_t w = (uint64_t)t2 * (uint32_t)kP0P1 + ((uint64_t)t1 * Prime<0>::p + r0);
+    const uint64_t v = (uint64_t)t2 * (uint32_t)(kP0P1 >> 32) + (w >> 32);
+    out[0] = (uint32_t)w;
+    out[1] = (uint32_t)v;
+    out[2] = (uint32_t)(v >> 32);
 }
 
-constexpr int kCrtV = 4;
-constexpr uint32_t kCrtSpan = kThreads * kCrtV;   // 1024 limbs per tile
+// CRT and carry: each thread turns eight consecutive coefficients into eight
+// limbs and two words that spill into the next thread's.  Thread 0 of a CTA
+// repeats the last chunk of the previous tile for its spill, so a tile is 255
+// chunks (repeating it in the tile's first thread after its own chunk kept the
+// CTA waiting for a second round of loads).
+constexpr int kCrtV = 8;
+constexpr uint32_t kCrtSpan = (kThreads - 1) * kCrtV;   // 2040 limbs per tile
+
+// x += h (two words), carries through the eight words; returns the carry out
+__device__ __forceinline__ uint32_t add_words(uint32_t (&x)[kCrtV], uint32_t h0, uint32_t h1) {
+    uint32_t c;
+    asm("add.cc.u32 %0, %0, %9;\n\taddc.cc.u32 %1, %1, %10;\n\taddc.cc.u32 %2, %2, 0;\n\t"
+        "addc.cc.u32 %3, %3, 0;\n\taddc.cc.u32 %4, %4, 0;\n\taddc.cc.u32 %5, %5, 0;\n\t"
+        "addc.cc.u32 %6, %6, 0;\n\taddc.cc.u32 %7, %7, 0;\n\taddc.u32 %8, 0, 0;"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "=r"(c)
+        : "r"(h0), "r"(h1));
+    return c;
+}
+
+// words += c (96 bits) where words = {a1, a2} is what lies above the words
+// already given out: returns the next word, leaves the rest in {a1, a2}
+__device__ __forceinline__ uint32_t next_word(const uint32_t (&c)[3], uint32_t &a1, uint32_t &a2) {
+    uint32_t w, b1, b2;
+    asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, 0;"
+        : "=&r"(w), "=&r"(b1), "=&r"(b2)
+        : "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(a1), "r"(a2));
+    a1 = b1;
+    a2 = b2;
+    return w;
+}
 
 struct CrtArgs {
     const uint32_t *F;
@@ -1158,21 +1193,20 @@ struct CrtArgs {
     const RaggedRow *rows;   // ragged batch: each row's output place and length
 };
 
-// Adds limbs base .. base + kCrtV - 1 of (D << dshift) to the chunk sum S
-// (carries run into S's three top words, which stay far from overflowing).
+// Adds limbs base .. base + 7 of (D << dshift) to a chunk's words (a carry
+// runs into its spill words, which stay far from overflowing).
 __device__ __forceinline__ void crt_add_shifted(const CrtArgs &a, const uint32_t *Dr, int64_t base,
-                                                uint32_t (&S)[kCrtV + 3]) {
-    const int64_t sw = a.dshift >> 5;
-    const uint32_t sb = a.dshift & 31u;
+                                                uint32_t (&S)[kCrtV + 2]) {
+    const int64_t i0 = base - (int64_t)(a.dshift >> 5);
+    uint32_t prev = ((uint64_t)(i0 - 1) < (uint64_t)a.Ld) ? Dr[i0 - 1] : 0u;   // below 0 wraps
     uint64_t cy = 0;
 #pragma unroll
-    for (int v = 0; v < kCrtV + 3; ++v) {
+    for (int v = 0; v < kCrtV + 2; ++v) {
         uint32_t d = 0u;
         if (v < kCrtV) {
-            const int64_t i = base + v - sw;   // source limb of the low part
-            const uint32_t lo = (i >= 0 && i < (int64_t)a.Ld) ? Dr[i] : 0u;
-            const uint32_t hi = (sb && i - 1 >= 0 && i - 1 < (int64_t)a.Ld) ? Dr[i - 1] : 0u;
-            d = sb ? ((lo << sb) | (hi >> (32u - sb))) : lo;
+            const uint32_t cur = ((uint64_t)(i0 + v) < (uint64_t)a.Ld) ? Dr[i0 + v] : 0u;
+            d = __funnelshift_l(prev, cur, a.dshift & 31u);
+            prev = cur;
         }
         const uint64_t t = (uint64_t)S[v] + d + cy;
         S[v] = (uint32_t)t;
@@ -1198,87 +1232,98 @@ struct CrtRow {
     }
 };
 
-__device__ __forceinline__ void crt_chunk(const CrtRow &r, int64_t base, uint32_t (&S)[kCrtV + 3]) {
-    uint32_t c[kCrtV][3];
+// S = sum_v c_(base + v) 2^(32 v): eight words and the spill
+__device__ __forceinline__ void crt_chunk(const CrtRow &r, int64_t base, uint32_t (&S)[kCrtV + 2]) {
     uint64_t K;
-    if (base >= 0 && base + kCrtV <= (int64_t)r.ncoef && (1 << r.log_k) >= kCrtV) {
-        // the chunk lies in one block: one 128-bit load per prime (K and base are multiples of 4)
+    uint32_t a1 = 0u, a2 = 0u, c[3];
+    if (base >= 0 && base + kCrtV <= (int64_t)r.ncoef && r.log_k >= 3) {
+        // the chunk lies in one block: two 128-bit loads per prime (K and base are multiples of 8)
         const uint32_t *f = r.at((uint64_t)base, K);
-        const uint4 r0 = *reinterpret_cast<const uint4 *>(f);
-        const uint4 r1 = *reinterpret_cast<const uint4 *>(f + K);
-        const uint4 r2 = *reinterpret_cast<const uint4 *>(f + 2 * K);
-        garner(r0.x, r1.x, r2.x, c[0]);
-        garner(r0.y, r1.y, r2.y, c[1]);
-        garner(r0.z, r1.z, r2.z, c[2]);
-        garner(r0.w, r1.w, r2.w, c[3]);
-        chunk_sum3<kCrtV>(c, S);
-        return;
-    }
+        uint4 q[3][2];
 #pragma unroll
-    for (int v = 0; v < kCrtV; ++v) {
-        const int64_t i = base + v;
-        if (i >= 0 && i < (int64_t)r.ncoef) {
-            const uint32_t *f = r.at((uint64_t)i, K);
-            garner(f[0], f[K], f[2 * K], c[v]);
-        } else {
-            c[v][0] = c[v][1] = c[v][2] = 0u;
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) q[p][h] = *reinterpret_cast<const uint4 *>(f + p * K + 4 * h);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            garner(q[0][h].x, q[1][h].x, q[2][h].x, c);
+            S[4 * h] = next_word(c, a1, a2);
+            garner(q[0][h].y, q[1][h].y, q[2][h].y, c);
+            S[4 * h + 1] = next_word(c, a1, a2);
+            garner(q[0][h].z, q[1][h].z, q[2][h].z, c);
+            S[4 * h + 2] = next_word(c, a1, a2);
+            garner(q[0][h].w, q[1][h].w, q[2][h].w, c);
+            S[4 * h + 3] = next_word(c, a1, a2);
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < kCrtV; ++v) {
+            const int64_t i = base + v;
+            c[0] = c[1] = c[2] = 0u;
+            if (i >= 0 && i < (int64_t)r.ncoef) {
+                const uint32_t *f = r.at((uint64_t)i, K);
+                garner(f[0], f[K], f[2 * K], c);
+            }
+            S[v] = next_word(c, a1, a2);
         }
     }
-    chunk_sum3<kCrtV>(c, S);
+    S[kCrtV] = a1;
+    S[kCrtV + 1] = a2;
 }
 
+// Bound by HBM (12 bytes read and 4 written per limb): 2^28 limbs 1.18 -> 0.70
+// ms (4.3 GB, 6.1 TB/s); 111 instructions per limb before (four coefficients per thread, 64-bit
+// sums of their words, scalar stores).
 __global__ void __launch_bounds__(kThreads) k_crt(CrtArgs a) {
     __shared__ uint32_t sg[kThreads / 32], sp[kThreads / 32];
-    __shared__ uint32_t spill[kThreads / 32][3];
+    __shared__ uint32_t spill[kThreads / 32][2];
     const uint32_t tile = blockIdx.x;
-    const uint64_t row = tile / a.tiles;
-    const uint32_t t = tile - (uint32_t)row * a.tiles;
+    const uint32_t row = tile / a.tiles;
+    const uint32_t t = tile - row * a.tiles;
     const uint32_t Lc = a.rows ? a.rows[row].La + a.rows[row].Lb : a.Lc;
-    const CrtRow cr{a.F + ((row * (uint64_t)a.M * 3) << a.log_k), a.F2 ? a.F2 + ((row * 3) << a.log_k2) : nullptr,
-                    a.log_k, a.log_k2, a.rows ? Lc - 1u : a.ncoef};
-    const int64_t base = (int64_t)t * kCrtSpan + threadIdx.x * kCrtV;
+    const CrtRow cr{a.F + (((uint64_t)row * a.M * 3) << a.log_k),
+                    a.F2 ? a.F2 + (((uint64_t)row * 3) << a.log_k2) : nullptr, a.log_k, a.log_k2,
+                    a.rows ? Lc - 1u : a.ncoef};
+    const int64_t base = (int64_t)t * kCrtSpan + ((int)threadIdx.x - 1) * kCrtV;
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    uint32_t S[kCrtV + 3];
-    const uint32_t *Dr = a.D ? a.D + row * a.sD : nullptr;
+    uint32_t S[kCrtV + 2];
     crt_chunk(cr, base, S);
-    if (Dr) crt_add_shifted(a, Dr, base, S);
-    // words of the previous chunk's sum that land in this chunk: from the
-    // previous lane, from the previous warp's last lane, and for the tile's
-    // first thread from the last chunk of the previous tile (recomputed)
-    uint32_t H[3];
-    H[0] = __shfl_up_sync(0xffffffffu, S[kCrtV], 1);
-    H[1] = __shfl_up_sync(0xffffffffu, S[kCrtV + 1], 1);
-    H[2] = __shfl_up_sync(0xffffffffu, S[kCrtV + 2], 1);
+    if (a.D) crt_add_shifted(a, a.D + row * a.sD, base, S);
+    // words of the previous chunk's sum that land in this chunk
+    uint32_t h0 = __shfl_up_sync(0xffffffffu, S[kCrtV], 1);
+    uint32_t h1 = __shfl_up_sync(0xffffffffu, S[kCrtV + 1], 1);
     if (lane == 31) {
         spill[warp][0] = S[kCrtV];
         spill[warp][1] = S[kCrtV + 1];
-        spill[warp][2] = S[kCrtV + 2];
-    }
-    if (threadIdx.x == 0) {
-        uint32_t Sp[kCrtV + 3];
-        crt_chunk(cr, base - kCrtV, Sp);
-        if (Dr) crt_add_shifted(a, Dr, base - kCrtV, Sp);
-        H[0] = Sp[kCrtV];
-        H[1] = Sp[kCrtV + 1];
-        H[2] = Sp[kCrtV + 2];
     }
     __syncthreads();
     if (lane == 0 && warp > 0) {
-        H[0] = spill[warp - 1][0];
-        H[1] = spill[warp - 1][1];
-        H[2] = spill[warp - 1][2];
+        h0 = spill[warp - 1][0];
+        h1 = spill[warp - 1][1];
     }
     uint32_t X[kCrtV];
-    const uint32_t g = chunk_add_spill<kCrtV>(S, H, X);
-    bool p = true;
 #pragma unroll
-    for (int v = 0; v < kCrtV; ++v) p = p && (X[v] == 0xffffffffu) && (base + v < (int64_t)Lc);
-    const BlockCarry bc = block_resolve<kThreads / 32>(g != 0u, p, sg, sp);
-    chunk_increment<kCrtV>(X, bc.cin);
+    for (int v = 0; v < kCrtV; ++v) X[v] = S[v];
+    bool g = add_words(X, h0, h1) != 0u, p = base + kCrtV <= (int64_t)Lc;
+#pragma unroll
+    for (int v = 0; v < kCrtV; ++v) p = p && (X[v] == 0xffffffffu);
+    if (threadIdx.x == 0) {   // the previous tile's chunk: neither generates nor stops a carry
+        g = false;
+        p = true;
+    }
+    const BlockCarry bc = block_resolve<kThreads / 32>(g, p, sg, sp);
+    add_words(X, bc.cin, 0u);
     uint32_t *out = a.C + (a.rows ? a.rows[row].offC : row * a.sC);
+    if (threadIdx.x > 0) {
+        if (base + kCrtV <= (int64_t)Lc && ((uintptr_t)(out + base) & 15u) == 0u) {
+            *reinterpret_cast<uint4 *>(out + base) = make_uint4(X[0], X[1], X[2], X[3]);
+            *reinterpret_cast<uint4 *>(out + base + 4) = make_uint4(X[4], X[5], X[6], X[7]);
+        } else {
 #pragma unroll
-    for (int v = 0; v < kCrtV; ++v)
-        if (base + v < (int64_t)Lc) out[base + v] = X[v];
+            for (int v = 0; v < kCrtV; ++v)
+                if (base + v < (int64_t)Lc) out[base + v] = X[v];
+        }
+    }
     if (a.tiles > 1u && threadIdx.x == 0) a.flags[tile] = bc.G | (bc.P << 1);
 }
 
