@@ -79,12 +79,16 @@ __host__ __device__ inline uint32_t up128(uint32_t x) { return (x + 127u) & ~127
 // writes one row of all eight planes per eight lanes).
 __host__ __device__ inline uint32_t plane_rows(uint32_t Q, uint32_t N) { return (N + Q - 1u) | 1u; }
 
+// Word of c_k: 4 words of padding per 32, so that the 16-byte reads of the
+// limb pass, 64 bytes apart from lane to lane, fall in different banks.
+__host__ __device__ inline uint32_t cs_at(uint32_t k) { return k + 4u * (k >> 5); }
+
 __host__ __device__ inline Layout layout_of(uint32_t maxQ, uint32_t maxN) {
     Layout l;
     l.abuf = 0u;
     const uint32_t abytes = up128(128u * maxQ + 160u);
     l.p = abytes;
-    const uint32_t psz = 16u * (128u * maxQ + 112u), csz = 4u * 128u * maxN;
+    const uint32_t psz = 16u * (128u * maxQ + 112u), csz = 4u * cs_at(128u * maxN);
     l.planes = l.p + up128(psz > csz ? psz : csz);
     l.total = l.planes + 8u * 16u * plane_rows(maxQ, maxN);
     return l;
@@ -154,7 +158,7 @@ constexpr uint32_t kProbeLimit = 1u << 12;  // polls of the self-test's never-co
 // S_L = c_4L + c_(4L+1) 2^8 + c_(4L+2) 2^16 + c_(4L+3) 2^24 (0 beyond the product)
 __device__ __forceinline__ uint64_t limb_sum(const uint32_t *cs, uint32_t L, uint32_t Lc) {
     if (L >= Lc) return 0ull;
-    const uint4 c = *reinterpret_cast<const uint4 *>(cs + 4u * L);
+    const uint4 c = *reinterpret_cast<const uint4 *>(cs + cs_at(4u * L));
     return (uint64_t)c.x + ((uint64_t)c.y << 8) + ((uint64_t)c.z << 16) + ((uint64_t)c.w << 24);
 }
 
@@ -229,18 +233,25 @@ __global__ void __launch_bounds__(kThreads, 8)
         }
         __syncthreads();
         // 3. P: stored row rr is P[rr - 112] = a[rr - 127 .. rr - 112], i.e.
-        //    abuf bytes rr + 1 .. rr + 16
-        for (uint32_t rr = tid; rr < prow_n; rr += kThreads) {
-            const uint32_t b0 = rr + 1u, i0 = b0 >> 2, sh8 = 8u * (b0 & 3u);
+        //    abuf bytes rr + 1 .. rr + 16.  A thread builds rows 4k .. 4k + 3
+        //    from the five words they share (a funnel shift by 8 (r + 1) bits,
+        //    32 for the last) and writes them starting with another one every
+        //    two lanes, so that the lanes' 16-byte stores, 64 bytes apart, fall
+        //    in different banks.
+        for (uint32_t k = tid; k < prow_n / 4u; k += kThreads) {
             uint32_t w[5];
 #pragma unroll
-            for (int e = 0; e < 5; ++e) w[e] = abuf[i0 + e];
-            uint4 v;
-            v.x = __funnelshift_r(w[0], w[1], sh8);
-            v.y = __funnelshift_r(w[1], w[2], sh8);
-            v.z = __funnelshift_r(w[2], w[3], sh8);
-            v.w = __funnelshift_r(w[3], w[4], sh8);
-            *reinterpret_cast<uint4 *>(P + 16u * rr) = v;
+            for (int e = 0; e < 5; ++e) w[e] = abuf[k + e];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j) {
+                const uint32_t r = (j + (lane >> 1)) & 3u, sh8 = 8u * (r + 1u);
+                uint4 v;
+                v.x = __funnelshift_rc(w[0], w[1], sh8);
+                v.y = __funnelshift_rc(w[1], w[2], sh8);
+                v.z = __funnelshift_rc(w[2], w[3], sh8);
+                v.w = __funnelshift_rc(w[3], w[4], sh8);
+                *reinterpret_cast<uint4 *>(P + 16u * (4u * k + r)) = v;
+            }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         fence_before();
@@ -288,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 8)
             break;
         }
         fence_after();
-        // 6. D -> shared memory: cs[128u + s] = c_(128u + s) (the MMAs no
+        // 6. D -> shared memory: cs[cs_at(128u + s)] = c_(128u + s) (the MMAs no
         //    longer read P, whose space this reuses); warp w reads lanes
         //    32w .. 32w + 31 of tensor memory
         {
@@ -297,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 8)
                 uint32_t r[16];
                 tmem_ld16(tmem + ((32u * warp) << 16) + 16u * g, r);
 #pragma unroll
-                for (int e = 0; e < 16; ++e) cs[128u * (16u * g + e) + s] = r[e];
+                for (int e = 0; e < 16; ++e) cs[cs_at(128u * (16u * g + e) + s)] = r[e];
             }
         }
         fence_before();
@@ -308,15 +319,19 @@ __global__ void __launch_bounds__(kThreads, 8)
         const uint32_t lt = (1u << lane) - 1u, wmask = (1u << warp) - 1u;
         for (uint32_t base = 0; base < Lc; base += 4u * kThreads) {
             const uint32_t L0 = base + 4u * tid;
-            uint64_t prev = (L0 > 0u) ? limb_sum(cs, L0 - 1u, Lc) : 0ull;
+            uint64_t S[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) S[v] = limb_sum(cs, L0 + v, Lc);
+            // the upper word of the limb sum below: the previous lane's last
+            uint32_t below = __shfl_up_sync(0xffffffffu, (uint32_t)(S[3] >> 32), 1);
+            if (lane == 0u) below = (L0 > 0u) ? (uint32_t)(limb_sum(cs, L0 - 1u, Lc) >> 32) : 0u;
             uint32_t X[4], cy = 0u;
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                const uint64_t S = limb_sum(cs, L0 + v, Lc);
-                const uint64_t t = (uint64_t)(uint32_t)S + (prev >> 32) + cy;
+                const uint64_t t = (uint64_t)(uint32_t)S[v] + below + cy;
                 X[v] = (uint32_t)t;
                 cy = (uint32_t)(t >> 32);
-                prev = S;
+                below = (uint32_t)(S[v] >> 32);
             }
             const bool p = (X[0] & X[1] & X[2] & X[3]) == 0xffffffffu;
             const BlockCarry bc = block_resolve<kWarps>(cy != 0u, p, sg, sp);
@@ -326,9 +341,13 @@ __global__ void __launch_bounds__(kThreads, 8)
             for (int k = 0; k < kWarps; ++k) wp |= sp[k] << k;
             const bool prev_all = ((pm & lt) == lt) && ((wp & wmask) == wmask);
             chunk_increment<4>(X, bc.cin | (prev_all ? pass_cin : 0u));
+            if (L0 + 4u <= Lc && ((uintptr_t)(out + L0) & 15u) == 0u) {
+                *reinterpret_cast<uint4 *>(out + L0) = make_uint4(X[0], X[1], X[2], X[3]);
+            } else {
 #pragma unroll
-            for (int v = 0; v < 4; ++v)
-                if (L0 + v < Lc) out[L0 + v] = X[v];
+                for (int v = 0; v < 4; ++v)
+                    if (L0 + v < Lc) out[L0 + v] = X[v];
+            }
             pass_cin = bc.G | (bc.P & pass_cin);
             __syncthreads();
         }
