@@ -20,10 +20,11 @@
 // broadcast), then the CRT tile flags.
 //
 // Passes (four-step decomposition K = R1 [* R2] * C, C = 4096):
-//   k_cols_r<first>   load limbs (fold + twist for cosets), R1-point DIF
-//                     down each column of a 4096-residue tile, twist by
+//   k_fold            operands of cosets, and longer than K: fold and twist
+//   k_cols_r<first>   load limbs (residues after k_fold), R1-point DIF down
+//                     each column of a 4096-residue tile, twist by
 //                     w_K^(col * bitrev(pos)), store
-//   k_cols_r          same on each segment for R2 (sizes above 2^21)
+//   k_cols_r          same on each segment for R2 (sizes above 2^22)
 //   k_rows_r          C-point DIF of the A and B segments, pointwise product
 //                     * K^-1, C-point inverse DIT, store
 //   k_cols_r<inv>     untwist + inverse DIT on columns, mirror order
@@ -114,22 +115,18 @@ __device__ __forceinline__ int grid_prime(uint64_t &b) {
 }
 
 struct ColsArgs {
-    const uint32_t *X;   // limbs (first forward pass only)
+    const uint32_t *X;   // limbs (first pass of operands that need no folding only)
     uint64_t sX;
     uint32_t Lx;
-    uint32_t nb;         // K-limb blocks of X folded into each coset (first pass)
     uint32_t *F;         // workspace of this operand: F[vrow][q][K]
     int log_k, log_s;
-    int M;               // cosets per row
-    int coset0;          // the first of them (1 for the second part of a two-part product)
     int scaled;          // inverse pass: times K^-1 R as well (the row pass leaves products x y R^-1)
-    // second operand of a paired forward pass (same shape, same tile)
+    // second operand of a paired pass (same shape, same tile)
     const uint32_t *X2;
     uint64_t sX2;
     uint32_t Lx2;
-    uint32_t nb2;
     uint32_t *F2;
-    const RaggedRow *rows;   // first pass of a ragged batch: per-row operands (nb, nb2 per row)
+    const RaggedRow *rows;   // first pass of a ragged batch: per-row operands
     int side;                // of X; X2 is side 1
 };
 
@@ -236,93 +233,150 @@ __device__ __forceinline__ void twist16(uint32_t (&x)[16], uint32_t (&y)[16], ui
     }
 }
 
-// The 16 first-pass residues of one operand: its limbs, or its residues mod
-// x^K - c, c = g^(coset K), twisted by g^(coset i) (coset 0: plain folding
-// mod x^K - 1 when the operand is longer than K).
-//
-// Residue j of a thread sits delta_j above its first one, i_0, and the bits of
-// j add up in delta_j (elem_delta), so it is g^(coset i_0) sum_b X_(b, j) W[b][j]
-// over the K-limb blocks b, with W[b][j] = c^b g^(coset delta_j) the same for the
-// whole CTA (coset_weights, in shared memory).  The sum of 64-bit products is
-// kept below 2^32 p by reducing its upper word only, and reduced once at the
-// end: per block one wide multiply-add and one reduction instead of a modular
-// product, a sum and their reductions, and no chain of powers.
-template <class First, int LOG_R, int Q>
-__device__ __forceinline__ void coset_weights(uint32_t *W, uint32_t blocks, int coset, int log_k, int log_cols,
-                                              const uint32_t *clo, const uint32_t *chi) {
-    const uint32_t c = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset << log_k);
-    uint32_t d[4];   // independent lookups
+// How a first pass gets its limbs: in general (an operand of at most K limbs),
+// from operands that fill at most the lower half of their K points (a balanced
+// product at one power-of-two transform: half the loads, and the first level
+// multiplies without adding), or through a ragged batch's descriptors (apart
+// from the others: operand addresses that come from memory are not uniform to
+// the compiler, and every access then needs 64-bit sums).  Operands that have
+// to be folded or twisted go through k_fold first.
+enum Load { kGeneral, kHalf, kRagged };
+
+template <class First, int LOG_R, int Q, bool HALF>
+__device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx, int log_cols,
+                                           uint32_t i0) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        d[k] = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * elem_delta<First, LOG_R>(1 << k, log_cols));
-    for (uint32_t e = threadIdx.x; e < 16u * blocks; e += kThreads) {
-        uint32_t w = PrimeC<Q>::r1;
-        for (uint32_t k = 0; k < (e >> 4); ++k) w = norm<Q>(mont<Q>(w, c));
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if ((e >> k) & 1u) w = norm<Q>(mont<Q>(w, d[k]));
-        W[e] = w;
+    for (int j = 0; j < 16; ++j) {
+        const uint32_t i = i0 + elem_delta<First, LOG_R>(j, log_cols);
+        const bool upper = HALF && ((j >> (First::kB - 1)) & 1);   // positions R / 2 .. R - 1
+        x[j] = (!upper && i < Lx) ? reduce_limb<Q>(__ldg(word_at(xr, i))) : 0u;
     }
 }
 
-template <class First, int LOG_R, int Q, bool HALF>
-__device__ __forceinline__ void load_limbs(uint32_t (&x)[16], const uint32_t *xr, uint32_t Lx, uint32_t nb,
-                                           uint64_t K, int log_cols, uint32_t i0, int coset, const uint32_t *W,
-                                           uint32_t f) {
-    if (HALF || (nb == 1u && coset == 0)) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const uint32_t i = i0 + elem_delta<First, LOG_R>(j, log_cols);
-            const bool upper = HALF && ((j >> (First::kB - 1)) & 1);   // positions R / 2 .. R - 1
-            x[j] = (!upper && i < Lx) ? reduce_limb<Q>(__ldg(word_at(xr, i))) : 0u;
-        }
+// ---------------------------------------------------------------------------
+// Residues of an operand X mod x^K - c_i, c_i = g^(iK), twisted by g^(ij), for
+// the cosets i = coset0 .. coset0 + M - 1 of each row: F[vrow][q][K], which the
+// column passes then transform in place.  A thread makes four consecutive
+// positions of every coset for one prime:
+//     residue (i, j + v) = g^(ij) sum_b X[j + v + b K] W[i][b][v],
+//     W[i][b][v] = c_i^b g^(iv)  (in shared memory, the same for the CTA),
+// so its limbs are loaded once for all cosets, g^(ij) is a chain over i, and a
+// block costs one wide multiply-add and one reduction: the 64-bit sum is kept
+// below 2^32 p by reducing its upper word only, and reduced once at the end.
+// Inside the first column pass, where every coset's CTA loaded all blocks anew,
+// the folding of eight cosets of four blocks (2^27 x 2^27 limbs) took 7.5 of
+// the pass's 10.2 ms for both operands; here it takes 1.29 ms an operand and
+// the pass on the residues 2.87 ms.
+// ---------------------------------------------------------------------------
+struct FoldArgs {
+    const uint32_t *X;
+    uint64_t sX;
+    uint32_t Lx;
+    uint32_t nb;   // K-limb blocks of the longest row
+    uint32_t *F;
+    int log_k;
+    int M, coset0;
+    const RaggedRow *rows;
+    int side;
+};
+constexpr int kFoldV = 4;
+constexpr int kFoldRegs = 4;   // blocks whose limbs a thread holds in registers
+
+// limbs i .. i + 3 of a row, 0 past its end
+__device__ __forceinline__ void limbs4(const LimbRow &X, uint32_t i, uint32_t (&v)[kFoldV]) {
+    const uint32_t *p = X.p + i;
+    if (i + kFoldV <= X.L && ((uintptr_t)p & 15u) == 0u) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+        v[0] = q.x;
+        v[1] = q.y;
+        v[2] = q.z;
+        v[3] = q.w;
         return;
     }
-    if constexpr (!HALF) {
-        // two halves of eight residues: their sums and loads fit the registers
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t lo[8], hi[8];
+    for (int k = 0; k < kFoldV; ++k) v[k] = (i + k < X.L) ? __ldg(p + k) : 0u;
+}
+
+template <int Q, bool REGS>
+__device__ __forceinline__ void fold_body(const NttParams &P, const FoldArgs &a, uint64_t b, uint32_t *W) {
+    const uint32_t tiles = (1u << a.log_k) / (kThreads * kFoldV);
+    const uint64_t row = b / tiles;
+    const uint32_t j = ((uint32_t)(b - row * tiles) * kThreads + threadIdx.x) * kFoldV;
+    const LimbRow X = limb_row(a.rows, a.side, a.X, a.sX, a.Lx, row);
+    const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q), *chi = coset_hi_ptr(P.tab, 0, Q);
+    uint32_t v[REGS ? kFoldRegs : 1][kFoldV];
+    if constexpr (REGS) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) lo[j] = hi[j] = 0u;
-#pragma unroll 1
-            for (uint32_t blk = 0; blk < nb; ++blk) {
-                const uint32_t *xb = xr + blk * K;
-                const uint32_t left = Lx - blk * (uint32_t)K;   // > 0
-                const uint4 wa = *reinterpret_cast<const uint4 *>(W + 16u * blk + 8u * h);
-                const uint4 wb = *reinterpret_cast<const uint4 *>(W + 16u * blk + 8u * h + 4u);
-                const uint32_t w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-                uint32_t v[8];
+        for (int k = 0; k < kFoldRegs; ++k)
+            limbs4(X, j + ((uint32_t)k << a.log_k), v[k]);   // beyond the row's blocks: zeros
+    }
+    for (uint32_t e = threadIdx.x; e < (uint32_t)a.M * a.nb * kFoldV; e += kThreads) {
+        const uint32_t u = e & (kFoldV - 1u), rest = e / kFoldV;
+        const uint32_t i = (uint32_t)a.coset0 + rest / a.nb, blk = rest % a.nb;
+        uint32_t w = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, i * u);
+        const uint32_t c = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, i << a.log_k);
+        for (uint32_t k = 0; k < blk; ++k) w = norm<Q>(mont<Q>(w, c));
+        W[e] = w;
+    }
+    const uint32_t h = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, j);   // g^j
+    uint32_t f = PrimeC<Q>::r1;                                         // g^(ij)
+    if (a.coset0) f = h;
+    __syncthreads();
+    uint32_t *F = a.F + (((row * a.M * 3 + Q) << a.log_k) + j);
+    const uint32_t nb = REGS ? a.nb : (X.L + (1u << a.log_k) - 1u) >> a.log_k;
+    for (int i = 0; i < a.M; ++i) {
+        uint32_t lo[kFoldV], hi[kFoldV];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t i = i0 + elem_delta<First, LOG_R>(8 * h + j, log_cols);
-                    v[j] = (i < left) ? __ldg(word_at(xb, i)) : 0u;
-                }
+        for (int k = 0; k < kFoldV; ++k) lo[k] = hi[k] = 0u;
+        auto add = [&](const uint32_t (&x)[kFoldV], uint32_t blk) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(W + ((uint32_t)i * a.nb + blk) * kFoldV);
+            const uint32_t w[kFoldV] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint64_t s = (uint64_t)v[j] * w[j] + (((uint64_t)hi[j] << 32) | lo[j]);
-                    lo[j] = (uint32_t)s;
-                    hi[j] = norm<Q>((uint32_t)(s >> 32));   // < p again
-                }
+            for (int k = 0; k < kFoldV; ++k) {
+                const uint64_t s = (uint64_t)x[k] * w[k] + (((uint64_t)hi[k] << 32) | lo[k]);
+                lo[k] = (uint32_t)s;
+                hi[k] = norm<Q>((uint32_t)(s >> 32));   // < p again
             }
+        };
+        if constexpr (REGS) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t r = redc<Q>(lo[j], hi[j]);   // < 2p
-                x[8 * h + j] = norm<Q>(mont<Q>(r, f));
+            for (uint32_t blk = 0; blk < (uint32_t)kFoldRegs; ++blk)
+                if (blk < nb) add(v[blk], blk);
+        } else {
+            for (uint32_t blk = 0; blk < nb; ++blk) {
+                uint32_t x[kFoldV];
+                limbs4(X, j + (blk << a.log_k), x);
+                add(x, blk);
             }
         }
+        uint32_t r[kFoldV];
+#pragma unroll
+        for (int k = 0; k < kFoldV; ++k) r[k] = norm<Q>(mont<Q>(redc<Q>(lo[k], hi[k]), f));
+        *reinterpret_cast<uint4 *>(F + ((uint64_t)(3 * i) << a.log_k)) = make_uint4(r[0], r[1], r[2], r[3]);
+        f = norm<Q>(mont<Q>(f, h));
     }
+}
+
+template <bool REGS>
+__global__ void __launch_bounds__(kThreads) k_fold(NttParams P, FoldArgs a) {
+    __shared__ __align__(16) uint32_t W[kMaxCosets * kMaxCosets * kFoldV];
+    uint64_t b;
+    const int q = grid_prime(b);
+    if (q == 0)
+        fold_body<0, REGS>(P, a, b, W);
+    else if (q == 1)
+        fold_body<1, REGS>(P, a, b, W);
+    else
+        fold_body<2, REGS>(P, a, b, W);
 }
 
 // Column pass: R = 2^LOG_R (<= 512) points per column, TC = 4096 / R columns
 // per CTA; segment of S = 2^log_s points viewed as [R][S/R].  PAIR: the
 // forward pass of A and B together (same tile, shared twiddles and twists).
-// HALF (first pass): each operand fills at most the lower half of its K points
-// (a balanced product at one power-of-two transform): half the loads, and the
-// first level multiplies without adding.
-template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, bool HALF, int Q>
+template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, Load LOAD, int Q>
 __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a, uint64_t b, uint32_t *Sm,
                                           uint32_t *Sm2, uint2 *tw) {
+    constexpr bool HALF = LOAD == kHalf;
     constexpr int LOG_TC = 12 - LOG_R;
     constexpr int NS = StagePlan<LOG_R>::n;
     using First = typename ExecStage<LOG_R, LOG_TC, INVERSE, 0>::S;
@@ -332,19 +386,10 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
     const uint32_t nseg = 1u << (a.log_k - a.log_s);
     uint32_t ct, seg;
     uint64_t vrow;
-    if constexpr (FROM_LIMBS) {
-        // virtual row fastest: the cosets of one tile run back to back and
-        // share its limbs in L2 (the first pass covers the whole transform)
-        const uint64_t vrows = (gridDim.x / kPrimes) / ctiles;
-        vrow = b % vrows;
-        ct = (uint32_t)(b / vrows);
-        seg = 0u;
-    } else {
-        ct = (uint32_t)(b % ctiles);
-        b /= ctiles;
-        seg = (uint32_t)(b % nseg);
-        vrow = b / nseg;
-    }
+    ct = (uint32_t)(b % ctiles);
+    b /= ctiles;
+    seg = (uint32_t)(b % nseg);
+    vrow = b / nseg;
     const int dir = INVERSE ? 1 : 0;
     const uint64_t K = 1ull << a.log_k;
     const uint2 *twhi = root_hi_ptr(P.tab, dir, Q);
@@ -362,28 +407,13 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
     const uint32_t i0 = (pos0 << log_cols) + c0 + col0;   // this thread's first residue
     uint32_t x[16], y[16];
     if constexpr (FROM_LIMBS) {
-        const uint64_t row = vrow / (uint32_t)a.M;
-        const int coset = a.coset0 + (int)(vrow - row * (uint32_t)a.M);
-        const LimbRow X = limb_row(a.rows, a.side, a.X, a.sX, a.Lx, row);
-        LimbRow Y = X;
-        uint32_t nb = a.nb, nb2 = a.nb2;
-        if constexpr (PAIR) Y = limb_row(a.rows, 1, a.X2, a.sX2, a.Lx2, row);
-        if (a.rows) {
-            nb = (uint32_t)((X.L + K - 1) >> a.log_k);
-            nb2 = (uint32_t)((Y.L + K - 1) >> a.log_k);
+        const RaggedRow *rows = LOAD == kRagged ? a.rows : nullptr;
+        const LimbRow X = limb_row(rows, a.side, a.X, a.sX, a.Lx, vrow);
+        load_limbs<First, LOG_R, Q, HALF>(x, X.p, X.L, log_cols, i0);
+        if constexpr (PAIR) {
+            const LimbRow Y = limb_row(rows, 1, a.X2, a.sX2, a.Lx2, vrow);
+            load_limbs<First, LOG_R, Q, HALF>(y, Y.p, Y.L, log_cols, i0);
         }
-        const uint32_t blocks = PAIR ? max(nb, nb2) : nb;
-        uint32_t f = 0u;    // g^(coset i_0), Montgomery form
-        uint32_t *W = Sm;   // weights in the tile, before its first use
-        if (!HALF && (coset || blocks > 1u)) {
-            const uint32_t *clo = coset_lo_ptr(P.tab, 0, Q);
-            const uint32_t *chi = coset_hi_ptr(P.tab, 0, Q);
-            f = mul_coset<Q, 0>(PrimeC<Q>::r1, clo, chi, (uint32_t)coset * i0);
-            coset_weights<First, LOG_R, Q>(W, blocks, coset, a.log_k, log_cols, clo, chi);
-            __syncthreads();
-        }
-        load_limbs<First, LOG_R, Q, HALF>(x, X.p, X.L, nb, K, log_cols, i0, coset, W, f);
-        if constexpr (PAIR) load_limbs<First, LOG_R, Q, HALF>(y, Y.p, Y.L, nb2, K, log_cols, i0, coset, W, f);
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -396,7 +426,7 @@ __device__ __forceinline__ void cols_body(const NttParams &P, const ColsArgs &a,
             twist16<First, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, one, a.scaled != 0);
         }
     }
-    __syncthreads();   // twiddle table ready (and the weights read)
+    __syncthreads();   // twiddle table ready
     run_stages_pair<LOG_R, LOG_TC, INVERSE, Q, 0, PAIR, CtaSync, HALF>(x, y, Sm, Sm2, t, tw, CtaSync{});
     if constexpr (!INVERSE) twist16<Last, LOG_R, Q, PAIR>(x, y, t, c0, twist_shift, twlo, twhi, PrimeC<Q>::r1, false);
     uint32_t pos1, c1;
@@ -419,7 +449,7 @@ constexpr size_t cols_smem_bytes() {   // one or two padded tiles + the twiddle 
 // operands' residues, and for the first of them a few words spill, but the
 // extra resident warps hide more of the limb and tile latency (first pass of
 // a 2^24 x 2^24-limb product 0.589 -> 0.541 ms against three CTAs per SM).
-template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, bool HALF>
+template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, Load LOAD>
 __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a) {
     extern __shared__ uint4 cols_smem[];
     uint32_t *Sm = reinterpret_cast<uint32_t *>(cols_smem);
@@ -428,11 +458,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a)
     uint64_t b;
     const int q = grid_prime(b);
     if (q == 0)
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 0>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, LOAD, 0>(P, a, b, Sm, Sm2, tw);
     else if (q == 1)
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 1>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, LOAD, 1>(P, a, b, Sm, Sm2, tw);
     else
-        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, HALF, 2>(P, a, b, Sm, Sm2, tw);
+        cols_body<LOG_R, FROM_LIMBS, INVERSE, PAIR, LOAD, 2>(P, a, b, Sm, Sm2, tw);
 }
 
 __device__ __forceinline__ void swap16(uint32_t (&x)[16], uint32_t (&y)[16]) {
@@ -1385,37 +1415,37 @@ constexpr int kPairMinLogR = 5;
 // pass against 0.41 ms in two.
 constexpr int kOnePassMaxLog = 10;
 
-template <int LOG_R, bool FL, bool INV, bool PAIR, bool HALF>
+template <int LOG_R, bool FL, bool INV, bool PAIR, Load LOAD>
 static void cols_launch(unsigned blocks, const NttParams &P, const ColsArgs &a, cudaStream_t st) {
     constexpr size_t smem = cols_smem_bytes<LOG_R, PAIR>();
     static bool attr = false;
     if (!attr) {
         if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_cols_r<LOG_R, FL, INV, PAIR, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(k_cols_r<LOG_R, FL, INV, PAIR, LOAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         attr = true;
     }
-    k_cols_r<LOG_R, FL, INV, PAIR, HALF><<<blocks, kThreads, smem, st>>>(P, a);
+    k_cols_r<LOG_R, FL, INV, PAIR, LOAD><<<blocks, kThreads, smem, st>>>(P, a);
 }
 
-template <bool FL, bool INV, bool PAIR, bool HALF = false>
+template <bool FL, bool INV, bool PAIR, Load LOAD = kGeneral>
 static void cols_r_dispatch(int log_r, unsigned blocks, const NttParams &P, const ColsArgs &a, cudaStream_t st) {
     if constexpr (!PAIR) {
         switch (log_r) {
-            case 1: cols_launch<1, FL, INV, false, HALF>(blocks, P, a, st); return;
-            case 2: cols_launch<2, FL, INV, false, HALF>(blocks, P, a, st); return;
-            case 3: cols_launch<3, FL, INV, false, HALF>(blocks, P, a, st); return;
-            case 4: cols_launch<4, FL, INV, false, HALF>(blocks, P, a, st); return;
+            case 1: cols_launch<1, FL, INV, false, LOAD>(blocks, P, a, st); return;
+            case 2: cols_launch<2, FL, INV, false, LOAD>(blocks, P, a, st); return;
+            case 3: cols_launch<3, FL, INV, false, LOAD>(blocks, P, a, st); return;
+            case 4: cols_launch<4, FL, INV, false, LOAD>(blocks, P, a, st); return;
             default: break;
         }
     }
     switch (log_r) {
-        case 5: cols_launch<5, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
-        case 6: cols_launch<6, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
-        case 7: cols_launch<7, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
-        case 8: cols_launch<8, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
-        case 9: cols_launch<9, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
-        default: cols_launch<10, FL, INV, PAIR, HALF>(blocks, P, a, st); break;
+        case 5: cols_launch<5, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
+        case 6: cols_launch<6, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
+        case 7: cols_launch<7, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
+        case 8: cols_launch<8, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
+        case 9: cols_launch<9, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
+        default: cols_launch<10, FL, INV, PAIR, LOAD>(blocks, P, a, st); break;
     }
 }
 
@@ -1426,24 +1456,32 @@ static void launch_cols_r(bool from_limbs, bool inverse, bool pair, int log_r, c
     const uint64_t nseg = 1ull << (a.log_k - a.log_s);
     const unsigned blocks = (unsigned)(vrows * kPrimes * nseg * ctiles);
     // algorithmic bytes: 4 B per residue read and written (3 primes per
-    // point); the first pass reads the limbs instead (once per coset)
+    // point); a first pass on limbs reads those instead
     const double K = (double)(1ull << a.log_k);
     const double limbs = (double)a.Lx + (pair ? (double)a.Lx2 : 0.0);
     const double ops = pair ? 2.0 : 1.0;
-    const double bytes = from_limbs ? (4.0 * limbs * (double)vrows / a.M + 12.0 * K * (double)vrows * ops)
+    const double bytes = from_limbs ? (4.0 * limbs * (double)vrows + 12.0 * K * (double)vrows * ops)
                                     : 24.0 * K * (double)vrows * ops;
     KernelTimed kt(from_limbs ? "ntt_cols_fwd_first" : (inverse ? "ntt_cols_inv" : "ntt_cols_fwd"), bytes);
     if (from_limbs) {
         const uint64_t half = 1ull << (a.log_k - 1);
-        const bool lower = a.M == 1 && !a.coset0 && !a.rows && a.Lx <= half && (!pair || a.Lx2 <= half);
-        if (pair && lower)
-            cols_r_dispatch<true, false, true, true>(log_r, blocks, P, a, st);
-        else if (pair)
-            cols_r_dispatch<true, false, true>(log_r, blocks, P, a, st);
-        else if (lower)
-            cols_r_dispatch<true, false, false, true>(log_r, blocks, P, a, st);
-        else
-            cols_r_dispatch<true, false, false>(log_r, blocks, P, a, st);
+        const bool lower = a.Lx <= half && (!pair || a.Lx2 <= half);
+        if (a.rows) {
+            if (pair)
+                cols_r_dispatch<true, false, true, kRagged>(log_r, blocks, P, a, st);
+            else
+                cols_r_dispatch<true, false, false, kRagged>(log_r, blocks, P, a, st);
+        } else if (lower) {
+            if (pair)
+                cols_r_dispatch<true, false, true, kHalf>(log_r, blocks, P, a, st);
+            else
+                cols_r_dispatch<true, false, false, kHalf>(log_r, blocks, P, a, st);
+        } else {
+            if (pair)
+                cols_r_dispatch<true, false, true>(log_r, blocks, P, a, st);
+            else
+                cols_r_dispatch<true, false, false>(log_r, blocks, P, a, st);
+        }
     } else if (!inverse) {
         if (pair)
             cols_r_dispatch<false, false, true>(log_r, blocks, P, a, st);
@@ -1607,10 +1645,51 @@ static bool two_parts(Shape s, int *log_k1, int *log_k2) {
     return true;
 }
 
+// One operand of a transform: rows of X, or one side of a ragged batch.
+struct Operand {
+    const uint32_t *X;
+    uint64_t sX;
+    uint32_t Lx;       // limbs of the longest row
+    uint32_t *F;
+    uint32_t N;        // rows
+};
+
+// Forward column passes of one operand, or of two of the same shape (Y.F
+// non-null; in the same launches where the columns are long enough to pair).
+// Operands longer than K and cosets are folded into residues first.
+static void forward_columns(const NttParams &P, int log_k, int M, int coset0, const Operand &X, const Operand &Y,
+                            const RaggedRow *rows, int side, cudaStream_t st) {
+    const uint64_t K = 1ull << log_k;
+    int passes[2];
+    const int npass = column_passes(log_k, passes);
+    const bool pair = Y.F && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
+    const bool fold = M > 1 || coset0 || X.Lx > K || (Y.F && Y.Lx > K);
+    for (int op = 0; fold && op < (Y.F ? 2 : 1); ++op) {
+        const Operand &o = op ? Y : X;
+        FoldArgs a{o.X, o.sX, o.Lx, (uint32_t)((o.Lx + K - 1) >> log_k), o.F, log_k, M, coset0, rows, side + op};
+        const unsigned blocks = (unsigned)((uint64_t)o.N * kPrimes * (K / (kThreads * kFoldV)));
+        KernelTimed kt("ntt_fold", 4.0 * (double)o.Lx * o.N + 12.0 * (double)K * M * o.N);
+        if (a.nb <= (uint32_t)kFoldRegs)
+            k_fold<true><<<blocks, kThreads, 0, st>>>(P, a);
+        else
+            k_fold<false><<<blocks, kThreads, 0, st>>>(P, a);
+        count_launch();
+    }
+    for (int op = 0; op < (Y.F && !pair ? 2 : 1); ++op) {
+        const Operand &o = op ? Y : X;
+        int log_s = log_k;
+        for (int ps = 0; ps < npass; ++ps) {
+            ColsArgs a{o.X, o.sX, o.Lx, o.F, log_k, log_s, 0, Y.X, Y.sX, Y.Lx, pair ? Y.F : nullptr, rows, side + op};
+            launch_cols_r(ps == 0 && !fold, false, pair, passes[ps], P, a, (uint64_t)o.N * M, st);
+            log_s -= passes[ps];
+        }
+    }
+}
+
 // Inverse column passes of vrows virtual rows of F, innermost first (the
 // first one scales by K^-1 R); of F2 as well, in the same launches where the
 // columns are long enough to pair.
-static void inverse_columns(const NttParams &P, int log_k, int M, uint64_t vrows, uint32_t *F, uint32_t *F2,
+static void inverse_columns(const NttParams &P, int log_k, uint64_t vrows, uint32_t *F, uint32_t *F2,
                             cudaStream_t st) {
     int passes[2];
     const int npass = column_passes(log_k, passes);
@@ -1619,7 +1698,7 @@ static void inverse_columns(const NttParams &P, int log_k, int M, uint64_t vrows
         int log_s = kRowLog;
         for (int ps = npass - 1; ps >= 0; --ps) {
             log_s += passes[ps];
-            ColsArgs a{nullptr, 0, 0, 0, op ? F2 : F, log_k, log_s, M, 0, ps == npass - 1, nullptr, 0, 0, 0,
+            ColsArgs a{nullptr, 0, 0, op ? F2 : F, log_k, log_s, ps == npass - 1, nullptr, 0, 0,
                        pair ? F2 : nullptr, nullptr, 0};
             launch_cols_r(false, true, pair, passes[ps], P, a, vrows, st);
         }
@@ -1628,7 +1707,7 @@ static void inverse_columns(const NttParams &P, int log_k, int M, uint64_t vrows
 
 struct Operands {
     const uint32_t *A, *B;
-    uint32_t N, La, Lb;
+    uint32_t N, La, Lb;   // of a ragged batch: the longest operand on each side
     uint64_t sA, sB;
     bool square, bcast;   // B is A / one row of B serves every row
     const RaggedRow *rows;
@@ -1640,33 +1719,16 @@ static void cyclic_product(const NttParams &P, const Operands &o, int log_k, int
                            uint32_t *FB, cudaStream_t st) {
     const uint64_t K = 1ull << log_k;
     const uint64_t VR = (uint64_t)o.N * M;   // virtual rows (row, coset)
-    int passes[2];
-    const int npass = column_passes(log_k, passes);
-    // forward column passes: A and B together (one launch per pass) unless
-    // B is A or a broadcast row
-    const bool pair = !o.square && !o.bcast && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
-    for (int op = 0; op < (pair || o.square ? 1 : 2); ++op) {
-        const uint32_t *X = op == 0 ? o.A : o.B;
-        const uint64_t sX = op == 0 ? o.sA : o.sB;
-        const uint32_t Lx = op == 0 ? o.La : o.Lb;
-        uint32_t *F = op == 0 ? FA : FB;
-        const uint64_t vrows = (op == 1 && o.bcast) ? (uint64_t)M : VR;
-        const uint32_t nb = (uint32_t)((Lx + K - 1) / K);
-        const uint32_t nb2 = (uint32_t)((o.Lb + K - 1) / K);
-        int log_s = log_k;
-        for (int ps = 0; ps < npass; ++ps) {
-            ColsArgs a{X, sX, Lx, nb, F, log_k, log_s, M, coset0, 0, pair ? o.B : nullptr, o.sB, o.Lb, nb2,
-                       pair ? FB : nullptr, o.rows, op};
-            launch_cols_r(ps == 0, false, pair, passes[ps], P, a, vrows, st);
-            log_s -= passes[ps];
-        }
-    }
+    // forward column passes: A and B together unless B is A or a broadcast row
+    const Operand a{o.A, o.sA, o.La, FA, o.N}, b{o.B, o.sB, o.Lb, FB, o.bcast ? 1u : o.N}, none{};
+    forward_columns(P, log_k, M, coset0, a, o.square || o.bcast ? none : b, o.rows, 0, st);
+    if (o.bcast) forward_columns(P, log_k, M, coset0, b, none, nullptr, 1, st);
     RowsArgs r{o.A, o.sA, o.La, o.B, o.sB, o.Lb, FA, FB, log_k, M, o.bcast ? 1 : 0, o.square ? 1 : 0, nullptr};
     {
         KernelTimed kt("ntt_rows_fused", 12.0 * (double)K * ((o.square ? 2.0 : 3.0) * (double)VR));
         launch_rows(log_k, false, (uint32_t)(VR * (K >> kRowLog)), P, r, st);
     }
-    inverse_columns(P, log_k, M, VR, FA, nullptr, st);
+    inverse_columns(P, log_k, VR, FA, nullptr, st);
 }
 
 static void launch_combine2(const NttParams &P, uint32_t *F1, int log_k1, uint32_t *F2, int log_k2, uint32_t N,
@@ -1698,7 +1760,7 @@ static void launch_combine2(const NttParams &P, uint32_t *F1, int log_k1, uint32
 // workspace's too) and the strides are unused.
 static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t *ws,
                 uint32_t N, uint32_t La, uint32_t Lb, uint64_t sA, uint64_t sB, uint64_t sC,
-                const RaggedRow *rows = nullptr) {
+                const RaggedRow *rows = nullptr, uint32_t longest_a = 0u, uint32_t longest_b = 0u) {
     cudaStream_t st = current_stream();
     const uint32_t Lc = La + Lb;
     if (N == 0u || Lc == 0u) return;
@@ -1717,6 +1779,7 @@ static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32
     }
     const bool square = (!rows && A == B && La == Lb && sA == sB);
     const bool bcast = (!rows && !square && sB == 0u && N > 1u);
+    const uint32_t oa = rows ? longest_a : La, ob = rows ? longest_b : Lb;
     const uint64_t points = (uint64_t)N * s.M * 3 << s.log_k;
     const uint64_t tiles = ((uint64_t)Lc + kCrtSpan - 1) / kCrtSpan;
     uint32_t *FA = ws;
@@ -1738,12 +1801,12 @@ static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32
         c.M = 1;
         c.F2 = FA + p1;
         c.log_k2 = log_k2;
-        const Operands o{A, B, N, La, Lb, sA, sB, square, bcast, rows};
+        const Operands o{A, B, N, oa, ob, sA, sB, square, bcast, rows};
         cyclic_product(P, o, c.log_k, 1, 0, FA, FB, st);
         cyclic_product(P, o, log_k2, 1, 1, FA + p1, square ? FA + p1 : FB + p1, st);
         launch_combine2(P, FA, c.log_k, FA + p1, log_k2, N, st);
     } else {
-        cyclic_product(P, Operands{A, B, N, La, Lb, sA, sB, square, bcast, rows}, s.log_k, s.M, 0, FA, FB, st);
+        cyclic_product(P, Operands{A, B, N, oa, ob, sA, sB, square, bcast, rows}, s.log_k, s.M, 0, FA, FB, st);
         if (s.M > 1) {
             CombineArgs m{};
             m.F = FA;
@@ -1780,23 +1843,7 @@ static void spectrum_forward(const NttParams &P, Shape s, uint32_t N, const uint
     const int log_k = s.log_k, M = s.M;
     const uint64_t K = 1ull << log_k;
     const uint64_t VR = (uint64_t)N * M;
-    int passes[2];
-    const int npass = column_passes(log_k, passes);
-    const bool pair = Y && passes[0] >= kPairMinLogR && (npass == 1 || passes[1] >= kPairMinLogR);
-    for (int op = 0; op < ((pair || !Y) ? 1 : 2); ++op) {
-        const uint32_t *Z = op == 0 ? X : Y;
-        const uint64_t sZ = op == 0 ? sX : sY;
-        const uint32_t Lz = op == 0 ? Lx : Ly;
-        uint32_t *F = op == 0 ? FX : FY;
-        const uint32_t nb = (uint32_t)((Lz + K - 1) / K);
-        const uint32_t nb2 = (uint32_t)((Ly + K - 1) / K);
-        int log_s = log_k;
-        for (int ps = 0; ps < npass; ++ps) {
-            ColsArgs a{Z, sZ, Lz, nb, F, log_k, log_s, M, 0, 0, pair ? Y : nullptr, sY, Ly, nb2, pair ? FY : nullptr, nullptr, 0};
-            launch_cols_r(ps == 0, false, pair, passes[ps], P, a, VR, st);
-            log_s -= passes[ps];
-        }
-    }
+    forward_columns(P, log_k, M, 0, Operand{X, sX, Lx, FX, N}, Operand{Y, sY, Ly, FY, N}, nullptr, 0, st);
     if (!rows) return;
     rows_split_attr();
     RowsFwdArgs r{FX, Y ? FY : nullptr, log_k};
@@ -1833,7 +1880,7 @@ static void spectrum_inverse(const NttParams &P, Shape s, uint32_t N, int terms,
         count_launch();
     }
     }
-    if (cols) inverse_columns(P, log_k, M, VR, Fout, nullptr, st);
+    if (cols) inverse_columns(P, log_k, VR, Fout, nullptr, st);
     if (M > 1) {
         CombineArgs c{};
         c.F = Fout;
@@ -1939,11 +1986,13 @@ size_t batch_mul_ntt_workspace_size(uint32_t N, uint32_t L_a, uint32_t L_b) {
 namespace gpupi {
 
 // A ragged batch of products of at most Lc limbs in all at one transform
-// shape, the largest product's (Lc >= 2); workspace: batch_mul_ntt_workspace_size(N,
+// shape, the largest product's (Lc >= 2), operands of at most longest_a and
+// longest_b limbs; workspace: batch_mul_ntt_workspace_size(N,
 // Lc - 1, 1).
 void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint32_t *A, const uint32_t *B,
-                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc) {
-    ntt::mul(ntt::make_params(tables), A, B, C, ws, N, Lc - 1u, 1u, 0, 0, 0, rows);
+                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc, uint32_t longest_a,
+                    uint32_t longest_b) {
+    ntt::mul(ntt::make_params(tables), A, B, C, ws, N, Lc - 1u, 1u, 0, 0, 0, rows, longest_a, longest_b);
 }
 
 // Transform shape a product of La x Lb limbs gets (tune table or built-in rule).
@@ -1996,7 +2045,7 @@ void spectrum_inverse(const NTTPrecomputedTables &tables, SpectrumShape s, uint3
 
 void spectrum_inverse_columns(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *F0,
                               uint32_t *F1) {
-    ntt::inverse_columns(ntt::make_params(tables), s.log_k, s.M, (uint64_t)N * s.M, F0, F1, current_stream());
+    ntt::inverse_columns(ntt::make_params(tables), s.log_k, (uint64_t)N * s.M, F0, F1, current_stream());
 }
 
 void spectrum_level_rows(const NTTPrecomputedTables &tables, SpectrumShape s, uint32_t N, uint32_t *Fpe,

@@ -33,7 +33,8 @@ cudaError_t tc_mul_ragged(const uint32_t *A, const uint32_t *B, uint32_t *C, uin
 void tc_shape(uint32_t La, uint32_t Lb, uint32_t *Q, uint32_t *N);
 void mul_kinds(uint32_t n, const uint32_t *La, const uint32_t *Lb, uint8_t *kinds);
 void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint32_t *A, const uint32_t *B,
-                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc);
+                    uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc, uint32_t longest_a,
+                    uint32_t longest_b);
 const NTTPrecomputedTables &context_tables(const BatchMPContext *ctx);
 const void *context_workspace(const BatchMPContext *ctx);
 
@@ -138,11 +139,16 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
     for (uint32_t g = kNttGroup; err == cudaSuccess && g < kGroups; ++g) {
         const uint32_t n = start[g + 1u] - start[g];
         if (!n) continue;
-        uint32_t most = 0;
-        for (uint32_t i = start[g]; i < start[g + 1u]; ++i) most = std::max(most, rows[i].La + rows[i].Lb);
+        uint32_t most = 0, la = 0, lb = 0;
+        for (uint32_t i = start[g]; i < start[g + 1u]; ++i) {
+            most = std::max(most, rows[i].La + rows[i].Lb);
+            la = std::max(la, rows[i].La);
+            lb = std::max(lb, rows[i].Lb);
+        }
         err = batch_mp_ensure_workspace(ctx, batch_mul_ntt_workspace_size(n, most - 1u, 1u));
         if (err == cudaSuccess)
-            ntt_mul_ragged(context_tables(ctx), (uint32_t *)context_workspace(ctx), A, B, C, n, dr + start[g], most);
+            ntt_mul_ragged(context_tables(ctx), (uint32_t *)context_workspace(ctx), A, B, C, n, dr + start[g], most,
+                           la, lb);
     }
     if (err == cudaSuccess) err = cudaGetLastError();
     scratch_free(dr);
