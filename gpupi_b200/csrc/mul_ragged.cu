@@ -8,9 +8,11 @@
 //   * L_a = 0 or L_b = 0: the L_a + L_b output limbs are zeroed;
 //   * products the tune table gives to the CUDA-core schoolbook: one
 //     k_school_cols launch; those it gives to the tensor-core schoolbook:
-//     up to four k_mul_tc launches by length, longest products first (a
-//     launch's shared memory is sized for its largest product, so short ones
-//     in a launch of their own get several CTAs per SM);
+//     up to four k_mul_tc launches by the shared memory their products need,
+//     the largest first (a launch's is sized for its largest product, so the
+//     others get several CTAs per SM in launches of their own; the shorter
+//     operand decides it: by length alone, products of a long and a short
+//     operand ran one per SM beside the balanced ones);
 //   * otherwise by transform size (powers of two up to 2^13 points, quarters of
 //     an octave above): one NTT batch per bucket at its largest product's shape.
 // 4096 products of 8..4096 limbs per operand: gathering the NTT products into
@@ -31,6 +33,7 @@ void school_mul_ragged(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32
 cudaError_t tc_mul_ragged(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t n, const RaggedRow *rows,
                           uint32_t maxQ, uint32_t maxN, uint64_t limbs_moved);
 void tc_shape(uint32_t La, uint32_t Lb, uint32_t *Q, uint32_t *N);
+uint32_t tc_smem_bytes(uint32_t La, uint32_t Lb);
 void mul_kinds(uint32_t n, const uint32_t *La, const uint32_t *Lb, uint8_t *kinds);
 void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint32_t *A, const uint32_t *B,
                     uint32_t *C, uint32_t N, const RaggedRow *rows, uint32_t Lc, uint32_t longest_a,
@@ -51,11 +54,12 @@ __global__ void __launch_bounds__(256) k_zero_rows(uint32_t *__restrict__ C, con
 
 unsigned grid_rows(uint32_t n) { return (unsigned)std::max<uint32_t>(1u, std::min<uint32_t>(n, kNumSMs * 16)); }
 
-// Group numbers: zero products, schoolbook, tensor-core length steps from the
-// longest (32 limbs each), NTT buckets.
+// Group numbers: zero products, schoolbook, tensor-core products by KiB of
+// shared memory from the largest, NTT buckets.
 constexpr uint32_t kZero = 0u, kSchoolGroup = 1u, kTensorGroup = 2u;
-constexpr uint32_t kTensorStep = 32u;
-constexpr uint32_t kTensorGroups = 8192u / kTensorStep + 1u;
+constexpr uint32_t kTensorGroups = 256u;
+// limits of the launches: one, two, four CTAs in an SM's 228 KiB, more
+constexpr uint32_t kTensorLimits[] = {112u, 56u, 28u, 0u};
 constexpr uint32_t kNttGroup = kTensorGroup + kTensorGroups;
 constexpr uint32_t kNttGroups = 4u * 32u;
 constexpr uint32_t kGroups = kNttGroup + kNttGroups;
@@ -91,7 +95,7 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         else if (kind[i] == 0u)
             g = kSchoolGroup;
         else if (kind[i] == 1u)
-            g = kTensorGroup + (kTensorGroups - 1u - (uint32_t)Lc / kTensorStep);
+            g = kTensorGroup + (kTensorGroups - 1u - std::min(kTensorGroups - 1u, tc_smem_bytes(La[i], Lb[i]) >> 10));
         else
             g = kNttGroup + ntt_bucket(Lc - 1u);
         group[i] = (uint16_t)g;
@@ -103,12 +107,19 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         std::vector<uint32_t> at(start.begin(), start.end() - 1);
         for (uint32_t i = 0; i < N; ++i) rows[at[group[i]]++] = RaggedRow{offA[i], offB[i], offC[i], La[i], Lb[i]};
     }
-    RaggedRow *dr = nullptr;
-    cudaError_t err = scratch_alloc((void **)&dr, (size_t)N * sizeof(RaggedRow));
-    if (err == cudaSuccess) {
-        err = cudaMemcpyAsync(dr, rows.data(), (size_t)N * sizeof(RaggedRow), cudaMemcpyHostToDevice, st);
-        note_h2d((size_t)N * sizeof(RaggedRow));
-    }
+    // descriptors on the device: those of the schoolbooks, and those of the NTT
+    // batches, copied while the former's kernels run
+    auto upload = [&](uint32_t from, uint32_t to, RaggedRow **d) {
+        const size_t bytes = (size_t)(to - from) * sizeof(RaggedRow);
+        if (!bytes) return cudaSuccess;
+        cudaError_t e = scratch_alloc((void **)d, bytes);
+        if (e != cudaSuccess) return e;
+        note_h2d(bytes);
+        return cudaMemcpyAsync(*d, rows.data() + from, bytes, cudaMemcpyHostToDevice, st);
+    };
+    const uint32_t ntt0 = start[kNttGroup];   // the first NTT product
+    RaggedRow *dr = nullptr, *dn = nullptr;
+    cudaError_t err = upload(0u, ntt0, &dr);
     const uint32_t nz = start[1], ns = start[2] - start[1];
     if (err == cudaSuccess && nz) {
         k_zero_rows<<<grid_rows(nz), 256, 0, st>>>(C, dr, nz);
@@ -119,23 +130,24 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         for (uint32_t i = start[1]; i < start[2]; ++i) work += (uint64_t)rows[i].La * rows[i].Lb;
         school_mul_ragged(A, B, C, ns, dr + start[1], work);
     }
-    // tensor-core launches: products above 2048, 1024 and 512 limbs, the rest
-    for (uint32_t first = start[kTensorGroup], end = start[kNttGroup]; err == cudaSuccess && first < end;) {
-        const uint32_t longest = rows[first].La + rows[first].Lb;
-        const uint32_t least = longest >= 2048u ? 2048u : longest >= 1024u ? 1024u : longest >= 512u ? 512u : 0u;
-        uint32_t last = first, maxQ = 0, maxN = 0;
+    uint32_t first = start[kTensorGroup];
+    for (const uint32_t limit : kTensorLimits) {
+        // products of at least `limit` KiB: groups up to kTensorGroups - 1 - limit
+        const uint32_t last = start[kTensorGroup + kTensorGroups - limit];
+        if (err != cudaSuccess || last == first) continue;
+        uint32_t maxQ = 0, maxN = 0;
         uint64_t limbs = 0;
-        // 32-limb groups: a group never spans one of the limits
-        for (; last < end && rows[last].La + rows[last].Lb >= least; ++last) {
+        for (uint32_t i = first; i < last; ++i) {
             uint32_t q = 0, n = 0;
-            tc_shape(rows[last].La, rows[last].Lb, &q, &n);
+            tc_shape(rows[i].La, rows[i].Lb, &q, &n);
             maxQ = std::max(maxQ, q);
             maxN = std::max(maxN, n);
-            limbs += 2ull * (rows[last].La + rows[last].Lb);
+            limbs += 2ull * (rows[i].La + rows[i].Lb);
         }
         err = tc_mul_ragged(A, B, C, last - first, dr + first, maxQ, maxN, limbs);
         first = last;
     }
+    if (err == cudaSuccess) err = upload(ntt0, N, &dn);
     for (uint32_t g = kNttGroup; err == cudaSuccess && g < kGroups; ++g) {
         const uint32_t n = start[g + 1u] - start[g];
         if (!n) continue;
@@ -147,11 +159,12 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         }
         err = batch_mp_ensure_workspace(ctx, batch_mul_ntt_workspace_size(n, most - 1u, 1u));
         if (err == cudaSuccess)
-            ntt_mul_ragged(context_tables(ctx), (uint32_t *)context_workspace(ctx), A, B, C, n, dr + start[g], most,
+            ntt_mul_ragged(context_tables(ctx), (uint32_t *)context_workspace(ctx), A, B, C, n, dn + (start[g] - ntt0), most,
                            la, lb);
     }
     if (err == cudaSuccess) err = cudaGetLastError();
-    scratch_free(dr);
+    if (dr) scratch_free(dr);
+    if (dn) scratch_free(dn);
     return err;
 }
 

@@ -455,6 +455,12 @@ void tc_shape(uint32_t La, uint32_t Lb, uint32_t *Q, uint32_t *N) {
     *N = sh.N;
 }
 
+// Shared memory one product needs: what limits its CTAs per SM.
+uint32_t tc_smem_bytes(uint32_t La, uint32_t Lb) {
+    const tc::Shape sh = tc::shape_of(std::min(La, Lb), std::max(La, Lb));
+    return tc::layout_of(sh.Q, sh.N).total;
+}
+
 uint32_t tc_error();
 
 // Timeout self-test: one 64 x 64-limb product whose CTA first waits on a
