@@ -68,14 +68,15 @@ NCU_TRAFFIC_SOURCE = {"ntt_rows_fused": "ncu capture of k_rows_r<12> on a 2^22 x
 # (profiles/int_pipes_pi1e8.md).  Scaled to this run's bytes and divided by
 # the live integer-pipe peaks they give each family's integer roofline.
 INT_WINST_PER_BYTE = {
-    "ntt_rows_level": (0.20437, 0.205252, 0.487605), "ntt_cols_fwd_first": (0.187598, 0.211507, 0.477682),
-    "ntt_cols_inv": (0.100109, 0.11195, 0.246731), "schoolbook_tc": (0.143044, 0.265617, 0.763927),
-    "ntt_crt_carry": (0.075663, 0.095934, 0.230741), "ntt_rows_fused": (0.223057, 0.220512, 0.527792),
-    "schoolbook": (0.212093, 0.176371, 0.49994), "ntt_cols_fwd": (0.080255, 0.096138, 0.204625),
-    "carry_chain": (0.077046, 0.098004, 0.245578), "ntt_local": (0.55531, 0.538007, 1.292256),
-    "ntt_rows_inv": (0.078142, 0.077174, 0.193306), "ntt_rows_fwd": (0.10064, 0.094374, 0.250671),
-    "ntt_coset_combine": (0.103479, 0.100658, 0.265951), "decimal_extract": (0.075693, 0.08626, 0.224201),
-    "decimal_leaf": (0.596097, 0.168555, 0.837855), "shift": (0.035647, 0.045182, 0.115069)}
+    "ntt_rows_level": (0.183426, 0.182728, 0.440234), "ntt_cols_fwd_first": (0.118559, 0.11696, 0.289975),
+    "ntt_cols_inv": (0.073674, 0.074348, 0.182748), "schoolbook_tc": (0.175881, 0.347193, 0.872551),
+    "ntt_crt_carry": (0.050113, 0.045814, 0.125112), "ntt_rows_fused": (0.180556, 0.177752, 0.424416),
+    "ntt_cols_fwd": (0.069824, 0.069802, 0.175721), "schoolbook": (0.219156, 0.17921, 0.53567),
+    "ntt_local": (0.439652, 0.430948, 1.015859), "carry_chain": (0.032343, 0.099566, 0.174273),
+    "ntt_rows_fwd": (0.097792, 0.091607, 0.244568), "ntt_rows_inv": (0.064503, 0.064857, 0.163097),
+    "ntt_fold": (0.113415, 0.126271, 0.417258), "decimal_extract": (0.075693, 0.08626, 0.224201),
+    "ntt_coset_combine": (0.090216, 0.077055, 0.224702), "shift": (0.035647, 0.045182, 0.115069),
+    "decimal_leaf": (0.704212, 0.245135, 1.12563)}
 INT_SOURCE = ("ncu sm__inst_executed_pipe_{fmaheavy,alu}.sum and sm__inst_executed.sum over every launch of "
               "pi_bs_gpu 100000000 (profiles/int_pipes_pi1e8.md), per algorithmic byte, scaled to this run")
 sys.path.insert(0, str(ROOT))
