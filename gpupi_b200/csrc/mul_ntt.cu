@@ -643,7 +643,7 @@ static_assert(RowLast::kLO == 0 && RowLast::kB == 4, "last row stage holds 16 co
 // product / R, inverse stages; the first inverse column pass multiplies by
 // K^-1 R with its twist.  The loads between the transforms come from L2, where
 // the group's next segment is sent while it transforms the one before.
-// One 2^28-point product (196,608 segments): 6.88 -> 5.45 ms.
+// One 2^28-point product (196,608 segments): 6.88 -> 5.13 ms.
 template <int Q>
 __device__ __forceinline__ void rows_run(const RowsArgs &a, uint32_t first, uint32_t last, const RowShared &s) {
     const uint32_t t = threadIdx.x & 255u;
