@@ -53,20 +53,33 @@ __device__ __forceinline__ BlockCarry block_resolve(bool g, bool p, uint32_t *sh
     return r;
 }
 
-// Limbs [start, end) of tile t of a row at `out`: tiles are `span` limbs, or,
-// with `aligned`, span limbs counted from the row's last 16-byte boundary at
-// or below its first limb (carry_ops.cu), so tile 0 is up to three limbs short.
+// Row `row` of a batch of results: C + row * sC with Lc limbs, or in a ragged
+// batch (rows non-null) its descriptor's place and its own La + Lb limbs.
+struct ResultRow {
+    uint32_t *p;
+    uint32_t L;
+};
+__device__ __forceinline__ ResultRow result_row(const RaggedRow *rows, uint32_t *C, uint64_t sC, uint32_t Lc,
+                                                uint32_t row) {
+    if (!rows) return {C + row * sC, Lc};
+    return {C + rows[row].offC, rows[row].La + rows[row].Lb};
+}
+
+// Limbs [start, end) of tile t of a row of L limbs at `out`: tiles are `span`
+// limbs, or, with `aligned`, span limbs counted from the row's last 16-byte
+// boundary at or below its first limb (carry_ops.cu), so tile 0 is up to three
+// limbs short.
 struct TileRange {
     uint64_t start, end;
 };
-__device__ __forceinline__ TileRange tile_range(const uint32_t *out, uint32_t t, uint32_t span, uint32_t Lc,
+__device__ __forceinline__ TileRange tile_range(const uint32_t *out, uint32_t t, uint32_t span, uint32_t L,
                                                 bool aligned) {
     const uint64_t mis = aligned ? (((uintptr_t)out >> 2) & 3u) : 0u;
     TileRange r;
     r.start = (uint64_t)t * span;
     r.start = r.start > mis ? r.start - mis : 0u;
     r.end = (uint64_t)(t + 1u) * span - mis;
-    if (r.end > Lc) r.end = Lc;
+    if (r.end > L) r.end = L;
     return r;
 }
 
@@ -109,8 +122,9 @@ __device__ __forceinline__ void patch_rest(uint32_t *out, TileRange r, bool all)
     }
 }
 
-// rows non-null: a ragged batch, each row's place from its descriptor (tiles
-// above a shorter row's end hold zeros and receive no carry).
+// rows non-null: a ragged batch; Lc and tiles_per_row are its longest row's.  A
+// shorter row's tiles end with the row (what follows is another product's, or
+// not the caller's); those wholly above it receive no carry.
 // Cross-tile carry fix-up for rows of at most 32 tiles: one warp per row, one
 // lane per tile.
 template <bool SUB>
@@ -120,17 +134,17 @@ __global__ void carry_fixup_kernel(uint32_t *C, uint64_t sC, uint32_t N, uint32_
     const uint32_t gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t row = gwarp; row < N; row += nwarps) {
-        uint32_t *out = C + (rows ? rows[row].offC : row * sC);
+        const ResultRow out = result_row(rows, C, sC, Lc, row);
         const uint32_t f = (lane < tiles_per_row) ? flags[(uint64_t)row * tiles_per_row + lane] : 0u;
         const uint32_t gm = __ballot_sync(0xffffffffu, (f & 1u) != 0u);
         const uint32_t pm = __ballot_sync(0xffffffffu, (f & 2u) != 0u);
         const GroupCarry gc = resolve_group(gm, pm, 0u);
         bool more = false;
         if (lane < tiles_per_row && ((gc.carry_in_mask >> lane) & 1u))
-            more = patch_first<SUB>(out, tile_range(out, lane, span, Lc, aligned));
+            more = patch_first<SUB>(out.p, tile_range(out.p, lane, span, out.L, aligned));
         for (uint32_t left = __ballot_sync(0xffffffffu, more); left; left &= left - 1u) {
             const uint32_t t = (uint32_t)(__ffs(left) - 1);
-            patch_rest<SUB>(out, tile_range(out, t, span, Lc, aligned), (pm >> t) & 1u);
+            patch_rest<SUB>(out.p, tile_range(out.p, t, span, out.L, aligned), (pm >> t) & 1u);
         }
     }
 }
@@ -157,7 +171,7 @@ __global__ void __launch_bounds__(kFixThreads) carry_fixup_rows_kernel(uint32_t 
     const uint32_t row = blockIdx.x / blocks_per_row;
     const uint32_t blk = blockIdx.x - row * blocks_per_row;
     const uint32_t *fr = flags + (uint64_t)row * tiles_per_row;
-    uint32_t *out = C + (rows ? rows[row].offC : row * sC);
+    const ResultRow out = result_row(rows, C, sC, Lc, row);
     // generate / propagate bits of this thread's four tiles of group b
     auto load = [&](uint32_t b, uint32_t &g, uint32_t &p) {
         g = p = 0u;
@@ -192,12 +206,12 @@ __global__ void __launch_bounds__(kFixThreads) carry_fixup_rows_kernel(uint32_t 
         const uint32_t t = t0 + k;
         bool more = false;
         if (t < tiles_per_row && ((into >> k) & 1u))
-            more = patch_first<SUB>(out, tile_range(out, t, span, Lc, aligned));
+            more = patch_first<SUB>(out.p, tile_range(out.p, t, span, out.L, aligned));
         for (uint32_t left = __ballot_sync(0xffffffffu, more); left; left &= left - 1u) {
             const int l = __ffs(left) - 1;
             const uint32_t tl = __shfl_sync(0xffffffffu, t, l);
             const uint32_t pl = __shfl_sync(0xffffffffu, (p >> k) & 1u, l);
-            patch_rest<SUB>(out, tile_range(out, tl, span, Lc, aligned), pl != 0u);
+            patch_rest<SUB>(out.p, tile_range(out.p, tl, span, out.L, aligned), pl != 0u);
         }
     }
 }

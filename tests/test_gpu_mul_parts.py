@@ -117,3 +117,32 @@ def test_ragged_in_place(ctx, table):
     finally:
         g.tune_load(g.TUNE_TABLE_PATH)
     assert np.array_equal(dC.numpy(), want)
+
+
+@pytest.mark.parametrize("last", [1366, 1370, 2041])
+def test_ragged_carry_to_a_short_rows_end(ctx, last):
+    """(2^(32m) + 1)(2^(64m) - 2^(32m) + 1) = 2^(96m) + 1, 3m + 1 limbs: its
+    coefficient sums leave all-ones limbs that a carry runs through to the
+    row's last limbs, in a bucket whose longest product is longer; the
+    product with m = `last` ends the output."""
+    rng = np.random.default_rng(last)
+    ms = [1366, 1367, 1400, 2100, last]
+    A, B = [], []
+    for m in ms:
+        a, b = np.zeros(m + 1, dtype=np.uint32), np.zeros(2 * m, dtype=np.uint32)
+        a[0] = a[m] = b[0] = 1
+        b[m:] = 0xFFFFFFFF
+        A.append(a)
+        B.append(b)
+    A.insert(1, rand_buf(rng, 1, 4001, 4001))
+    B.insert(1, rand_buf(rng, 1, 4100, 4100))
+    La, Lb = (np.array([len(x) for x in v], dtype=np.uint32) for v in (A, B))
+    oa, ob, oc = (np.concatenate([[0], np.cumsum(x)[:-1]]).astype(np.uint64) for x in (La, Lb, La + Lb))
+    want = []
+    for a, b in zip(A, B):
+        x, y = (int.from_bytes(v.tobytes(), "little") for v in (a, b))
+        want.append(np.frombuffer((x * y).to_bytes(4 * (len(a) + len(b)), "little"), dtype=np.uint32))
+    want = np.concatenate(want)
+    dA, dB, dC = to_dev(np.concatenate(A)), to_dev(np.concatenate(B)), to_dev(np.zeros_like(want))
+    ctx.mul_ragged(dA.ptr, oa, La, dB.ptr, ob, Lb, dC.ptr, oc)
+    assert np.array_equal(dC.numpy(), want)
