@@ -158,12 +158,12 @@ __device__ __forceinline__ void chunk_raw(const uint32_t (&x)[4], const uint32_t
     if (SUB)
         asm("sub.cc.u32 %0, %5, %9;\n\tsubc.cc.u32 %1, %6, %10;\n\tsubc.cc.u32 %2, %7, %11;\n\t"
             "subc.cc.u32 %3, %8, %12;\n\tsubc.u32 %4, 0, 0;"
-            : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(c)
+            : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "=r"(c)
             : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
     else
         asm("add.cc.u32 %0, %5, %9;\n\taddc.cc.u32 %1, %6, %10;\n\taddc.cc.u32 %2, %7, %11;\n\t"
             "addc.cc.u32 %3, %8, %12;\n\taddc.u32 %4, 0, 0;"
-            : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(c)
+            : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "=r"(c)
             : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]));
     g = c != 0u;
     p = SUB ? (s[0] | s[1] | s[2] | s[3]) == 0u : (s[0] & s[1] & s[2] & s[3]) == 0xffffffffu;

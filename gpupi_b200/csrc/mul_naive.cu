@@ -285,7 +285,7 @@ __device__ __forceinline__ void mac3(uint32_t &c0, uint32_t &c1, uint32_t &c2, u
     asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
         "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
         "addc.u32 %2, %2, 0;"
-        : "+r"(c0), "+r"(c1), "+r"(c2)
+        : "+&r"(c0), "+&r"(c1), "+r"(c2)
         : "r"(a), "r"(b));
 }
 
