@@ -1374,18 +1374,19 @@ struct Shape {
 // Smallest shape with M * K >= L_a + L_b - 1: one power-of-two transform up to
 // 2^25 points, above that M cosets of 2^25 points.
 }  // namespace ntt
-bool ntt_shape_override(uint64_t need, int *log_k, int *M);   // tune.cu
+bool ntt_shape_override(uint64_t need, uint32_t N, int *log_k, int *M);   // tune.cu
+uint32_t ntt_small_batch(uint64_t need);                                  // tune.cu
 namespace ntt {
 
 static Shape shape_for(uint32_t La, uint32_t Lb);
 
-// The product's transform shape: the tune table's, else the built-in rule
-// (shape_for).  Used by the plain product and its workspace size; the
-// tuned splitting tree's spectra keep the built-in rule.
-static Shape shape_tuned(uint32_t La, uint32_t Lb) {
+// The transform shape of a batch of N products: the tune table's, else the
+// built-in rule (shape_for).  Used by the plain product and its workspace size;
+// the tuned splitting tree's spectra keep the built-in rule.
+static Shape shape_tuned(uint32_t N, uint32_t La, uint32_t Lb) {
     int lk = 0, M = 0;
     const uint64_t need = (uint64_t)La + Lb - 1u;
-    if (ntt_shape_override(need, &lk, &M)) return Shape{lk, M};
+    if (ntt_shape_override(need, N, &lk, &M)) return Shape{lk, M};
     // just above one transform: 2^25 points and a second part instead of two
     // cosets of 2^25
     if (need > (1ull << kMaxLog) && need <= (5ull << (kMaxLog - 2))) return Shape{kMaxLog - 2, 5};
@@ -1627,11 +1628,14 @@ static void launch_combine(int M, const NttParams &P, const CombineArgs &c, uint
 
 size_t workspace_bytes(uint32_t N, uint32_t La, uint32_t Lb) {
     if (N == 0u || La == 0u || Lb == 0u) return 0;
-    const Shape s = shape_tuned(La, Lb);
-    const uint64_t K = 1ull << s.log_k;
+    const Shape s = shape_tuned(N, La, Lb);
     const uint64_t Lc = (uint64_t)La + Lb;
     const uint64_t tiles = (Lc + kCrtSpan - 1) / kCrtSpan;
-    return (size_t)(2ull * N * s.M * 3 * K * 4 + N * tiles * 4 + 256);
+    // a smaller batch may take a shape of more points: this size holds it too
+    const Shape f = shape_for(La, Lb);
+    const uint64_t few = std::min<uint64_t>(N, ntt_small_batch(Lc - 1u) - 1u);
+    const uint64_t points = std::max(((uint64_t)N * s.M) << s.log_k, (few * f.M) << f.log_k);
+    return (size_t)(2ull * points * 3 * 4 + N * tiles * 4 + 256);
 }
 
 // The two-part split of a shape of M K points (M with two bits set, the larger
@@ -1768,7 +1772,7 @@ static void mul(const NttParams &P, const uint32_t *A, const uint32_t *B, uint32
         cudaMemset2DAsync(C, sC * 4, 0, (size_t)Lc * 4, N, st);
         return;
     }
-    const Shape s = shape_tuned(La, Lb);
+    const Shape s = shape_tuned(N, La, Lb);
     if (s.M > kMaxCosets) {
         fprintf(stderr, "gpupi_b200: product of %u limbs exceeds the 20 * 2^25-point limit\n", Lc);
         return;
@@ -1995,9 +1999,10 @@ void ntt_mul_ragged(const NTTPrecomputedTables &tables, uint32_t *ws, const uint
     ntt::mul(ntt::make_params(tables), A, B, C, ws, N, Lc - 1u, 1u, 0, 0, 0, rows, longest_a, longest_b);
 }
 
-// Transform shape a product of La x Lb limbs gets (tune table or built-in rule).
+// Transform shape products of La x Lb limbs get (tune table or built-in rule) in
+// a large batch.
 void ntt_shape_of(uint32_t La, uint32_t Lb, int *log_k, int *M) {
-    const ntt::Shape s = ntt::shape_tuned(La, Lb);
+    const ntt::Shape s = ntt::shape_tuned(UINT32_MAX, La, Lb);
     *log_k = s.log_k;
     *M = s.M;
 }

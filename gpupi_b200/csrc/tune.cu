@@ -18,7 +18,13 @@
 // File format (text, one entry per line, '#' starts a comment):
 //   mul <max_sum> school|tc|ntt        products with L_a + L_b <= max_sum
 //                                      (and above the previous entry)
-//   ntt <min_need> <max_need> <log_k> <M>   transforms for min_need <= need <= max_need
+//   ntt <min_need> <max_need> <log_k> <M> [<rows>]   transforms for min_need <= need <= max_need
+//                                      in batches of at least rows (1) products;
+//                                      smaller ones use the next power of two
+// A shape of several parts transforms fewer points in about twice as many
+// dependent launches, so it pays from some batch on: one product of 10,000 x
+// 9,000 limbs takes 75 us in two parts (13 launches) and 35 us in one
+// transform (6 launches), 205 products of 20,000 x 20,000 limbs 435 and 512 us.
 // The table is read at context creation from $GPUPI_TUNE_TABLE, else from
 // tune_table.txt beside libgpupi_b200.so; gpupi_autotune() measures the
 // candidates on the current GPU (CUDA events, best of several runs, each
@@ -59,6 +65,7 @@ struct MulEntry {
 struct NttEntry {
     uint64_t min_need, max_need;
     int log_k, M;
+    uint32_t rows;   // smallest batch that uses it
 };
 struct Table {
     std::mutex mu;
@@ -105,7 +112,7 @@ int parse_table(const std::string &text, const std::string &source) {
         const size_t hash = l.find('#');
         if (hash != std::string::npos) l.resize(hash);
         char word[16] = {0}, kind[16] = {0};
-        unsigned long long a = 0, a2 = 0;
+        unsigned long long a = 0, a2 = 0, rows = 1;
         int b = 0, c = 0;
         if (sscanf(l.c_str(), " %15s", word) != 1) continue;   // blank
         if (!strcmp(word, "mul")) {
@@ -114,9 +121,10 @@ int parse_table(const std::string &text, const std::string &source) {
                 return -line;
             mul.push_back(MulEntry{(uint32_t)a, parse_kind(kind)});
         } else if (!strcmp(word, "ntt")) {
-            if (sscanf(l.c_str(), " ntt %llu %llu %d %d", &a, &a2, &b, &c) != 4 || a > a2 || !shape_ok(a2, b, c))
+            if (sscanf(l.c_str(), " ntt %llu %llu %d %d %llu", &a, &a2, &b, &c, &rows) < 4 || a > a2 ||
+                !shape_ok(a2, b, c) || rows == 0 || rows > 0xffffffffull)
                 return -line;
-            ntt.push_back(NttEntry{a, a2, b, c});
+            ntt.push_back(NttEntry{a, a2, b, c, (uint32_t)rows});
         } else {
             return -line;
         }
@@ -196,9 +204,9 @@ void mul_kinds(uint32_t n, const uint32_t *La, const uint32_t *Lb, uint8_t *kind
     for (uint32_t i = 0; i < n; ++i) kinds[i] = (uint8_t)mul_kind_locked(t, La[i], Lb[i], false);
 }
 
-// NTT shape for `need` points from the table (or the tuner's forced
-// shape); false: use the built-in rule.
-bool ntt_shape_override(uint64_t need, int *log_k, int *M) {
+// NTT shape for N products of `need` points from the table (or the tuner's
+// forced shape); false: use the built-in rule.
+bool ntt_shape_override(uint64_t need, uint32_t N, int *log_k, int *M) {
     Table &t = table();
     std::lock_guard<std::mutex> g(t.mu);
     if (t.force_log_k > 0 && shape_ok(need, t.force_log_k, t.force_M)) {
@@ -209,12 +217,29 @@ bool ntt_shape_override(uint64_t need, int *log_k, int *M) {
     if (!t.loaded) return false;
     for (const NttEntry &e : t.ntt)
         if (need >= e.min_need && need <= e.max_need) {
-            if (!shape_ok(need, e.log_k, e.M)) return false;
+            if (!shape_ok(need, e.log_k, e.M) || N < e.rows) return false;
             *log_k = e.log_k;
             *M = e.M;
             return true;
         }
     return false;
+}
+
+// Batches of fewer than this many products may use the built-in rule where
+// the table gives larger ones another shape: the largest `rows` of the needs up
+// to the same power of two.
+uint32_t ntt_small_batch(uint64_t need) {
+    auto octave = [](uint64_t n) {
+        int k = 0;
+        while ((1ull << k) < n) ++k;
+        return k;
+    };
+    Table &t = table();
+    std::lock_guard<std::mutex> g(t.mu);
+    uint32_t rows = 1u;
+    for (const NttEntry &e : t.ntt)
+        if (octave(e.min_need) <= octave(need) && octave(e.max_need) >= octave(need)) rows = std::max(rows, e.rows);
+    return rows;
 }
 
 void tune_load_default() {
@@ -257,9 +282,10 @@ std::string tune_describe() {
         s += line;
     }
     for (const NttEntry &e : t.ntt) {
-        snprintf(line, sizeof line, "ntt %llu %llu %d %d\n", (unsigned long long)e.min_need,
+        snprintf(line, sizeof line, "ntt %llu %llu %d %d", (unsigned long long)e.min_need,
                  (unsigned long long)e.max_need, e.log_k, e.M);
         s += line;
+        s += e.rows > 1u ? " " + std::to_string(e.rows) + "\n" : "\n";
     }
     return s;
 }
@@ -284,6 +310,9 @@ __global__ void k_count_diff(const uint32_t *a, const uint32_t *b, uint64_t n, u
         c += (a[i] != b[i]);
     if (c) atomicAdd(out, c);
 }
+
+constexpr int kReps = 5;
+constexpr float kClear = 0.98f;
 
 struct Bench {
     BatchMPContext *ctx;
@@ -336,6 +365,20 @@ bool same_result(Bench &b, uint64_t words) {
 
 }  // namespace
 
+// Measures `need` points in the shape given: N products of La x Lb limbs.
+static float run_shape(Bench &b, int log_k, int M, uint32_t N, uint32_t La, uint32_t Lb) {
+    auto force = [](int lk, int m) {
+        Table &t = table();
+        std::lock_guard<std::mutex> g(t.mu);
+        t.force_log_k = lk;
+        t.force_M = m;
+    };
+    force(log_k, M);
+    const float ms = run_kind(b, kNtt, N, La, Lb, kReps);
+    force(0, 0);
+    return ms;
+}
+
 // Measures every candidate and writes the table to `path` (then loads it).
 // budget_limbs: total limbs of the operands of one measured batch.
 cudaError_t autotune(BatchMPContext *ctx, const char *path, uint64_t budget_limbs, std::string *report) {
@@ -375,29 +418,30 @@ cudaError_t autotune(BatchMPContext *ctx, const char *path, uint64_t budget_limb
         out += " (" + std::to_string(prop.multiProcessorCount) + " SMs)\n";
     }
     out += "# balanced products (L_a = L_b), batches of about " + std::to_string(budget_limbs) +
-           " operand limbs; times in ms (best of 3)\n";
+           " operand limbs; times in ms (best of 5)\n"
+           "# last number of an ntt line: the smallest batch it is for (1 if missing)\n";
     std::string log;
     char line[256];
     // 1. product kernel per length bucket (L_a + L_b up to 8192)
     static const uint32_t sums[] = {40,   48,   64,   96,   128,  192,  256,  320,  384,  448,  512,  640,
-                                    768,  896,  1024, 1536, 2048, 3072, 4096, 6144, 8192};
+                                    768,  896,  1024, 1536, 2048, 2560, 3072, 4096, 6144, 8192};
     for (uint32_t L : sums) {
         const uint32_t La = L / 2, Lb = L - La;
         const uint32_t N = (uint32_t)std::max<uint64_t>(1, budget_limbs / L);
         float t[3] = {-1.f, -1.f, -1.f};
         // reference result: the NTT
-        t[kNtt] = run_kind(b, kNtt, N, La, Lb, 3);
+        t[kNtt] = run_kind(b, kNtt, N, La, Lb, kReps);
         if (t[kNtt] < 0.f) {
             release();
             return cudaErrorUnknown;
         }
         cudaMemcpyAsync(b.R, b.C, (size_t)N * L * 4, cudaMemcpyDeviceToDevice, b.st);
         if (L <= 1024u) {
-            t[kSchool] = run_kind(b, kSchool, N, La, Lb, 3);
+            t[kSchool] = run_kind(b, kSchool, N, La, Lb, kReps);
             if (t[kSchool] > 0.f && !same_result(b, (uint64_t)N * L)) t[kSchool] = -2.f;
         }
         if (tc_fits(La, Lb)) {
-            t[kTensor] = run_kind(b, kTensor, N, La, Lb, 3);
+            t[kTensor] = run_kind(b, kTensor, N, La, Lb, kReps);
             if (t[kTensor] > 0.f && !same_result(b, (uint64_t)N * L)) t[kTensor] = -2.f;
         }
         int best = kNtt;
@@ -424,30 +468,34 @@ cudaError_t autotune(BatchMPContext *ctx, const char *path, uint64_t budget_limb
                 if (shape_ok(need, lk, M)) cands.push_back(Cand{lk, M, -1.f});
             }
             for (size_t i = 0; i < cands.size(); ++i) {
-                {
-                    Table &t = table();
-                    std::lock_guard<std::mutex> g(t.mu);
-                    t.force_log_k = cands[i].log_k;
-                    t.force_M = cands[i].M;
-                }
-                cands[i].ms = run_kind(b, kNtt, N, La, Lb, 3);
+                cands[i].ms = run_shape(b, cands[i].log_k, cands[i].M, N, La, Lb);
                 if (i == 0)
                     cudaMemcpyAsync(b.R, b.C, (size_t)N * L * 4, cudaMemcpyDeviceToDevice, b.st);
                 else if (cands[i].ms > 0.f && !same_result(b, (uint64_t)N * L))
                     cands[i].ms = -2.f;
             }
-            {
-                Table &t = table();
-                std::lock_guard<std::mutex> g(t.mu);
-                t.force_log_k = t.force_M = 0;
-            }
+            // fewer parts unless more are faster by more than repeated runs differ
             size_t best = 0;
             for (size_t i = 1; i < cands.size(); ++i)
-                if (cands[i].ms > 0.f && (cands[best].ms < 0.f || cands[i].ms < cands[best].ms)) best = i;
+                if (cands[i].ms > 0.f && (cands[best].ms < 0.f || cands[i].ms < kClear * cands[best].ms)) best = i;
+            // the smallest batch in which it is still the faster: by halves, then
+            // between the last two to an eighth
+            auto wins = [&](uint32_t n) {
+                return run_shape(b, cands[best].log_k, cands[best].M, n, La, Lb) <
+                       run_shape(b, cands[0].log_k, cands[0].M, n, La, Lb);
+            };
+            uint32_t rows = cands[best].M > 1 ? N : 1u;
+            while (rows > 1u && wins(rows / 2u)) rows /= 2u;
+            for (uint32_t under = rows / 2u; rows - under > std::max(1u, rows / 8u);) {
+                const uint32_t mid = under + (rows - under) / 2u;
+                (wins(mid) ? rows : under) = mid;
+            }
             const uint64_t lo = (1ull << k) + ((uint64_t)(qtr - 1) << (k - 2)) + 1u;
-            snprintf(line, sizeof line, "ntt %llu %llu %d %d   #", (unsigned long long)lo, (unsigned long long)need,
+            snprintf(line, sizeof line, "ntt %llu %llu %d %d", (unsigned long long)lo, (unsigned long long)need,
                      cands[best].log_k, cands[best].M);
             out += line;
+            if (rows > 1u) out += " " + std::to_string(rows);
+            out += "   #";
             for (const Cand &c : cands) {
                 snprintf(line, sizeof line, " K=2^%d,M=%d:%.4f", c.log_k, c.M, c.ms);
                 out += line;

@@ -137,8 +137,9 @@ int gpupi_int_peak(double *imad_winst_per_s, double *alu_winst_per_s);
  * (CUDA-core schoolbook, tensor-core schoolbook or NTT) and the NTT's
  * transform shape (K points x M cosets).  Text lines
  *     mul <max_sum> school|tc|ntt
- *     ntt <min_need> <max_need> <log_k> <M>
- * ('#' comments).  Read at context creation from $GPUPI_TUNE_TABLE, else
+ *     ntt <min_need> <max_need> <log_k> <M> [<rows>]
+ * ('#' comments; rows: the smallest batch the shape is for, 1 if missing,
+ * smaller ones take the next power of two).  Read at context creation from $GPUPI_TUNE_TABLE, else
  * tune_table.txt beside the library.  Results are bit-identical whatever the
  * table says.  load / load_text return the number of entries, or
  * -(line number) of the first malformed line (the table is then unchanged);
@@ -153,8 +154,8 @@ int gpupi_tune_load_text(const char *text);
 int gpupi_tune_reset(void);
 size_t gpupi_tune_describe(char *buf, size_t cap);
 int gpupi_mul_kind(uint32_t L_a, uint32_t L_b, int public_api);
-/* Transform shape (2^log_k points x M cosets) of an NTT product of L_a x L_b
- * limbs under the table in effect (host only). */
+/* Transform shape (2^log_k points x M cosets) of NTT products of L_a x L_b
+ * limbs, in a large batch, under the table in effect (host only). */
 int gpupi_ntt_shape(uint32_t L_a, uint32_t L_b, int *log_k, int *M);
 int gpupi_autotune(gpupi_ctx *ctx, const char *path, uint64_t budget_limbs);
 

@@ -120,3 +120,43 @@ def test_autotune_writes_a_table_that_keeps_pi_exact(ctx, tmp_path):
     import pi_ref
     r = g.pi_compute(fx["digits"], ctx)
     assert r.ret_len == fx["ret_len"] and pi_ref.mod_hash(r.ret) == fx["ret_hash"]
+
+
+def _product(c, N, La, Lb, seed):
+    """launches, families and workspace of N exact products"""
+    import gpupi_b200 as g
+    rng = np.random.default_rng(seed)
+    A = rng.integers(0, 1 << 32, size=N * La, dtype=np.uint64).astype(np.uint32)
+    B = rng.integers(0, 1 << 32, size=N * Lb, dtype=np.uint64).astype(np.uint32)
+    C = np.zeros(N * (La + Lb), dtype=np.uint32)
+    dA, dB, dC = to_dev(A), to_dev(B), to_dev(C)
+    n0 = g.launch_count()
+    fams = _families(lambda: c.mul(N, dA.ptr, La, La, dB.ptr, Lb, Lb, dC.ptr, La + Lb, La + Lb))
+    n = g.launch_count() - n0
+    assert np.array_equal(dC.numpy(), ref.mul(N, A, La, La, B, Lb, Lb, C, La + Lb))
+    return n, fams, c.workspace_size
+
+
+@pytest.mark.parametrize("La,Lb", [(10000, 9000), (20000, 20000), (40000, 39000), (200000, 150000)])
+def test_single_products_take_few_launches(ctx, La, Lb):
+    """Under the shipped table one product is not split into parts, whose
+    launches cost more than the points they save: columns of A and B, rows,
+    inverse columns, CRT and fix-up."""
+    assert _product(ctx, 1, La, Lb, La)[0] <= 6
+
+
+def test_smallest_batch_of_a_shape():
+    """Either side of an entry's smallest batch, and room for the smaller
+    batches in the workspace of the larger."""
+    import gpupi_b200 as g
+    c = g.Context()
+    g.tune_load(text="ntt 16385 24576 13 3 5\nntt 24577 32768 13 4 3\n")
+    try:
+        _, fams, room = _product(c, 5, 10000, 9000, 1)
+        assert "ntt_coset_combine" in fams
+        for N, La, Lb in [(4, 10000, 9000), (1, 12000, 12577), (2, 8200, 8187)]:
+            _, fams, now = _product(c, N, La, Lb, N)
+            assert "ntt_coset_combine" not in fams and now == room
+        assert "ntt_coset_combine" in _product(c, 3, 16000, 15000, 9)[1]
+    finally:
+        c.close()

@@ -68,3 +68,11 @@ def test_table_file_round_trip(tmp_path):
     assert g.mul_kind(1000, 1000) == "tc" and g.ntt_shape(9000, 9000) == (14, 2)
     with pytest.raises(g.GpupiError):
         g.tune_load(tmp_path / "missing.txt")
+
+
+def test_smallest_batch_of_a_shape():
+    assert g.tune_load(text="ntt 16385 24576 13 3 48\nntt 32769 40960 13 5\n") == 2
+    assert "ntt 16385 24576 13 3 48\n" in g.tune_describe() and "ntt 32769 40960 13 5\n" in g.tune_describe()
+    assert g.ntt_shape(10000, 9000) == (13, 3)      # of a large batch
+    with pytest.raises(g.GpupiError):
+        g.tune_load(text="ntt 16385 24576 13 3 0\n")
