@@ -586,9 +586,20 @@ constexpr int kRowCtas = 2;   // per SM: 64 registers a thread, 2 x 97 KiB share
 static_assert(kRowPoints == 16 * 256, "a group holds one segment in registers");
 
 constexpr size_t row_smem_bytes() { return (size_t)kRowGroups * kTilePad * 4u + 2u * kRowPoints * 8u; }
-inline unsigned row_grid(uint64_t segments) {   // all primes' segments
-    return (unsigned)std::min<uint64_t>((segments + kRowGroups - 1) / kRowGroups, (uint64_t)kNumSMs * kRowCtas);
+// CTAs for all primes' segments.  Up to one per SM a segment has a CTA of its
+// own: two in one CTA would share an SM while others idle, and a CTA's share
+// across two primes loads both primes' tables one after the other (the three
+// segments of one 2047 x 2047-limb product in two CTAs: 22.6 us a product, in three
+// 16.4).  Above that the groups of a CTA share the tables (297 segments: 26.7 us
+// in 149 CTAs, 27.9 in 296).
+constexpr unsigned row_grid(uint64_t segments) {
+    return segments <= (uint64_t)kNumSMs ? (unsigned)segments
+           : (segments + kRowGroups - 1) / kRowGroups < (uint64_t)kNumSMs * kRowCtas
+               ? (unsigned)((segments + kRowGroups - 1) / kRowGroups)
+               : (unsigned)(kNumSMs * kRowCtas);
 }
+static_assert(row_grid(3) == 3 && row_grid(148) == 148 && row_grid(297) == 149 &&
+              row_grid(1 << 20) == kNumSMs * kRowCtas, "CTAs of the row kernels");
 
 struct RowShared {
     uint32_t *tile;   // this group's

@@ -68,15 +68,17 @@ def test_column_lengths(ctx, shape, log_k, M):
     product(ctx, 1, full - 300, 300, "pair", rng)
 
 
-@pytest.mark.parametrize("N", [1, 2, 99, 197, 198, 297])
+@pytest.mark.parametrize("N", [1, 2, 49, 50, 99, 197, 198, 297])
 def test_row_groups(ctx, N):
-    """Rows of one 4096-point segment per prime, around two groups per CTA and
-    148 x 2 CTAs (3 N segments in all), and a prime change inside a CTA's run."""
+    """Rows of one 4096-point segment per prime, around a CTA per segment (148),
+    two groups per CTA and 148 x 2 CTAs (3 N segments in all), and a prime
+    change inside a CTA's run; operands longer than half a segment and not
+    (the first level then only multiplies)."""
     rng = np.random.default_rng(N)
-    La, Lb = 70, 4000
-    product(ctx, N, La, Lb, "pair", rng)
-    product(ctx, N, La, Lb, "bcast", rng)
-    product(ctx, N, 90, 90, "square", rng)
+    product(ctx, N, 70, 4000, "pair", rng)
+    product(ctx, N, 70, 4000, "bcast", rng)
+    product(ctx, N, 2048, 2040, "pair", rng)
+    product(ctx, N, 2047, 0, "square", rng)
 
 
 @pytest.mark.parametrize("table", [None, "mul 24 school\n", "mul 48 school\nmul 3072 tc\n"])
