@@ -229,16 +229,13 @@ bool ntt_shape_override(uint64_t need, uint32_t N, int *log_k, int *M) {
 // the table gives larger ones another shape: the largest `rows` of the needs up
 // to the same power of two.
 uint32_t ntt_small_batch(uint64_t need) {
-    auto octave = [](uint64_t n) {
-        int k = 0;
-        while ((1ull << k) < n) ++k;
-        return k;
-    };
+    uint64_t top = 1;
+    while (top < need) top <<= 1;
     Table &t = table();
     std::lock_guard<std::mutex> g(t.mu);
     uint32_t rows = 1u;
     for (const NttEntry &e : t.ntt)
-        if (octave(e.min_need) <= octave(need) && octave(e.max_need) >= octave(need)) rows = std::max(rows, e.rows);
+        if (e.min_need <= top && e.max_need > top / 2u) rows = std::max(rows, e.rows);
     return rows;
 }
 
