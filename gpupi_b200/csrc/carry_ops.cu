@@ -22,7 +22,8 @@
 //   * lanes per row    - rows of up to 125 limbs: 4, 8, 16 or 32 lanes per
 //                        row, one ballot pair;
 //   * warp per row     - longer rows up to 4096 limbs (or very many rows):
-//                        512 limbs per step, the carry kept warp-uniform;
+//                        256 or 512 limbs per step, the carry kept warp-uniform; rows
+//                        that fill little of that one limb per lane;
 //   * tiles + fix-up   - long rows: each CTA owns a 4096-limb tile, writes its
 //                        result assuming carry-in 0 plus (generate, propagate)
 //                        flags; a second kernel scans the flags of each row and
@@ -45,18 +46,32 @@ namespace gpupi {
 
 // ---------------------------------------------------------------------------
 // Operand generators: read() gives limbs j .. j + 3 of the two streams (j may
-// be as low as -3; limbs below 0 are 0).
+// be as low as -3; limbs below 0 are 0), limb() limb j.
 // ---------------------------------------------------------------------------
+
+// How a chunk is read: limb by limb; in 128-bit loads where the chunk's words
+// lie inside the row; or where those of the whole warp (its lanes' chunks in
+// sequence) do.  Inside one warp lanes that take different paths wait for one
+// another's loads, which rows of a few hundred limbs, mostly ends, pay for
+// (65,536 sums of 200 limbs 67 -> 53 us with kByWarp); in the long rows' tiles the
+// ends are few, and the common decision costs more than it saves (2^26 limbs,
+// five operations: 574 us with kByLane, 587 with kByWarp).
+enum Read { kByLimb, kByLane, kByWarp };
 
 // out[v] = r[j + v], 0 outside [0, len).  Inside the row: one 128-bit load
 // when r + j is 16-byte aligned; otherwise the two aligned words that hold the
 // four limbs, where both lie inside the row (the second is the neighbouring
 // thread's first and comes from L1); limb by limb at the row's ends.  The
 // misalignment is the same for all chunks of a row.
-template <bool VEC>
+template <Read MODE>
 __device__ __forceinline__ void read4(const uint32_t *r, uint32_t len, int64_t j, uint32_t (&o)[4]) {
     const uint32_t *p = r + j;
-    if (VEC && j >= 0 && j + 4 <= (int64_t)len) {
+    bool within = j >= 0 && j + 4 <= (int64_t)len;   // the four limbs
+    if (MODE == kByWarp) {   // and the words that hold those of the warp
+        const int64_t first = j - 4 * (int64_t)lane_id();
+        within = first >= 3 && first + 132 <= (int64_t)len;
+    }
+    if (MODE != kByLimb && within) {
         const uint32_t m = ((uintptr_t)p >> 2) & 3u;
         if (m == 0u) {
             const uint4 q = *reinterpret_cast<const uint4 *>(p);
@@ -66,7 +81,7 @@ __device__ __forceinline__ void read4(const uint32_t *r, uint32_t len, int64_t j
             o[3] = q.w;
             return;
         }
-        if (j >= (int64_t)m && j - m + 8 <= (int64_t)len) {
+        if (MODE == kByWarp || (j >= (int64_t)m && j - m + 8 <= (int64_t)len)) {
             const uint4 a = *reinterpret_cast<const uint4 *>(p - m);
             const uint4 b = *reinterpret_cast<const uint4 *>(p - m + 4);
             o[0] = m == 1u ? a.y : (m == 2u ? a.z : a.w);
@@ -81,42 +96,53 @@ __device__ __forceinline__ void read4(const uint32_t *r, uint32_t len, int64_t j
 }
 
 struct GenTwo {
+    static constexpr int kStreams = 2;   // operands read from memory
     const uint32_t *A;
     const uint32_t *B;
     uint32_t La, Lb;
     uint64_t sA, sB;
-    template <bool VEC>
+    template <Read MODE>
     __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
-        read4<VEC>(A + row * sA, La, j, x);
-        read4<VEC>(B + row * sB, Lb, j, y);
+        read4<MODE>(A + row * sA, La, j, x);
+        read4<MODE>(B + row * sB, Lb, j, y);
+    }
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+        x = (j < La) ? A[row * sA + j] : 0u;
+        y = (j < Lb) ? B[row * sB + j] : 0u;
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc) + std::min(Lb, Lc); }
 };
 
 struct GenSmall {
+    static constexpr int kStreams = 1;   // operands read from memory
     const uint32_t *A;
     uint32_t b;
     uint32_t La;
     uint64_t sA;
-    template <bool VEC>
+    template <Read MODE>
     __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
-        read4<VEC>(A + row * sA, La, j, x);
+        read4<MODE>(A + row * sA, La, j, x);
 #pragma unroll
         for (int v = 0; v < 4; ++v) y[v] = (j + v == 0) ? b : 0u;
+    }
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+        x = (j < La) ? A[row * sA + j] : 0u;
+        y = (j == 0u) ? b : 0u;
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
 
 struct GenMulSmall {
+    static constexpr int kStreams = 1;   // operands read from memory
     const uint32_t *A;
     uint32_t b;
     uint32_t La;
     uint64_t sA;
-    template <bool VEC>
+    template <Read MODE>
     __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
         const uint32_t *r = A + row * sA;
         uint32_t a[4];
-        read4<VEC>(r, La, j, a);
+        read4<MODE>(r, La, j, a);
         const uint32_t prev = ((uint64_t)(j - 1) < (uint64_t)La) ? r[j - 1] : 0u;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -124,25 +150,39 @@ struct GenMulSmall {
             y[v] = __umulhi(v ? a[v - 1] : prev, b);
         }
     }
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+        const uint32_t *r = A + row * sA;
+        x = (j < La) ? r[j] * b : 0u;
+        y = (j >= 1u && j - 1u < La) ? __umulhi(r[j - 1u], b) : 0u;
+    }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
 
 struct GenShiftTwo {
+    static constexpr int kStreams = 2;   // operands read from memory
     const uint32_t *A;
     const uint32_t *B;
     uint32_t La, Lb;
     uint64_t sA, sB;
     uint32_t word, bit;
-    template <bool VEC>
+    template <Read MODE>
     __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
         const uint32_t *r = A + row * sA;
         const int64_t i = j - (int64_t)word;
         uint32_t a[4];
-        read4<VEC>(r, La, i, a);
+        read4<MODE>(r, La, i, a);
         const uint32_t prev = ((uint64_t)(i - 1) < (uint64_t)La) ? r[i - 1] : 0u;
 #pragma unroll
         for (int v = 0; v < 4; ++v) x[v] = __funnelshift_l(v ? a[v - 1] : prev, a[v], bit);   // bit < 32
-        read4<VEC>(B + row * sB, Lb, j, y);
+        read4<MODE>(B + row * sB, Lb, j, y);
+    }
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+        const uint32_t *r = A + row * sA;
+        const uint32_t i = j - word;
+        const uint32_t lo = (j >= word && i < La) ? r[i] : 0u;
+        const uint32_t prev = (j > word && i - 1u < La) ? r[i - 1u] : 0u;
+        x = __funnelshift_l(prev, lo, bit);   // bit < 32
+        y = (j < Lb) ? B[row * sB + j] : 0u;
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc) + std::min(Lb, Lc); }
 };
@@ -222,7 +262,7 @@ __global__ void __launch_bounds__(256) carry_lane_rows(Gen gen, uint32_t *C, uin
             g[u] = p[u] = false;
             if (row < N) {
                 uint32_t x[4], y[4];
-                gen.template read<false>((uint32_t)row, 4 * (int64_t)gl - row_offset(C + row * sC), x, y);
+                gen.template read<kByLimb>((uint32_t)row, 4 * (int64_t)gl - row_offset(C + row * sC), x, y);
                 chunk_raw<SUB>(x, y, s[u], g[u], p[u]);
             }
         }
@@ -241,6 +281,47 @@ __global__ void __launch_bounds__(256) carry_lane_rows(Gen gen, uint32_t *C, uin
     }
 }
 
+// A warp per row, one limb per lane, four 32-limb groups per step: for rows
+// whose last 128-limb group of carry_warp_rows would be mostly empty and whose
+// chunks are mostly at an end of the row (see run_carry).
+template <class Gen, bool SUB>
+__global__ void __launch_bounds__(256) carry_limb_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
+    constexpr int kGroups = 4;
+    const uint32_t lane = lane_id();
+    const uint32_t warps_per_cta = blockDim.x >> 5;
+    const uint32_t gwarp = blockIdx.x * warps_per_cta + (threadIdx.x >> 5);
+    const uint32_t nwarps = gridDim.x * warps_per_cta;
+    for (uint32_t row = gwarp; row < N; row += nwarps) {
+        uint32_t *out = C + row * sC;
+        uint32_t cin = 0u;
+        for (uint32_t base = 0; base < Lc; base += 32u * kGroups) {
+            uint32_t s[kGroups], gm[kGroups], pm[kGroups];
+#pragma unroll
+            for (int u = 0; u < kGroups; ++u) {
+                const uint32_t j = base + u * 32u + lane;
+                uint32_t x = 0u, y = 0u;
+                if (j < Lc) gen.limb(row, j, x, y);
+                s[u] = SUB ? x - y : x + y;
+                gm[u] = __ballot_sync(0xffffffffu, SUB ? x < y : s[u] < x);
+                pm[u] = __ballot_sync(0xffffffffu, s[u] == (SUB ? 0u : 0xffffffffu));
+            }
+#pragma unroll
+            for (int u = 0; u < kGroups; ++u) {
+                const uint32_t j = base + u * 32u + lane;
+                const GroupCarry gc = resolve_group(gm[u], pm[u], cin);
+                cin = gc.carry_out;
+                const uint32_t c = (gc.carry_in_mask >> lane) & 1u;
+                if (j < Lc) out[j] = SUB ? s[u] - c : s[u] + c;
+            }
+        }
+    }
+}
+
+// A warp per row, UNROLL groups of 128 limbs per step.  Two for batches: the
+// registers of four (64 a thread) leave 32 warps per SM, which cost rows of 500
+// to 1000 limbs a second wave (20,000 sums of 600 limbs 45 us with four, 37 with
+// two; 65,536 of 1600 limbs 306 and 284).  Four for rows that run alone (one of
+// 4000 limbs 18.5 us with four, 20.5 with two).
 template <class Gen, bool SUB, int UNROLL>
 __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
     const uint32_t lane = lane_id();
@@ -256,7 +337,7 @@ __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uin
             for (int u = 0; u < UNROLL; ++u) {
                 uint32_t x[4], y[4];
                 bool g, p;
-                gen.template read<true>(row, base + u * 128 + 4 * lane, x, y);
+                gen.template read<kByWarp>(row, base + u * 128 + 4 * lane, x, y);
                 chunk_raw<SUB>(x, y, s[u], g, p);
                 gm[u] = __ballot_sync(0xffffffffu, g);
                 pm[u] = __ballot_sync(0xffffffffu, p);
@@ -303,7 +384,7 @@ carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_r
     for (int u = 0; u < kTileSub; ++u) {
         uint32_t x[4], y[4];
         bool g, p;
-        gen.template read<true>(row, base + u * (128 * kTileWarps), x, y);
+        gen.template read<kByLane>(row, base + u * (128 * kTileWarps), x, y);
         chunk_raw<SUB>(x, y, s[u], g, p);
         gm[u] = __ballot_sync(0xffffffffu, g);
         pm[u] = __ballot_sync(0xffffffffu, p);
@@ -368,8 +449,17 @@ static void run_carry(const Gen &gen, uint32_t *C, uint32_t N, uint32_t Lc, uint
             launch_lanes<Gen, SUB, 32, 2>(gen, C, N, Lc, sC, st);
         GPUPI_LAUNCH_CHECK();
     } else if (plan == CarryPlan::Warp) {
-        const unsigned warps = 8;
-        carry_warp_rows<Gen, SUB, 4><<<grid_for(N, warps), warps * 32, 0, st>>>(gen, C, sC, N, Lc);
+        const unsigned warps = 8, grid = grid_for(N, warps);
+        // Measured, one limb per lane against four (us, 65,536 rows): sums of 126
+        // limbs 20 / 29, 160 35 / 37, 200 42 / 40, 253 49 / 43, 300 60 / 64, 350
+        // 67 / 68, 400 78 / 75; one operand times a limb 126 16 / 23, 160 27 / 23.
+        const bool limbs = Gen::kStreams == 2 ? Lc <= 192u || (Lc > 253u && Lc <= 381u && N >= 4096u) : Lc <= 144u;
+        if (limbs)
+            carry_limb_rows<Gen, SUB><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
+        else if (N <= (uint32_t)kNumSMs)
+            carry_warp_rows<Gen, SUB, 4><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
+        else
+            carry_warp_rows<Gen, SUB, 2><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
         GPUPI_LAUNCH_CHECK();
     } else {
         const uint32_t tiles = carry_tile_count(Lc);

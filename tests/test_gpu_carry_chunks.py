@@ -57,8 +57,8 @@ def test_in_place_misaligned(ctx, op, L):
 @pytest.mark.parametrize("tiles", [33, 1023, 1024, 1025, 3 * 1024 + 1])
 @pytest.mark.parametrize("off", [0, 1])
 def test_carry_through_many_tiles(ctx, tiles, off):
-    """(2^(32 L) - 1) + 1 and its mirror 2^(32 L) - 1 - (2^(32 L) - 1) ... through
-    every tile, then the same with one absorbing limb on the way."""
+    """(2^(32 L) - 1) + 1 through every tile, then with one absorbing limb on the
+    way; 0 - 1 through every tile, and up to one limb that absorbs it."""
     import torch
     L = tiles * 4096 - 5
     A = torch.full((L + off,), -1, dtype=torch.int32, device="cuda")
@@ -73,9 +73,42 @@ def test_carry_through_many_tiles(ctx, tiles, off):
     ctx.add(1, a, L, L, b, 1, 1, c, L + 1, L + 1)
     assert int(C[off:off + stop].ne(0).sum()) == 0 and int(C[off + stop]) == 42
     assert int(C[off + stop + 1:off + L].ne(-1).sum()) == 0 and int(C[off + L]) == 0
-    # 0 - 1 borrows through every limb up to the first nonzero one
+    # 0 - 1 borrows through every limb, or up to the first nonzero one
     A.zero_()
+    ctx.sub(1, a, L, L, b, 1, 1, c, L + 1, L + 1)
+    assert int(C[off:off + L + 1].ne(-1).sum()) == 0
     A[off + stop] = 41
     ctx.sub(1, a, L, L, b, 1, 1, c, L + 1, L + 1)
     assert int(C[off:off + stop].ne(-1).sum()) == 0 and int(C[off + stop]) == 40
     assert int(C[off + stop + 1:off + L + 1].ne(0).sum()) == 0
+
+
+WARP_ROWS = [(5, Lc) for Lc in (127, 128, 129, 144, 145, 192, 193, 253, 254, 381, 382, 511, 1021, 1300)]
+WARP_ROWS += [(148, 400), (149, 400), (149, 193), (4095, 254), (4096, 254), (4096, 381), (4096, 382)]
+
+
+@pytest.mark.parametrize("N,Lc", WARP_ROWS)
+def test_rows_of_a_warp(ctx, N, Lc):
+    """Rows a warp handles one limb or four limbs per lane, either side of each
+    change between the two and between 256 and 512 limbs per step, with rows
+    that carry all the way and strides that change the alignment."""
+    rng = np.random.default_rng(Lc * 5000 + N)
+    La, Lb, sA, sB, sC = Lc - 1, Lc - 2, Lc, Lc + 1, Lc + 2
+    A, B, C = rand_buf(rng, N, sA, La), rand_buf(rng, N, sB, Lb), rand_buf(rng, N, sC, 0)
+    for r in range(0, N, 3):
+        A[r * sA:r * sA + La] = 0xFFFFFFFF if r % 2 else 0
+        B[r * sB:r * sB + Lb] = 0
+        B[r * sB] = 1
+    for op in ("add", "sub", "add_small", "sub_small", "mul_small", "shift_add", "shift_sub"):
+        dA, dB, dC = to_dev(A), to_dev(B), to_dev(C)
+        a, b, c = (dA.ptr, La, sA), (dB.ptr, Lb, sB), (dC.ptr, Lc, sC)
+        if op.endswith("small"):
+            getattr(ctx, op)(N, *a, 0xFFFFFFFB, *c)
+            want = getattr(ref, op)(N, A, La, sA, 0xFFFFFFFB, C, Lc, sC)
+        elif op.startswith("shift"):
+            getattr(ctx, op)(N, *a, *b, 45, *c)
+            want = getattr(ref, op)(N, A, La, sA, B, Lb, sB, 45, C, Lc, sC)
+        else:
+            getattr(ctx, op)(N, *a, *b, *c)
+            want = getattr(ref, op)(N, A, La, sA, B, Lb, sB, C, Lc, sC)
+        assert np.array_equal(dC.numpy(), want), op
