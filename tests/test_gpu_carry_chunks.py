@@ -112,3 +112,15 @@ def test_rows_of_a_warp(ctx, N, Lc):
             getattr(ctx, op)(N, *a, *b, *c)
             want = getattr(ref, op)(N, A, La, sA, B, Lb, sB, C, Lc, sC)
         assert np.array_equal(dC.numpy(), want), op
+
+
+@pytest.mark.parametrize("N,L", [(1, 1), (7, 33), (7, 128), (8, 8), (8, 9), (9, 31), (33, 32), (33, 33), (40, 40),
+                                 (40, 41), (65, 102), ((1 << 18) - 1, 3), (1 << 18, 3), ((1 << 18) + 5, 1)])
+def test_exactdiv_kernels(ctx, N, L):
+    """Either side of the choice between the two kernels, and of their groups
+    of eight limbs; rows need not be multiples of the divisor."""
+    rng = np.random.default_rng(N + L)
+    A = rand_buf(rng, N, L + 1, L)
+    dA = to_dev(A)
+    ctx.exactdiv_small(N, dA.ptr, L, L + 1, 0x13579BDF)
+    assert np.array_equal(dA.numpy(), ref.exactdiv_small(N, A, L, L + 1, 0x13579BDF))
