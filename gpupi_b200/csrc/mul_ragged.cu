@@ -7,12 +7,14 @@
 // written in place:
 //   * L_a = 0 or L_b = 0: the L_a + L_b output limbs are zeroed;
 //   * products the tune table gives to the CUDA-core schoolbook: one
-//     k_school_cols launch; those it gives to the tensor-core schoolbook:
-//     up to four k_mul_tc launches by the shared memory their products need,
-//     the largest first (a launch's is sized for its largest product, so the
-//     others get several CTAs per SM in launches of their own; the shorter
-//     operand decides it: by length alone, products of a long and a short
-//     operand ran one per SM beside the balanced ones);
+//     k_school_cols launch; those it gives to the tensor-core schoolbook: one
+//     k_mul_tc launch, those that need most shared memory first, so that the
+//     last CTAs to finish hold short products.  (Launches of their own for
+//     those of less than 112, 56 and 28 KiB, with more CTAs per SM, were faster
+//     only for some batches of thousands (4096 products of 300..2000 limbs 214
+//     against 222 us, of 100..1300 limbs equal) and slower for all smaller
+//     ones, a launch's last wave each: 600 of 200..1400 limbs 42 against 29
+//     us, 16 of 64..512 limbs 18.5 against 12.8.)
 //   * otherwise by transform size (powers of two up to 2^13 points, quarters of
 //     an octave above): one NTT batch per bucket at its largest product's shape.
 // 4096 products of 8..4096 limbs per operand: gathering the NTT products into
@@ -58,8 +60,6 @@ unsigned grid_rows(uint32_t n) { return (unsigned)std::max<uint32_t>(1u, std::mi
 // shared memory from the largest, NTT buckets.
 constexpr uint32_t kZero = 0u, kSchoolGroup = 1u, kTensorGroup = 2u;
 constexpr uint32_t kTensorGroups = 256u;
-// limits of the launches: one, two, four CTAs in an SM's 228 KiB, more
-constexpr uint32_t kTensorLimits[] = {112u, 56u, 28u, 0u};
 constexpr uint32_t kNttGroup = kTensorGroup + kTensorGroups;
 constexpr uint32_t kNttGroups = 4u * 32u;
 constexpr uint32_t kGroups = kNttGroup + kNttGroups;
@@ -130,22 +130,18 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         for (uint32_t i = start[1]; i < start[2]; ++i) work += (uint64_t)rows[i].La * rows[i].Lb;
         school_mul_ragged(A, B, C, ns, dr + start[1], work);
     }
-    uint32_t first = start[kTensorGroup];
-    for (const uint32_t limit : kTensorLimits) {
-        // products of at least `limit` KiB: groups up to kTensorGroups - 1 - limit
-        const uint32_t last = start[kTensorGroup + kTensorGroups - limit];
-        if (err != cudaSuccess || last == first) continue;
+    const uint32_t tc0 = start[kTensorGroup];
+    if (err == cudaSuccess && ntt0 > tc0) {
         uint32_t maxQ = 0, maxN = 0;
         uint64_t limbs = 0;
-        for (uint32_t i = first; i < last; ++i) {
+        for (uint32_t i = tc0; i < ntt0; ++i) {
             uint32_t q = 0, n = 0;
             tc_shape(rows[i].La, rows[i].Lb, &q, &n);
             maxQ = std::max(maxQ, q);
             maxN = std::max(maxN, n);
             limbs += 2ull * (rows[i].La + rows[i].Lb);
         }
-        err = tc_mul_ragged(A, B, C, last - first, dr + first, maxQ, maxN, limbs);
-        first = last;
+        err = tc_mul_ragged(A, B, C, ntt0 - tc0, dr + tc0, maxQ, maxN, limbs);
     }
     if (err == cudaSuccess) err = upload(ntt0, N, &dn);
     for (uint32_t g = kNttGroup; err == cudaSuccess && g < kGroups; ++g) {

@@ -148,3 +148,28 @@ def test_ragged_carry_to_a_short_rows_end(ctx, last):
     dA, dB, dC = to_dev(np.concatenate(A)), to_dev(np.concatenate(B)), to_dev(np.zeros_like(want))
     ctx.mul_ragged(dA.ptr, oa, La, dB.ptr, ob, Lb, dC.ptr, oc)
     assert np.array_equal(dC.numpy(), want)
+
+
+def test_ragged_tensor_products_in_one_launch(ctx):
+    import gpupi_b200 as g
+    rng = np.random.default_rng(2)
+    La, Lb = (rng.integers(70, 1200, size=40).astype(np.uint32) for _ in range(2))
+    A, B = rand_buf(rng, 1, int(La.sum()), int(La.sum())), rand_buf(rng, 1, int(Lb.sum()), int(Lb.sum()))
+    oa, ob, oc = (np.concatenate([[0], np.cumsum(x)[:-1]]).astype(np.uint64) for x in (La, Lb, La + Lb))
+    dA, dB, dC = to_dev(A), to_dev(B), to_dev(np.zeros(int((La + Lb).sum()), dtype=np.uint32))
+    try:
+        g.tune_load(text="mul 2560 tc\n")
+        g.timer_reset()
+        g.timer_enable(True)
+        ctx.mul_ragged(dA.ptr, oa, La, dB.ptr, ob, Lb, dC.ptr, oc)
+        g.timer_enable(False)
+        assert g.timer_report()["schoolbook_tc"][0] == 1
+    finally:
+        g.timer_enable(False)
+        g.timer_reset()
+        g.tune_load(g.TUNE_TABLE_PATH)
+    got = dC.numpy()
+    for i in range(40):
+        x, y, z = (int.from_bytes(v[int(o[i]):int(o[i]) + int(n)].tobytes(), "little")
+                   for v, o, n in ((A, oa, La[i]), (B, ob, Lb[i]), (got, oc, La[i] + Lb[i])))
+        assert z == x * y
