@@ -634,7 +634,7 @@ extern "C" int gpupi_mp_add_noalloc(uint32_t N, const uint32_t *d_A, uint32_t L_
     if (N == 0u || L_c == 0u) return 0;
     uint32_t *flags = nullptr;
     if (plan_for(N, L_c) == CarryPlan::Tiles) {
-        const uint64_t tiles = (uint64_t)N * ((L_c + kTileSpan - 1u) / kTileSpan);
+        const uint64_t tiles = N * (((uint64_t)L_c + kTileSpan - 1u) / kTileSpan);
         if (tiles > kNoAllocMaxTiles) return (int)cudaErrorInvalidValue;   // beyond the fixed array
         const cudaError_t err = noalloc_flags_address(&flags);
         if (err != cudaSuccess) return (int)err;

@@ -1,6 +1,7 @@
 """CPU checks of the native boundary: the library builds for sm_100a, loads,
 and exports every symbol include/gpupi_c.h declares plus the reference's C++
 API (mangled names) so gpupi's own callers link unchanged.  No compute calls."""
+import ctypes
 import re
 import subprocess
 from pathlib import Path
@@ -79,3 +80,12 @@ def test_no_cpu_fallback_without_gpu():
         pytest.skip("a GPU is present")
     with pytest.raises(g.GpupiError):
         g.Context()
+
+
+@pytest.mark.parametrize("L", [(1 << 28) + 1, (1 << 32) - 4096, (1 << 32) - 4095, (1 << 32) - 1])
+def test_noalloc_add_refuses_beyond_its_flags(built, L):
+    """More tiles than the fixed flag array holds: an invalid value before any
+    device work, up to the longest length (whose tile count must not wrap)."""
+    import gpupi_b200 as g
+    p = ctypes.c_void_p(4096)   # never dereferenced
+    assert g.lib().gpupi_mp_add_noalloc(1, p, 1, 1, p, 1, 1, p, L, L) == 1
