@@ -44,19 +44,15 @@ from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent
 
-# DRAM traffic of the dominant kernel family relative to its algorithmic
-# bytes, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum of
-# k_rows_r<12> on a 2^22 x 2^22-limb product: 264.0 MB against 302.0 MB of
-# algorithmic bytes; part of the output is still in L2 at kernel end).  The
-# pi run's launches are scaled by their algorithmic bytes.
 BBP_POSITIONS = 64
 # DRAM bytes (read + write) over algorithmic bytes of one launch, from ncu
-# captures (profiles/ntt_rows_cols_4Mi.md, profiles/ntt_split_rows_4Mi.md,
-# profiles/ntt_rows_level_pi1e8.md); applied to each launch of the family
-NCU_TRAFFIC_RATIO = {"ntt_rows_fused": 264.006 / 301.990,
-                     "ntt_cols_fwd_first": 229.642496 / 234.881024,
-                     "ntt_rows_level": (2630.51 + 1619.05) / 4026.531840}
-NCU_TRAFFIC_SOURCE = {"ntt_rows_fused": "ncu capture of k_rows_r<12> on a 2^22 x 2^22-limb product, "
+# captures of dram__bytes_read.sum + dram__bytes_write.sum
+# (profiles/ntt_passes_2_26.md, profiles/ntt_rows_level_pi1e8.md); applied to
+# each launch of the family
+NCU_TRAFFIC_RATIO = {"ntt_rows_fused": (206.430 + 56.106) / 301.990,
+                     "ntt_cols_fwd_first": (83.938 + 142.818) / 234.881,
+                     "ntt_rows_level": (3956.55 + 1584.26) / 4026.532}
+NCU_TRAFFIC_SOURCE = {"ntt_rows_fused": "ncu capture of k_rows on a 2^22 x 2^22-limb product, "
                                         "scaled to each launch by its algorithmic bytes",
                       "ntt_cols_fwd_first": "ncu capture of k_cols_r<6, first, fwd, pair> on a 2^22 x 2^22-limb "
                                             "product, scaled to each launch by its algorithmic bytes",
@@ -67,16 +63,17 @@ NCU_TRAFFIC_SOURCE = {"ntt_rows_fused": "ncu capture of k_rows_r<12> on a 2^22 x
 # 1e8 digits with the library's kernel-timer bytes of the same computation
 # (profiles/int_pipes_pi1e8.md).  Scaled to this run's bytes and divided by
 # the live integer-pipe peaks they give each family's integer roofline.
+# (The folding kernel has none: its instructions grow with cosets times
+# blocks, not with bytes, so its count at 1e8 digits says nothing about 1e9.)
 INT_WINST_PER_BYTE = {
-    "ntt_rows_level": (0.183426, 0.182728, 0.440234), "ntt_cols_fwd_first": (0.118559, 0.11696, 0.289975),
-    "ntt_cols_inv": (0.073674, 0.074348, 0.182748), "schoolbook_tc": (0.175881, 0.347193, 0.872551),
-    "ntt_crt_carry": (0.050113, 0.045814, 0.125112), "ntt_rows_fused": (0.180556, 0.177752, 0.424416),
-    "ntt_cols_fwd": (0.069824, 0.069802, 0.175721), "schoolbook": (0.219156, 0.17921, 0.53567),
-    "ntt_local": (0.439652, 0.430948, 1.015859), "carry_chain": (0.032343, 0.099566, 0.174273),
+    "ntt_rows_level": (0.183426, 0.182728, 0.440234), "ntt_cols_fwd_first": (0.119126, 0.117517, 0.291312),
+    "ntt_cols_inv": (0.073824, 0.074517, 0.183087), "schoolbook_tc": (0.177557, 0.350959, 0.882674),
+    "ntt_crt_carry": (0.050188, 0.045934, 0.12533), "ntt_rows_fused": (0.18048, 0.17761, 0.423874),
+    "ntt_cols_fwd": (0.069918, 0.069917, 0.17593), "schoolbook": (0.219156, 0.17921, 0.53567),
+    "ntt_local": (0.444573, 0.436102, 1.027391), "carry_chain": (0.027847, 0.08159, 0.142997),
     "ntt_rows_fwd": (0.097792, 0.091607, 0.244568), "ntt_rows_inv": (0.064503, 0.064857, 0.163097),
-    "ntt_fold": (0.113415, 0.126271, 0.417258), "decimal_extract": (0.075693, 0.08626, 0.224201),
-    "ntt_coset_combine": (0.090216, 0.077055, 0.224702), "shift": (0.035647, 0.045182, 0.115069),
-    "decimal_leaf": (0.704212, 0.245135, 1.12563)}
+    "decimal_extract": (0.075693, 0.08626, 0.224201), "ntt_coset_combine": (0.086067, 0.074986, 0.215792),
+    "shift": (0.035647, 0.045182, 0.115069), "decimal_leaf": (0.704212, 0.245135, 1.12563)}
 INT_SOURCE = ("ncu sm__inst_executed_pipe_{fmaheavy,alu}.sum and sm__inst_executed.sum over every launch of "
               "pi_bs_gpu 100000000 (profiles/int_pipes_pi1e8.md), per algorithmic byte, scaled to this run")
 sys.path.insert(0, str(ROOT))

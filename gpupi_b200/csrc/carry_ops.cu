@@ -22,8 +22,9 @@
 //   * lanes per row    - rows of up to 125 limbs: 4, 8, 16 or 32 lanes per
 //                        row, one ballot pair;
 //   * warp per row     - longer rows up to 4096 limbs (or very many rows):
-//                        256 or 512 limbs per step, the carry kept warp-uniform; rows
-//                        that fill little of that one limb per lane;
+//                        256 or 512 limbs per step, the carry kept warp-
+//                        uniform; rows that fill little of that, one limb per
+//                        lane;
 //   * tiles + fix-up   - long rows: each CTA owns a 4096-limb tile, writes its
 //                        result assuming carry-in 0 plus (generate, propagate)
 //                        flags; a second kernel scans the flags of each row and

@@ -155,8 +155,8 @@ __global__ void carry_fixup_kernel(uint32_t *C, uint64_t sC, uint32_t N, uint32_
 // lets a carry through, so nearly always one step; a row of all ones looks
 // back over the whole row, 1024 tiles per step).  Every CTA works for itself
 // and none waits for another; only C is written, never the flags.  A single
-// CTA walking the row instead took 276 us on the 262,144 tiles of a
-// 2^28-limb product and 40 us on 16,385 tiles of 4096 limbs; this takes 3.8
+// CTA walking the row instead took 276 us on the 262,144 tiles of 1024 limbs of
+// a 2^28-limb product and 40 us on 16,385 tiles of 4096 limbs; this takes 3.8
 // and 7.1 us.
 constexpr uint32_t kFixThreads = 256;
 constexpr uint32_t kFixTiles = 4u * kFixThreads;

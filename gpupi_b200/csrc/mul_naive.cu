@@ -1,6 +1,6 @@
 // Batched schoolbook multiplication (gpupi batch_mul_naive.cu:8-273).
 //
-// Two shapes:
+// Three shapes:
 //   * k_school_rows<MB>: one thread per product for operands of at most 16
 //     limbs each (the bottom levels of the splitting tree: 3..16-limb rows in
 //     batches of millions), staged through shared memory.
@@ -11,7 +11,8 @@
 //     3-word register with mad.lo.cc / madc.hi.cc / addc (3 instructions per
 //     32x32 product), then the 96-bit column sums are carried into limbs with
 //     the same chunk/ballot carry as the NTT's CRT stage.  L_a + L_b <= 1024.
-// Both are IMAD-bound; algorithmic work = L_a * L_b 32x32->64 products.
+// The latter two are IMAD-bound, the first by its staging; algorithmic work =
+// L_a * L_b 32x32->64 products.
 #include "common.cuh"
 #include "carry_tile.cuh"
 #include "batch_mul_naive.h"
@@ -188,10 +189,12 @@ struct MadChain<8> {
 // multiply-adds (one instruction each) with no other carry handling; the two
 // lowest words are final after the step and the rest moves down by two words
 // as the second limb's chains write their results.
-// Bound by the multiply-adds (half rate: 4 cycles per warp and scheduler):
-// 262,144 products of 14 x 13 limbs 41.9 -> 26.6 us a call (the previous kernel read
-// and wrote one row per thread straight from memory and kept one serial carry
-// chain per limb of A).
+// Bound by the staging (one 4-byte copy and one index division per limb, no
+// overlap with the arithmetic inside a CTA): 262,144 products of 14 x 13 limbs
+// 41.9 -> 26.6 us a call, of which the multiply-adds (half rate: 4 cycles per
+// warp and scheduler) take about 5.5 (the previous kernel read and wrote one
+// row per thread straight from memory and kept one serial carry chain per limb
+// of A).
 constexpr int kRowsCta = 128;
 constexpr uint32_t kDivShift = 20;   // e / d = e * ceil(2^20 / d) >> 20 for e < 4096, d <= 32
 

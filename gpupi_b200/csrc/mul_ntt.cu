@@ -25,16 +25,19 @@
 //                     each column of a 4096-residue tile, twist by
 //                     w_K^(col * bitrev(pos)), store
 //   k_cols_r          same on each segment for R2 (sizes above 2^22)
-//   k_rows_r          C-point DIF of the A and B segments, pointwise product
-//                     * K^-1, C-point inverse DIT, store
-//   k_cols_r<inv>     untwist + inverse DIT on columns, mirror order
+//   k_rows            C-point DIF of the A and B segments, pointwise product,
+//                     C-point inverse DIT, store (products / R)
+//   k_cols_r<inv>     untwist + inverse DIT on columns, mirror order; the first
+//                     multiplies by K^-1 R too
 //   k_combine<M>      (M > 1) untwist the cosets, inverse Vandermonde
+//   k_combine2        (two parts) T and C's lower coefficients
 //   k_crt             Garner CRT to 96-bit coefficients, carry into limbs
 //                     (+ carry_fixup_kernel when a row spans several tiles)
-// Small products (K <= 4096) are one k_rows_r (or k_rows_small) launch and
-// k_crt.  Every CTA handles one prime, fixed at compile time inside the CTA;
-// the prime is the slowest grid index, so an SM works on one prime's tables
-// and code at a time.
+// Small products (K <= 4096) are one k_rows<limbs> (4096 points), k_rows_r or
+// k_rows_small launch and k_crt.  Code is compiled per prime (immediate
+// operands) and the prime is the slowest index, so an SM works on one prime's
+// tables and code at a time: a CTA of most kernels handles one prime, one of
+// the persistent row kernels a run of segments in that order.
 #include "ntt_core.cuh"
 #include "carry_tile.cuh"
 #include "batch_mul_ntt.h"
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(kThreads) k_fold(NttParams P, FoldArgs a) {
         fold_body<2, REGS>(P, a, b, W);
 }
 
-// Column pass: R = 2^LOG_R (<= 512) points per column, TC = 4096 / R columns
+// Column pass: R = 2^LOG_R (<= 1024) points per column, TC = 4096 / R columns
 // per CTA; segment of S = 2^log_s points viewed as [R][S/R].  PAIR: the
 // forward pass of A and B together (same tile, shared twiddles and twists).
 template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, Load LOAD, int Q>
@@ -445,10 +448,10 @@ constexpr size_t cols_smem_bytes() {   // one or two padded tiles + the twiddle 
     return (size_t)(PAIR ? 2 : 1) * kTilePad * 4u + (size_t)((1 << LOG_R) - 1) * 8u;
 }
 
-// Four CTAs per SM for every pass (64 registers): the paired passes hold two
-// operands' residues, and for the first of them a few words spill, but the
-// extra resident warps hide more of the limb and tile latency (first pass of
-// a 2^24 x 2^24-limb product 0.589 -> 0.541 ms against three CTAs per SM).
+// Four CTAs per SM for every pass (64 registers; of them all, two unpaired first
+// passes spill 16 and 36 bytes): the extra resident warps hide more of the limb
+// and tile latency (first pass of a 2^24 x 2^24-limb product 0.589 -> 0.541 ms
+// against three CTAs per SM).
 template <int LOG_R, bool FROM_LIMBS, bool INVERSE, bool PAIR, Load LOAD>
 __global__ void __launch_bounds__(kThreads, 4) k_cols_r(NttParams P, ColsArgs a) {
     extern __shared__ uint4 cols_smem[];
@@ -819,7 +822,7 @@ __global__ void __launch_bounds__(128) k_rows_small(NttParams P, RowsArgs a) {
 // that order, forms sum_t X_t Y_t / R (mod p), moves the result back to
 // the last stage's order through the tile and runs the inverse stages,
 // leaving the segment in the order the inverse column passes expect, as the
-// fused k_rows_r does.  So a transform computed once serves every product
+// fused k_rows does.  So a transform computed once serves every product
 // it takes part in, and a sum of products costs one inverse transform.
 // ---------------------------------------------------------------------------
 constexpr int kSplitLogC = kRowLog;
@@ -1034,6 +1037,7 @@ __device__ __forceinline__ void level_run(const RowsLevelArgs &a, uint32_t first
     }
 }
 
+// 64 registers a thread (two CTAs of 512): 64 bytes of spill stores.
 __global__ void __launch_bounds__(kRowThreads, kRowCtas) k_rows_level(NttParams P, RowsLevelArgs a, uint32_t segs) {
     extern __shared__ uint4 rows_smem[];
     const RowShared s = row_shared(rows_smem);
@@ -1415,8 +1419,8 @@ static Shape shape_for(uint32_t La, uint32_t Lb) {
     return {kMaxLog, (int)((need + K - 1) / K)};
 }
 
-// Paired passes exist for R >= 32 only (shorter columns twist per residue
-// and would spill with two operands).
+// Paired passes exist for R >= 32 only: shorter columns, of small transforms and
+// second parts, run operand by operand.
 constexpr int kPairMinLogR = 5;
 // Column lengths up to 1024 run as one pass (tiles of 4096 / R columns; for
 // R = 1024 a row segment is half a 32-byte sector, whose other half the

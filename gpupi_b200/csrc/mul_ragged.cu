@@ -107,8 +107,9 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
         std::vector<uint32_t> at(start.begin(), start.end() - 1);
         for (uint32_t i = 0; i < N; ++i) rows[at[group[i]]++] = RaggedRow{offA[i], offB[i], offC[i], La[i], Lb[i]};
     }
-    // descriptors on the device: those of the schoolbooks, and those of the NTT
-    // batches, copied while the former's kernels run
+    // descriptors on the device: those of the schoolbooks first, so that their
+    // kernels start while the host stages those of the NTT batches (pageable
+    // memory; the device copies them after those kernels)
     auto upload = [&](uint32_t from, uint32_t to, RaggedRow **d) {
         const size_t bytes = (size_t)(to - from) * sizeof(RaggedRow);
         if (!bytes) return cudaSuccess;
