@@ -59,8 +59,10 @@ unsigned grid_rows(uint32_t n) { return (unsigned)std::max<uint32_t>(1u, std::mi
 // Group numbers: zero products, schoolbook, tensor-core products by KiB of
 // shared memory from the largest, NTT buckets.
 constexpr uint32_t kZero = 0u, kSchoolGroup = 1u, kTensorGroup = 2u;
-constexpr uint32_t kTensorGroups = 256u;
-constexpr uint32_t kNttGroup = kTensorGroup + kTensorGroups;
+// Products that need half an SM's shared memory or more (sums above 2560 limbs)
+// go to the NTT: one of them would leave the whole launch one CTA per SM.
+constexpr uint32_t kTensorMax = 112u;
+constexpr uint32_t kNttGroup = kTensorGroup + kTensorMax;
 constexpr uint32_t kNttGroups = 4u * 32u;
 constexpr uint32_t kGroups = kNttGroup + kNttGroups;
 
@@ -94,8 +96,8 @@ cudaError_t mul_ragged(BatchMPContext *ctx, uint32_t N, const uint32_t *A, const
             g = kZero;
         else if (kind[i] == 0u)
             g = kSchoolGroup;
-        else if (kind[i] == 1u)
-            g = kTensorGroup + (kTensorGroups - 1u - std::min(kTensorGroups - 1u, tc_smem_bytes(La[i], Lb[i]) >> 10));
+        else if (const uint32_t kib = tc_smem_bytes(La[i], Lb[i]) >> 10; kind[i] == 1u && kib < kTensorMax)
+            g = kTensorGroup + (kTensorMax - 1u - kib);
         else
             g = kNttGroup + ntt_bucket(Lc - 1u);
         group[i] = (uint16_t)g;

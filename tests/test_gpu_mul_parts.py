@@ -81,11 +81,13 @@ def test_row_groups(ctx, N):
     product(ctx, N, 2047, 0, "square", rng)
 
 
-@pytest.mark.parametrize("table", [None, "mul 24 school\n", "mul 48 school\nmul 3072 tc\n"])
+@pytest.mark.parametrize("table", [None, "mul 24 school\n", "mul 48 school\nmul 3072 tc\n",
+                                   "ntt 8100 8192 13 2\nntt 16385 40960 13 5\n"])
 def test_ragged_in_place(ctx, table):
     """Uneven products read and written where they lie: every bucket from a
-    few limbs to the two-part and column-pass sizes, empty operands, operands
-    of very different lengths, unordered output places with gaps left alone."""
+    few limbs to the column-pass sizes, with the last table equal cosets and
+    two-part transforms too, empty operands, operands of very different
+    lengths, unordered output places with gaps left alone."""
     import gpupi_b200 as g
     rng = np.random.default_rng(5)
     pairs = [(1, 1), (0, 7), (9, 0), (3, 40), (200, 3), (130, 126), (255, 2), (250, 260), (1000, 30), (700, 1300),
