@@ -50,6 +50,14 @@ namespace gpupi {
 // be as low as -3; limbs below 0 are 0), limb() limb j.
 // ---------------------------------------------------------------------------
 
+// mul_small reads the source limb below its own, which in place (C is A) may be
+// a result already: at the first limb of a warp's step or of a tile it is taken
+// from here, read before those results were written.
+struct Edge {
+    int64_t at = INT64_MIN;   // limb index
+    uint32_t below = 0u;      // source limb at - 1
+};
+
 // How a chunk is read: limb by limb; in 128-bit loads where the chunk's words
 // lie inside the row; or where those of the whole warp (its lanes' chunks in
 // sequence) do.  Inside one warp lanes that take different paths wait for one
@@ -98,16 +106,17 @@ __device__ __forceinline__ void read4(const uint32_t *r, uint32_t len, int64_t j
 
 struct GenTwo {
     static constexpr int kStreams = 2;   // operands read from memory
+    static constexpr bool kBelow = false;   // reads the limb below its own in place
     const uint32_t *A;
     const uint32_t *B;
     uint32_t La, Lb;
     uint64_t sA, sB;
     template <Read MODE>
-    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4], Edge) const {
         read4<MODE>(A + row * sA, La, j, x);
         read4<MODE>(B + row * sB, Lb, j, y);
     }
-    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y, Edge) const {
         x = (j < La) ? A[row * sA + j] : 0u;
         y = (j < Lb) ? B[row * sB + j] : 0u;
     }
@@ -116,58 +125,71 @@ struct GenTwo {
 
 struct GenSmall {
     static constexpr int kStreams = 1;   // operands read from memory
+    static constexpr bool kBelow = false;   // reads the limb below its own in place
     const uint32_t *A;
     uint32_t b;
     uint32_t La;
     uint64_t sA;
     template <Read MODE>
-    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4], Edge) const {
         read4<MODE>(A + row * sA, La, j, x);
 #pragma unroll
         for (int v = 0; v < 4; ++v) y[v] = (j + v == 0) ? b : 0u;
     }
-    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y, Edge) const {
         x = (j < La) ? A[row * sA + j] : 0u;
         y = (j == 0u) ? b : 0u;
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
 
+// IN_PLACE: C is A (instantiations of their own: the tests at every chunk cost the
+// others 10 to 30 %).
+template <bool IN_PLACE>
 struct GenMulSmall {
     static constexpr int kStreams = 1;   // operands read from memory
+    static constexpr bool kBelow = IN_PLACE;
     const uint32_t *A;
     uint32_t b;
     uint32_t La;
     uint64_t sA;
+    const uint32_t *edges;   // tiles in place: the limb below each tile, else null
+    __device__ __forceinline__ uint32_t below(uint32_t row, int64_t j) const {
+        return ((uint64_t)(j - 1) < (uint64_t)La) ? A[row * sA + j - 1] : 0u;
+    }
     template <Read MODE>
-    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4], Edge e) const {
         const uint32_t *r = A + row * sA;
         uint32_t a[4];
         read4<MODE>(r, La, j, a);
-        const uint32_t prev = ((uint64_t)(j - 1) < (uint64_t)La) ? r[j - 1] : 0u;
+        uint32_t prev = ((uint64_t)(j - 1) < (uint64_t)La) ? r[j - 1] : 0u;
+        if (IN_PLACE && j == e.at) prev = e.below;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             x[v] = a[v] * b;
             y[v] = __umulhi(v ? a[v - 1] : prev, b);
         }
     }
-    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y, Edge e) const {
         const uint32_t *r = A + row * sA;
         x = (j < La) ? r[j] * b : 0u;
-        y = (j >= 1u && j - 1u < La) ? __umulhi(r[j - 1u], b) : 0u;
+        uint32_t prev = (j >= 1u && j - 1u < La) ? r[j - 1u] : 0u;
+        if (IN_PLACE && (int64_t)j == e.at) prev = e.below;
+        y = __umulhi(prev, b);
     }
     double read_limbs(uint32_t Lc) const { return (double)std::min(La, Lc); }
 };
 
 struct GenShiftTwo {
     static constexpr int kStreams = 2;   // operands read from memory
+    static constexpr bool kBelow = false;   // reads the limb below its own in place
     const uint32_t *A;
     const uint32_t *B;
     uint32_t La, Lb;
     uint64_t sA, sB;
     uint32_t word, bit;
     template <Read MODE>
-    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4]) const {
+    __device__ __forceinline__ void read(uint32_t row, int64_t j, uint32_t (&x)[4], uint32_t (&y)[4], Edge) const {
         const uint32_t *r = A + row * sA;
         const int64_t i = j - (int64_t)word;
         uint32_t a[4];
@@ -177,7 +199,7 @@ struct GenShiftTwo {
         for (int v = 0; v < 4; ++v) x[v] = __funnelshift_l(v ? a[v - 1] : prev, a[v], bit);   // bit < 32
         read4<MODE>(B + row * sB, Lb, j, y);
     }
-    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y) const {
+    __device__ __forceinline__ void limb(uint32_t row, uint32_t j, uint32_t &x, uint32_t &y, Edge) const {
         const uint32_t *r = A + row * sA;
         const uint32_t i = j - word;
         const uint32_t lo = (j >= word && i < La) ? r[i] : 0u;
@@ -263,7 +285,7 @@ __global__ void __launch_bounds__(256) carry_lane_rows(Gen gen, uint32_t *C, uin
             g[u] = p[u] = false;
             if (row < N) {
                 uint32_t x[4], y[4];
-                gen.template read<kByLimb>((uint32_t)row, 4 * (int64_t)gl - row_offset(C + row * sC), x, y);
+                gen.template read<kByLimb>((uint32_t)row, 4 * (int64_t)gl - row_offset(C + row * sC), x, y, Edge{});
                 chunk_raw<SUB>(x, y, s[u], g[u], p[u]);
             }
         }
@@ -282,6 +304,16 @@ __global__ void __launch_bounds__(256) carry_lane_rows(Gen gen, uint32_t *C, uin
     }
 }
 
+// The limb below a warp's next step, before this step's results are written.
+template <class Gen>
+__device__ __forceinline__ void next_edge(const Gen &gen, uint32_t row, int64_t next, Edge &e) {
+    if constexpr (Gen::kBelow) {
+        e.at = next;
+        e.below = gen.below(row, next);
+        __syncwarp();
+    }
+}
+
 // A warp per row, one limb per lane, four 32-limb groups per step: for rows
 // whose last 128-limb group of carry_warp_rows would be mostly empty and whose
 // chunks are mostly at an end of the row (see run_carry).
@@ -295,17 +327,19 @@ __global__ void __launch_bounds__(256) carry_limb_rows(Gen gen, uint32_t *C, uin
     for (uint32_t row = gwarp; row < N; row += nwarps) {
         uint32_t *out = C + row * sC;
         uint32_t cin = 0u;
+        Edge edge;
         for (uint32_t base = 0; base < Lc; base += 32u * kGroups) {
             uint32_t s[kGroups], gm[kGroups], pm[kGroups];
 #pragma unroll
             for (int u = 0; u < kGroups; ++u) {
                 const uint32_t j = base + u * 32u + lane;
                 uint32_t x = 0u, y = 0u;
-                if (j < Lc) gen.limb(row, j, x, y);
+                if (j < Lc) gen.limb(row, j, x, y, edge);
                 s[u] = SUB ? x - y : x + y;
                 gm[u] = __ballot_sync(0xffffffffu, SUB ? x < y : s[u] < x);
                 pm[u] = __ballot_sync(0xffffffffu, s[u] == (SUB ? 0u : 0xffffffffu));
             }
+            next_edge(gen, row, (int64_t)base + 32 * kGroups, edge);
 #pragma unroll
             for (int u = 0; u < kGroups; ++u) {
                 const uint32_t j = base + u * 32u + lane;
@@ -331,6 +365,7 @@ __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uin
     const uint32_t nwarps = gridDim.x * warps_per_cta;
     for (uint32_t row = gwarp; row < N; row += nwarps) {
         uint32_t cin = 0u;
+        Edge edge;
         uint32_t *out = C + row * sC;
         for (int64_t base = -row_offset(out); base < (int64_t)Lc; base += 128 * UNROLL) {
             uint32_t s[UNROLL][4], gm[UNROLL], pm[UNROLL];
@@ -338,11 +373,12 @@ __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uin
             for (int u = 0; u < UNROLL; ++u) {
                 uint32_t x[4], y[4];
                 bool g, p;
-                gen.template read<kByWarp>(row, base + u * 128 + 4 * lane, x, y);
+                gen.template read<kByWarp>(row, base + u * 128 + 4 * lane, x, y, edge);
                 chunk_raw<SUB>(x, y, s[u], g, p);
                 gm[u] = __ballot_sync(0xffffffffu, g);
                 pm[u] = __ballot_sync(0xffffffffu, p);
             }
+            next_edge(gen, row, base + 128 * UNROLL, edge);
 #pragma unroll
             for (int u = 0; u < UNROLL; ++u) {
                 const GroupCarry gc = resolve_group(gm[u], pm[u], cin);
@@ -381,11 +417,14 @@ carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_r
     uint32_t *out = C + row * sC;
     const int64_t base = (int64_t)t * kTileSpan - row_offset(out) + w * 128 + 4 * lane;
     uint32_t s[kTileSub][4], gm[kTileSub], pm[kTileSub];
+    Edge edge;
+    if constexpr (Gen::kBelow)
+        if (gen.edges) edge = Edge{(int64_t)t * kTileSpan - row_offset(out), gen.edges[tile]};
 #pragma unroll
     for (int u = 0; u < kTileSub; ++u) {
         uint32_t x[4], y[4];
         bool g, p;
-        gen.template read<kByLane>(row, base + u * (128 * kTileWarps), x, y);
+        gen.template read<kByLane>(row, base + u * (128 * kTileWarps), x, y, edge);
         chunk_raw<SUB>(x, y, s[u], g, p);
         gm[u] = __ballot_sync(0xffffffffu, g);
         pm[u] = __ballot_sync(0xffffffffu, p);
@@ -408,6 +447,17 @@ carry_tiles(Gen gen, uint32_t *C, uint64_t sC, uint32_t Lc, uint32_t tiles_per_r
     // P: the tile's result is all ones (all zeros), which with carry-in 0 means
     // that every limb's raw sum is
     if (threadIdx.x == 0) flags[tile] = tc.carry_out | ((tp == 0xffffffffu) ? 2u : 0u);
+}
+
+// In-place mul_small of rows in tiles: each tile's limb below, before any
+// tile's results are written.
+__global__ void __launch_bounds__(256) tile_edges(GenMulSmall<true> gen, const uint32_t *C, uint64_t sC, uint64_t total,
+                                                  uint32_t tiles_per_row, uint32_t *edges) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const uint32_t row = (uint32_t)(i / tiles_per_row);
+    const int64_t t = (int64_t)(i - (uint64_t)row * tiles_per_row);
+    edges[i] = gen.below(row, t * kTileSpan - row_offset(C + row * sC));
 }
 
 // ---------------------------------------------------------------------------
@@ -529,13 +579,26 @@ size_t batch_sub_small_workspace_size(uint32_t N, uint32_t L_a, uint32_t L_c) {
 
 void batch_mul_small(const uint32_t *A, uint32_t B, uint32_t *C, uint32_t *workspace, uint32_t N,
                      uint32_t L_a, uint32_t L_c, uint32_t stride_A, uint32_t stride_C) {
-    GenMulSmall g{A, B, L_a, stride_A};
-    run_carry<GenMulSmall, false>(g, C, N, L_c, stride_C, workspace);
+    if (A != C) {
+        run_carry<GenMulSmall<false>, false>({A, B, L_a, stride_A, nullptr}, C, N, L_c, stride_C, workspace);
+        return;
+    }
+    GenMulSmall<true> g{A, B, L_a, stride_A, nullptr};
+    if (N && L_c && plan_for(N, L_c) == CarryPlan::Tiles) {
+        const uint32_t tiles = carry_tile_count(L_c);
+        const uint64_t total = (uint64_t)N * tiles;
+        uint32_t *edges = workspace + total;   // behind the flags
+        tile_edges<<<(unsigned)((total + 255u) / 256u), 256, 0, current_stream()>>>(g, C, stride_C, total, tiles,
+                                                                                    edges);
+        GPUPI_LAUNCH_CHECK();
+        g.edges = edges;
+    }
+    run_carry<GenMulSmall<true>, false>(g, C, N, L_c, stride_C, workspace);
 }
 
 size_t batch_mul_small_workspace_size(uint32_t N, uint32_t L_a, uint32_t L_c) {
     (void)L_a;
-    return carry_workspace_bytes(N, L_c);
+    return 2u * carry_workspace_bytes(N, L_c);   // flags, and in place the tiles' edges
 }
 
 void batch_shift_add_simple(const uint32_t *A, const uint32_t *B, uint32_t *C, uint32_t *workspace,

@@ -43,6 +43,22 @@ def test_lengths_and_alignments(ctx, Lc):
             assert np.array_equal(got[:oc], C[:oc])
 
 
+@pytest.mark.parametrize("L", [5, 125, 126, 130, 144, 145, 254, 300, 509, 513, 1300, 4090, 4096, 4097, 13000, 70001])
+@pytest.mark.parametrize("N", [1, 3, 150])
+def test_small_in_place(ctx, N, L):
+    """C is A: also for mul_small, whose limbs read the one below."""
+    if N * L > 1 << 20:
+        pytest.skip("one of the smaller batches covers this length")
+    rng = np.random.default_rng(L + N)
+    A = rand_buf(rng, N + 1, L + 1, L)
+    A[2:2 + L // 2] = 0xFFFFFFFF
+    for op in ("mul_small", "add_small", "sub_small"):
+        dA = to_dev(A)
+        getattr(ctx, op)(N, dA.at(1), L, L + 1, 0xFFFFFFFB, dA.at(1), L, L + 1)
+        want = getattr(ref, op)(N, A[1:], L, L + 1, 0xFFFFFFFB, A[1:], L, L + 1)
+        assert np.array_equal(dA.numpy()[1:], want), op
+
+
 @pytest.mark.parametrize("L", [7, 61, 4095, 13000])
 @pytest.mark.parametrize("op", ["add", "sub"])
 def test_in_place_misaligned(ctx, op, L):
