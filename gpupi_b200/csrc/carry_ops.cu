@@ -355,9 +355,10 @@ __global__ void __launch_bounds__(256) carry_limb_rows(Gen gen, uint32_t *C, uin
 // A warp per row, UNROLL groups of 128 limbs per step.  Two for batches: the
 // registers of four (64 a thread) leave 32 warps per SM, which cost rows of 500
 // to 1000 limbs a second wave (20,000 sums of 600 limbs 45 us with four, 37 with
-// two; 65,536 of 1600 limbs 306 and 284).  Four for rows that run alone (one of
-// 4000 limbs 18.5 us with four, 20.5 with two).
-template <class Gen, bool SUB, int UNROLL>
+// two; 65,536 of 1600 limbs 306 and 284).  Four, each lane reading by its own
+// path, for long rows that run alone (one of 4000 limbs 18.5 us with four, 20.5
+// with two; one of 1600 limbs times a limb 6.2 us by lane, 8.2 by warp).
+template <class Gen, bool SUB, int UNROLL, Read MODE>
 __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uint64_t sC, uint32_t N, uint32_t Lc) {
     const uint32_t lane = lane_id();
     const uint32_t warps_per_cta = blockDim.x >> 5;
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(256) carry_warp_rows(Gen gen, uint32_t *C, uin
             for (int u = 0; u < UNROLL; ++u) {
                 uint32_t x[4], y[4];
                 bool g, p;
-                gen.template read<kByWarp>(row, base + u * 128 + 4 * lane, x, y, edge);
+                gen.template read<MODE>(row, base + u * 128 + 4 * lane, x, y, edge);
                 chunk_raw<SUB>(x, y, s[u], g, p);
                 gm[u] = __ballot_sync(0xffffffffu, g);
                 pm[u] = __ballot_sync(0xffffffffu, p);
@@ -507,10 +508,10 @@ static void run_carry(const Gen &gen, uint32_t *C, uint32_t N, uint32_t Lc, uint
         const bool limbs = Gen::kStreams == 2 ? Lc <= 192u || (Lc > 253u && Lc <= 381u && N >= 4096u) : Lc <= 144u;
         if (limbs)
             carry_limb_rows<Gen, SUB><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
-        else if (N <= (uint32_t)kNumSMs)
-            carry_warp_rows<Gen, SUB, 4><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
+        else if (N <= (uint32_t)kNumSMs && Lc > 509u)   // with the 3 limbs below a row: more than one step
+            carry_warp_rows<Gen, SUB, 4, kByLane><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
         else
-            carry_warp_rows<Gen, SUB, 2><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
+            carry_warp_rows<Gen, SUB, 2, kByWarp><<<grid, warps * 32, 0, st>>>(gen, C, sC, N, Lc);
         GPUPI_LAUNCH_CHECK();
     } else {
         const uint32_t tiles = carry_tile_count(Lc);

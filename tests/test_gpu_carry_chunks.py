@@ -100,7 +100,7 @@ def test_carry_through_many_tiles(ctx, tiles, off):
 
 
 WARP_ROWS = [(5, Lc) for Lc in (127, 128, 129, 144, 145, 192, 193, 253, 254, 381, 382, 511, 1021, 1300)]
-WARP_ROWS += [(148, 400), (149, 400), (149, 193), (4095, 254), (4096, 254), (4096, 381), (4096, 382)]
+WARP_ROWS += [(148, 509), (148, 510), (149, 510), (149, 193), (4095, 254), (4096, 254), (4096, 381), (4096, 382)]
 
 
 @pytest.mark.parametrize("N,Lc", WARP_ROWS)
