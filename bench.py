@@ -67,10 +67,10 @@ NCU_TRAFFIC_SOURCE = {"ntt_rows_fused": "ncu capture of k_rows on a 2^22 x 2^22-
 # blocks, not with bytes, so its count at 1e8 digits says nothing about 1e9.)
 INT_WINST_PER_BYTE = {
     "ntt_rows_level": (0.183426, 0.182728, 0.440234), "ntt_cols_fwd_first": (0.119126, 0.117517, 0.291312),
-    "ntt_cols_inv": (0.073824, 0.074517, 0.183087), "schoolbook_tc": (0.177557, 0.350959, 0.882674),
-    "ntt_crt_carry": (0.050188, 0.045934, 0.12533), "ntt_rows_fused": (0.18048, 0.17761, 0.423874),
+    "ntt_cols_inv": (0.073824, 0.074517, 0.183087), "schoolbook_tc": (0.175881, 0.347193, 0.872551),
+    "ntt_crt_carry": (0.050113, 0.045819, 0.125058), "ntt_rows_fused": (0.18048, 0.17761, 0.423874),
     "ntt_cols_fwd": (0.069918, 0.069917, 0.17593), "schoolbook": (0.219156, 0.17921, 0.53567),
-    "ntt_local": (0.444573, 0.436102, 1.027391), "carry_chain": (0.027847, 0.08159, 0.142997),
+    "ntt_local": (0.439653, 0.430949, 1.015864), "carry_chain": (0.027847, 0.08159, 0.142997),
     "ntt_rows_fwd": (0.097792, 0.091607, 0.244568), "ntt_rows_inv": (0.064503, 0.064857, 0.163097),
     "decimal_extract": (0.075693, 0.08626, 0.224201), "ntt_coset_combine": (0.086067, 0.074986, 0.215792),
     "shift": (0.035647, 0.045182, 0.115069), "decimal_leaf": (0.704212, 0.245135, 1.12563)}
