@@ -109,10 +109,11 @@ void batch_exactdiv_small(uint32_t *A, uint32_t B, uint32_t N, uint32_t L, uint3
     if (N == 0u || L == 0u || (B & 1u) == 0u) return;
     const uint32_t binv = inverse_mod_2_32(B);
     const unsigned grid = grid_for(N, kDivRows * kDivWarps, kNumSMs * 8);
-    // Measured, loads ahead against plain: one row of 1 to 28 limbs 4.0 / 3.5 us,
-    // of 101 8.2 / 6.2; 32 rows of 28 limbs 4.1 / 6.2, of 101 6.2 / 14.4; 500,000
-    // rows of 1 to 28 limbs 18.7 to 24.6 / 14.4 to 22.6, of 40 36.2 / 37.0.
-    if (N < 8u || (L <= 32u && N >= (1u << 18)))
+    // Measured, loads ahead against plain: one row of 64 limbs 5.1 / 4.1 us, of 128
+    // 6.7 / 6.2; three rows of 64 limbs 4.6 / 6.2, of 128 6.7 / 8.2; 32 rows of 28
+    // limbs 4.1 / 6.2, of 101 7.3 / 16.4; 500,000 rows of 1 to 28 limbs 18.7 to
+    // 24.6 / 14.4 to 22.6, of 40 36.2 / 37.0.
+    if (N == 1u || (L <= 32u && N >= (1u << 18)))
         exactdiv_plain_kernel<<<grid, kDivRows * kDivWarps, 0, current_stream()>>>(A, B, binv, N, L, stride_A);
     else
         exactdiv_kernel<<<grid, kDivRows * kDivWarps, 0, current_stream()>>>(A, B, binv, N, L, stride_A);

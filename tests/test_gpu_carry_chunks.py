@@ -132,7 +132,7 @@ def test_rows_of_a_warp(ctx, N, Lc):
         assert np.array_equal(dC.numpy(), want), op
 
 
-@pytest.mark.parametrize("N,L", [(1, 1), (7, 33), (7, 128), (8, 8), (8, 9), (9, 31), (33, 32), (33, 33), (40, 40),
+@pytest.mark.parametrize("N,L", [(1, 1), (1, 33), (1, 128), (2, 33), (2, 128), (8, 8), (8, 9), (9, 31), (33, 32), (33, 33), (40, 40),
                                  (40, 41), (65, 102), ((1 << 18) - 1, 3), (1 << 18, 3), ((1 << 18) + 5, 1)])
 def test_exactdiv_kernels(ctx, N, L):
     """Either side of the choice between the two kernels, and of their groups
